@@ -1,0 +1,441 @@
+"""What the speed of this library is measured on: calls of its public entry points
+(``unap_gb300.capi``) over the sizes, matrix families and options of the benchmark's
+configurations and of the serving stream (8 thousand to 2 million cells).
+
+``listed`` names the cases, ``draw`` gives more of the same ranges, ``prepare`` makes what a
+caller has in hand (matrix handle, hierarchy, device vectors), ``run`` makes one call, ``work``
+says what a call cannot do without and ``exact`` what it should return, in 64 bits.
+
+Matrices are made on the GPU from the seed alone, with the structure and distributions of
+``unap_gb300.workloads`` (hex grids; Laplacian, log-normal Poisson, convection-diffusion), cells
+numbered at random where "permuted" says so.
+"""
+import math
+import random
+
+import numpy as np
+import torch
+
+from unap_gb300 import capi
+from unap_gb300.workloads import LduSystem
+
+# the headline V-cycle of the benchmark: one Gauss-Seidel sweep before and after on the two finest
+# levels, Chebyshev of degree 3 below them
+HEADLINE = dict(smoother=1, cheby_degree=3, cheby_from=2, eig_ratio=60.0, n_pre=1, n_post=1)
+# the V-cycle that the solve server gives a request
+SERVED = dict(smoother=1, cheby_degree=3, cheby_from=0, eig_ratio=30.0, n_coarsest=200)
+
+
+def _case(name, kind, nx, ny, nz, family, permuted, **more):
+    c = dict(kind=kind, nx=nx, ny=ny, nz=nz, family=family, permuted=permuted)
+    c.update(more)
+    if name:
+        c["name"] = name
+    return c
+
+
+def listed():
+    return [
+        # one y = A x of a small pressure matrix inside a caller's own loop: launches and host work
+        _case("spmv_20cube", "spmv", 20, 20, 20, "lognormal", True),
+        # y = A x of the 200^3 convection-diffusion matrix (lower and upper coefficients): bandwidth
+        _case("spmv_200cube_nonsym", "spmv", 200, 200, 200, "convdiff", True),
+        # the DIC preconditioner as a caller's own solver applies it, an odd elongated grid
+        _case("dic_apply_61x97x43", "precond", 61, 97, 43, "laplace", True, precond=2),
+        # two Gauss-Seidel sweeps in FP64 on the 128^3 Laplacian
+        _case("gs_2_sweeps_128cube", "gauss_seidel", 128, 128, 128, "laplace", True, sweeps=2,
+              backward=False),
+        # the 32^3 natural-order Laplacian, PCG+DIC: 94 wavefronts, a small whole solve
+        _case("pcg_dic_32cube", "krylov", 32, 32, 32, "laplace", False, method=0, precond=2,
+              rel_tol=1e-8),
+        # PBiCGStab+DILU on a million-cell convection-diffusion matrix, odd edges
+        _case("bicg_dilu_97x101x103", "krylov", 97, 101, 103, "convdiff", True, method=1,
+              precond=3, rel_tol=1e-9),
+        # the mixed-precision preconditioner alone: one FP32 V-cycle of the headline's smoothers
+        _case("vcycle_fp32_160cube", "vcycle", 160, 160, 160, "lognormal", True, precision=1,
+              smoothers="headline"),
+        # the FP64 V-cycle with two Gauss-Seidel sweeps on every level (the library's defaults)
+        _case("vcycle_fp64_gs_128cube", "vcycle", 128, 128, 128, "laplace", True, precision=0,
+              smoothers="default"),
+        # the headline solve: mixed AMG-PCG of the 256^3 log-normal Poisson, tolerance 1e-10
+        _case("amg_mixed_256cube", "amg_solve", 256, 256, 256, "lognormal", True, precision=1,
+              smoothers="headline", rel_tol=1e-10),
+        # one request of the serving stream on its own: matrix, hierarchy and solve from host arrays
+        _case("request_110x66x70", "request", 110, 66, 70, "lognormal", True, precision=1,
+              smoothers="served", rel_tol=1e-8),
+        # many small systems of uneven size solved together
+        _case("batch_48_small", "batch", 20, 20, 20, "mixed", True, count=48, largest=32),
+        # the reference's multigrid solver with its Gauss-Seidel smoother
+        _case("mg_gs_57x44x39", "mg", 57, 44, 39, "laplace", True, smoother=1, rel_tol=1e-6),
+    ]
+
+
+def _edges(rng, lo, hi):
+    """An uneven grid of lo to hi cells (log-uniform), aspect up to 4, odd edges as they come."""
+    cells = math.exp(rng.uniform(math.log(lo), math.log(hi)))
+    aspect = rng.uniform(1.0, 4.0) if rng.random() < 0.5 else 1.0
+    e = (cells / aspect) ** (1.0 / 3.0)
+    dims = [max(4, round(e * aspect)), max(4, round(e * rng.uniform(0.9, 1.0))), max(4, round(e))]
+    rng.shuffle(dims)
+    return dims
+
+
+def draw(rng):
+    kind = rng.choice(["spmv", "spmv", "precond", "gauss_seidel", "krylov", "krylov", "vcycle",
+                       "vcycle", "amg_solve", "request", "batch", "mg"])
+    if kind == "spmv":
+        return _case(None, kind, *_edges(rng, 8e3, 8e6),
+                     rng.choice(["lognormal", "laplace", "convdiff"]), rng.random() < 0.8)
+    if kind == "precond":
+        family, precond = rng.choice([("laplace", 2), ("lognormal", 2), ("convdiff", 3)])
+        return _case(None, kind, *_edges(rng, 8e3, 2e6), family, True, precond=precond)
+    if kind == "gauss_seidel":
+        return _case(None, kind, *_edges(rng, 8e3, 2e6), rng.choice(["laplace", "convdiff"]), True,
+                     sweeps=rng.choice([1, 2]), backward=rng.random() < 0.5)
+    if kind == "krylov":
+        if rng.random() < 0.5:
+            return _case(None, kind, *_edges(rng, 8e3, 5e5), "laplace", rng.random() < 0.8,
+                         method=0, precond=2, rel_tol=1e-8)
+        return _case(None, kind, *_edges(rng, 8e3, 2e6), "convdiff", True, method=1, precond=3,
+                     rel_tol=1e-9)
+    if kind == "vcycle":
+        return _case(None, kind, *_edges(rng, 8e3, 4e6), rng.choice(["lognormal", "laplace"]),
+                     True, precision=rng.choice([0, 1, 1]),
+                     smoothers=rng.choice(["headline", "headline", "default", "served"]))
+    if kind == "amg_solve":
+        return _case(None, kind, *_edges(rng, 1e5, 4e6), "lognormal", True, precision=1,
+                     smoothers="headline", rel_tol=1e-10)
+    if kind == "request":
+        return _case(None, kind, *_edges(rng, 3e4, 1e6), "lognormal", True, precision=1,
+                     smoothers="served", rel_tol=1e-8)
+    if kind == "batch":
+        return _case(None, kind, 20, 20, 20, "mixed", True, count=rng.choice([5, 12, 33, 64]),
+                     largest=rng.choice([24, 28, 36]))
+    return _case(None, kind, *_edges(rng, 8e3, 2e5), "laplace", True,
+                 smoother=rng.choice([1, 2]), rel_tol=1e-6)
+
+
+# ---- matrices ---------------------------------------------------------------
+
+def _system(nx, ny, nz, family, permuted, seed):
+    """(LduSystem, its arrays as CUDA tensors) of an nx x ny x nz hex grid."""
+    dev = "cuda"
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(seed)
+    n = nx * ny * nz
+    f64 = dict(dtype=torch.float64, device=dev)
+    cells = torch.arange(n, device=dev).view(nz, ny, nx)
+    # the pairs of neighbours along x, y and z, and the slices of the grid they belong to
+    pairs = [((slice(None), slice(None), slice(0, -1)), (slice(None), slice(None), slice(1, None))),
+             ((slice(None), slice(0, -1)), (slice(None), slice(1, None))),
+             ((slice(0, -1),), (slice(1, None),))]
+    kappa = None
+    if family == "lognormal":
+        kappa = torch.exp(2.0 * torch.randn(n, generator=gen, **f64)).view(nz, ny, nx)
+    rows = torch.zeros(nz, ny, nx, **f64)  # sum of |off-diagonal| of each row
+    a, b, ca, cb = [], [], [], []
+    for lo, hi in pairs:
+        first, second = cells[lo], cells[hi]
+        if family == "laplace":
+            wa = wb = -torch.ones(first.shape, **f64)
+        elif family == "lognormal":
+            wa = wb = -2.0 * kappa[lo] * kappa[hi] / (kappa[lo] + kappa[hi])
+        else:
+            flux = 5.0 * torch.randn(first.shape, generator=gen, **f64)
+            wa = -(1.0 + torch.clamp(-flux, min=0.0))
+            wb = -(1.0 + torch.clamp(flux, min=0.0))
+        rows[lo] -= wa
+        rows[hi] -= wb
+        a.append(first.reshape(-1))
+        b.append(second.reshape(-1))
+        ca.append(wa.reshape(-1))
+        cb.append(wb.reshape(-1))
+    a, b, ca, cb = (torch.cat(t) for t in (a, b, ca, cb))
+    shift = {"laplace": 1e-6, "lognormal": 1e-8, "convdiff": 0.01}[family]
+    diag = (rows + shift).view(-1)
+    if permuted:
+        perm = torch.randperm(n, generator=gen, device=dev)
+        inv = torch.empty_like(perm)
+        inv[perm] = torch.arange(n, device=dev)
+        a, b, diag = perm[a], perm[b], diag[inv]
+    low, up = torch.minimum(a, b), torch.maximum(a, b)
+    order = torch.sort(low * n + up).indices
+    swapped = (a > b)[order]
+    low, up = low[order].int(), up[order].int()
+    ca, cb = ca[order], cb[order]
+    upper = torch.where(swapped, cb, ca)   # A[low][up]
+    lower = None if family != "convdiff" else torch.where(swapped, ca, cb)
+    if family == "lognormal":
+        rhs = torch.randn(n, generator=gen, **f64)
+        rhs -= rhs.mean()
+    elif family == "laplace":
+        rhs = 2.0 * torch.rand(n, generator=gen, **f64) - 1.0
+    else:
+        rhs = torch.rand(n, generator=gen, **f64)
+    t = dict(n=n, low=low, up=up, lower=lower, diag=diag, upper=upper, b=rhs)
+    host = {k: None if v is None else v.cpu().numpy() for k, v in t.items() if k != "n"}
+    s = LduSystem(n, host["low"], host["up"], host["lower"], host["diag"], host["upper"],
+                  host["b"], name=family)
+    return s, t
+
+
+def _faces(nx, ny, nz):
+    return 3 * nx * ny * nz - nx * ny - ny * nz - nx * nz
+
+
+def _amg_options(case):
+    o = {"headline": HEADLINE, "served": SERVED, "default": {}}[case["smoothers"]]
+    return dict(o, precision=case["precision"], rel_tol=case.get("rel_tol", 1e-10))
+
+
+def _batch_systems(case):
+    """(nx, ny, nz, family) of each system of a batch: 8 thousand cells and up, as the small
+    requests of the serving stream, two thirds PCG+DIC, the others PBiCGStab+DILU."""
+    rng = random.Random(case["count"])
+    return [(rng.randint(20, case["largest"]), rng.randint(20, case["largest"]),
+             rng.randint(20, case["largest"]), "convdiff" if k % 3 == 2 else "laplace")
+            for k in range(case["count"])]
+
+
+# ---- the calls --------------------------------------------------------------
+
+def prepare(case, seed):
+    kind = case["kind"]
+    if kind == "batch":
+        made = [_system(nx, ny, nz, family, True, seed * 1000 + k)
+                for k, (nx, ny, nz, family) in enumerate(_batch_systems(case))]
+        sizes = [s.n for s, _ in made]
+        b = torch.cat([t["b"] for _, t in made])
+        x = torch.zeros_like(b)
+        xs, bs = x.split(sizes), b.split(sizes)
+        items = [dict(matrix=capi.DeviceMatrix(s), method=0 if s.symm else 1,
+                      precond=2 if s.symm else 3, x=xi, b=bi, rel_tol=1e-8, max_iter=1000)
+                 for (s, _), xi, bi in zip(made, xs, bs)]
+        return dict(case=case, batch=capi.Batch(), items=items, x=x, b=b)
+    s, t = _system(case["nx"], case["ny"], case["nz"], case["family"], case["permuted"], seed)
+    st = dict(case=case, b=t["b"], x=torch.zeros_like(t["b"]))
+    if kind == "request":
+        st["system"] = s
+        return st
+    st["matrix"] = capi.DeviceMatrix(s)
+    if kind in ("vcycle", "amg_solve"):
+        st["amg"] = capi.DeviceAmg(st["matrix"], **_amg_options(case))
+    elif kind == "mg":
+        st["mg"] = capi.DeviceMG(st["matrix"], smoother=case["smoother"],
+                                 rel_tol=case["rel_tol"], max_iter=100)
+    return st
+
+
+def run(state):
+    case, x, b = state["case"], state["x"], state["b"]
+    kind = case["kind"]
+    if kind == "spmv":
+        state["matrix"].spmv(b, x)
+        return x
+    if kind == "precond":
+        state["matrix"].precondition(case["precond"], b, x)
+        return x
+    if kind == "vcycle":
+        state["amg"].vcycle(b, x)
+        return x
+    if kind == "request":
+        s = state["system"]
+        matrix = capi.DeviceMatrix(s)
+        amg = capi.DeviceAmg(matrix, **_amg_options(case))
+        solution = np.zeros(s.n)
+        stats = amg.solve_host(solution, s.b)
+        amg.close()
+        matrix.close()
+        return dict(x=solution, iterations=stats["nIterations"], converged=stats["converged"])
+    x.zero_()
+    if kind == "gauss_seidel":
+        state["matrix"].gauss_seidel(x, b, case["sweeps"], case["backward"])
+        return x
+    if kind == "batch":
+        stats, _ = state["batch"].solve(state["items"])
+        return dict(x=x, iterations=[s["nIterations"] for s in stats][:60])
+    if kind == "krylov":
+        stats = state["matrix"].krylov_solve(case["method"], case["precond"], x, b,
+                                             rel_tol=case["rel_tol"], max_iter=1000)
+    elif kind == "amg_solve":
+        stats = state["amg"].solve(x, b)
+    else:
+        stats = state["mg"].solve(x, b)
+    return dict(x=x, iterations=stats["nIterations"], converged=stats["converged"])
+
+
+def work(case):
+    """Bytes and operations of one pass.  A product, a sweep or a preconditioner reads the
+    matrix as LDU holds it (two 4-byte addresses and one or two 8-byte coefficients a face, the
+    diagonal) and its vectors once; a V-cycle does three such passes on a hierarchy of twice the
+    finest level; a solve repeats its iteration about as often as it takes to converge."""
+    if case["kind"] == "batch":
+        cells = sum(nx * ny * nz for nx, ny, nz, _ in _batch_systems(case))
+        return {"bytes": 40.0 * (40 * cells + 24 * 3 * cells), "flops": 40.0 * 60 * cells}
+    n = case["nx"] * case["ny"] * case["nz"]
+    f = _faces(case["nx"], case["ny"], case["nz"])
+    face = 24 if case["family"] == "convdiff" else 16
+    kind = case["kind"]
+    product = 24 * n + face * f
+    if kind == "spmv":
+        return {"bytes": product, "flops": 2 * n + 4 * f}
+    if kind == "precond":
+        return {"bytes": 32 * n + face * f, "flops": 3 * n + 6 * f}
+    if kind == "gauss_seidel":
+        return {"bytes": case["sweeps"] * (8 * n + product), "flops": case["sweeps"] * 4 * (n + f)}
+    size = 4 if case.get("precision") else 8
+    vcycle = 2 * 3 * ((3 * size + 4) * n + (8 + size) * f)
+    times = 1
+    if kind == "krylov":
+        halves = 2 if case["method"] else 1
+        iteration = halves * (product + 32 * n + face * f + 48 * n)
+        times = 60
+    elif kind == "mg":
+        iteration = vcycle + 2 * product
+        times = 30
+    elif kind == "vcycle":
+        iteration = vcycle
+    else:
+        iteration = vcycle + product + 96 * n
+        times = 50 if kind == "amg_solve" else 25
+    return {"bytes": float(times) * iteration, "flops": float(times) * iteration / 4}
+
+
+# ---- the same in 64 bits, by plain torch ------------------------------------
+
+def _product(t):
+    """x -> A x, by a compressed-row matrix."""
+    n, low, up = t["n"], t["low"].long(), t["up"].long()
+    lower = t["upper"] if t["lower"] is None else t["lower"]
+    every = torch.arange(n, device=low.device)
+    rows = torch.cat([every, low, up])
+    cols = torch.cat([every, up, low])
+    vals = torch.cat([t["diag"], t["upper"], lower])
+    order = torch.sort(rows * n + cols).indices
+    start = torch.zeros(n + 1, dtype=torch.int64, device=low.device)
+    start[1:] = torch.cumsum(torch.bincount(rows, minlength=n), 0)
+    m = torch.sparse_csr_tensor(start, cols[order], vals[order], (n, n))
+    return lambda x: m @ x
+
+
+def _levels(t):
+    """Each cell's place in the order that the sweeps need: after all its lower neighbours."""
+    low, up = t["low"].long(), t["up"].long()
+    level = torch.zeros(t["n"], dtype=torch.int64, device=low.device)
+    while True:
+        new = level.clone().scatter_reduce_(0, up, level[low] + 1, "amax")
+        if torch.equal(new, level):
+            return level
+        level = new
+
+
+def _by_level(level, at):
+    """Indices of `at` (cells) grouped by their level, as a list of index tensors."""
+    of = level[at]
+    order = torch.sort(of, stable=True).indices
+    counts = torch.bincount(of, minlength=int(level.max()) + 1).tolist()
+    return list(order.split(counts))
+
+
+def _ldu_precond(t, dilu, r):
+    """DIC or DILU (factored by rows in cell order) applied to r."""
+    level = _levels(t)
+    low, up, upper = t["low"].long(), t["up"].long(), t["upper"]
+    lower = upper if t["lower"] is None else t["lower"]
+    down = _by_level(level, up)
+    d = t["diag"].clone()
+    for f in down:
+        d.index_add_(0, up[f], -(upper[f] * (lower if dilu else upper)[f]) / d[low[f]])
+    w = r / d
+    for f in down:
+        w.index_add_(0, up[f], -(lower if dilu else upper)[f] * w[low[f]] / d[up[f]])
+    for f in reversed(_by_level(level, low)):
+        w.index_add_(0, low[f], -upper[f] * w[up[f]] / d[low[f]])
+    return w
+
+
+def _gauss_seidel(t, x, b, sweeps, backward):
+    level = _levels(t)
+    low, up, upper = t["low"].long(), t["up"].long(), t["upper"]
+    lower = upper if t["lower"] is None else t["lower"]
+    cells = _by_level(level, torch.arange(t["n"], device=low.device))
+    steps = list(zip(cells, _by_level(level, up), _by_level(level, low)))
+    for _ in range(sweeps):
+        for c, f_up, f_low in (reversed(steps) if backward else steps):
+            x[c] = b[c]
+            x.index_add_(0, up[f_up], -lower[f_up] * x[low[f_up]])
+            x.index_add_(0, low[f_low], -upper[f_low] * x[up[f_low]])
+            x[c] /= t["diag"][c]
+    return x
+
+
+def _solution(t, most=20000):
+    """A x = b by conjugate gradients (or BiCGStab) with the diagonal as preconditioner, carried
+    on until the residual falls no further."""
+    mul, b, d = _product(t), t["b"], t["diag"]
+    x = torch.zeros_like(b)
+    best, best_x = float(b.norm()), x.clone()
+    for _ in range(4):  # restarts from the true residual
+        r = b - mul(x)
+        goal = max(1e-15 * float(b.norm()), 1e-9 * float(r.norm()))
+        if t["lower"] is None:
+            z = r / d
+            p, rz = z.clone(), torch.dot(r, z)
+            for it in range(most):
+                q = mul(p)
+                alpha = rz / torch.dot(p, q)
+                x = x + alpha * p
+                r = r - alpha * q
+                z = r / d
+                new = torch.dot(r, z)
+                p = z + (new / rz) * p
+                rz = new
+                if it % 20 == 19 and not float(r.norm()) > goal:
+                    break
+        else:
+            r0, p, q, s = r.clone(), torch.zeros_like(r), torch.zeros_like(r), None
+            rho = alpha = omega = torch.ones((), dtype=r.dtype, device=r.device)
+            for it in range(most):
+                new = torch.dot(r0, r)
+                p = r + (new / rho) * (alpha / omega) * (p - omega * q)
+                rho = new
+                y = p / d
+                q = mul(y)
+                alpha = rho / torch.dot(r0, q)
+                s = r - alpha * q
+                z = s / d
+                u = mul(z)
+                omega = torch.dot(u, s) / torch.dot(u, u)
+                x = x + alpha * y + omega * z
+                r = s - omega * u
+                if it % 10 == 9 and not float(r.norm()) > goal:
+                    break
+        now = float((b - mul(x)).norm())
+        if not now < 0.5 * best:
+            if now < best:
+                best_x = x
+            break
+        best, best_x = now, x.clone()
+    return best_x
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "batch":
+        xs = [_solution(_system(nx, ny, nz, family, True, seed * 1000 + k)[1])
+              for k, (nx, ny, nz, family) in enumerate(_batch_systems(case))]
+        return dict(x=torch.cat(xs), iterations=None)
+    if kind == "vcycle":  # the hierarchy would have to be made by a loop over the cells
+        return None
+    n = case["nx"] * case["ny"] * case["nz"]
+    if kind in ("amg_solve", "request", "krylov", "mg") and n > 2.5e6:
+        return None
+    _, t = _system(case["nx"], case["ny"], case["nz"], case["family"], case["permuted"], seed)
+    if kind == "spmv":
+        return _product(t)(t["b"])
+    if kind == "precond":
+        return _ldu_precond(t, case["precond"] == 3, t["b"])
+    if kind == "gauss_seidel":
+        return _gauss_seidel(t, torch.zeros_like(t["b"]), t["b"], case["sweeps"], case["backward"])
+    x = _solution(t)
+    return dict(x=x.cpu().numpy() if kind == "request" else x, iterations=None, converged=None)
