@@ -498,7 +498,9 @@ int unap_cuda_set_executor(int persistent);
  * (the first CUDA call of the process on that device). */
 int unap_cuda_set_host_wait(int mode);
 
-/* Per-wavefront Gauss-Seidel launches use programmatic dependent launch:
+/* Per-wavefront Gauss-Seidel launches (the FP32 V-cycle's on levels of more
+ * than 2,097,152 rows, and every level's under unap_cuda_set_packed_sweeps 0,
+ * 2 or 3; other sweeps are one launch) use programmatic dependent launch:
  * the next wavefront's kernel starts launching while the previous one runs
  * and loads its rows' matrix data before it waits for it (1, default); 0
  * launches them one after the other.  Results are identical.  Returns the
@@ -512,12 +514,15 @@ int unap_cuda_set_wave_pdl(int on);
  * the reference. */
 int unap_cuda_set_wave_grid(int oneRowPerThread);
 
-/* AMG V-cycle Gauss-Seidel sweeps on levels whose rows average more than 8
- * entries read a row-packed copy of the level (a row's entries as 16-byte
- * records, loaded before the dependency wait): mode 1 (default) holds the
- * first 16 (FP32) / 8 (FP64) entries in registers on levels averaging under
- * 12.5 entries per row and 24 / 12 above; mode 2 always 16 / 8, mode 3
- * always 24 / 12; mode 0 reads the SELL-32 storage.  Results are
+/* AMG V-cycle Gauss-Seidel sweeps.  Mode 1 (default): one launch a sweep on
+ * every FP64 level and on FP32 levels of up to 2,097,152 rows, a launch per
+ * wavefront above; the other modes launch per wavefront on every level.
+ * Per-wavefront launches on levels whose rows average more than 8 entries
+ * read a row-packed copy of the level (a row's entries as 16-byte records,
+ * loaded before the dependency wait): mode 1 holds the first 16 (FP32) / 8
+ * (FP64) entries in registers on levels averaging under 12.5 entries per row
+ * and 24 / 12 above; mode 2 always 16 / 8, mode 3 always 24 / 12; mode 0
+ * reads the SELL-32 storage.  Results are
  * identical.  Returns the previous setting.  No counterpart in the
  * reference. */
 int unap_cuda_set_packed_sweeps(int mode);
@@ -555,9 +560,9 @@ int unap_cuda_set_cheby_tail_rows(int rows);
  * the dense coarsest solve and back, runs in one launch of a single
  * thread-block cluster, wavefronts separated by the cluster barrier; tail
  * levels with at most singleRows rows run on the cluster's first CTA alone.
- * tailRows = 0 launches one kernel per wavefront on every level.  The
- * V-cycle result is bit-identical either way.  Defaults: FP64 2097152 and
- * 8192, FP32 8192 and 8192; the previous values are returned through the
+ * tailRows = 0 runs no level in it.  The
+ * V-cycle result is bit-identical either way.  Defaults: FP64 0 and 8192,
+ * FP32 8192 and 8192; the previous values are returned through the
  * (nullable) pointers.  Applies to V-cycles launched after the call, CUDA
  * graphs captured before keep their launches.  No counterpart in the
  * reference. */

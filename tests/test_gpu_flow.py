@@ -1,0 +1,77 @@
+"""Gauss-Seidel sweeps in one launch: rows wait for their neighbours by value.
+
+Bit-identical to the oracle's sweeps (the same entry order and roundings, so
+the tolerance is zero) at the sizes where the launch can go wrong: single
+rows, wavefronts of one row, tasks cut at slice and wavefront boundaries, rows
+longer than a chunk, every lane count of the size rule, more sweeps than one
+launch takes, and NaNs with the bit pattern that marks a value still missing.
+"""
+import numpy as np
+import pytest
+
+from unap_gb300 import capi
+from unap_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def random_system(n, faces, seed, symm=False, near=None):
+    """About `faces` random faces (distinct pairs, at most `near` cells apart),
+    owner-sorted, diagonally dominant."""
+    rng = np.random.default_rng(seed)
+    a = rng.integers(0, n, faces)
+    d = rng.integers(1, (near or n), faces)
+    b = a + d
+    ok = b < n
+    key = np.unique(a[ok].astype(np.int64) * n + b[ok])
+    l, u = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    upper = rng.standard_normal(l.size)
+    lower = upper if symm else rng.standard_normal(l.size)
+    diag = W._fast_row_abs_sum(n, l, u, upper, lower) + 1.0
+    return W.LduSystem(n, l, u, None if symm else lower, diag, upper, rng.standard_normal(n))
+
+
+CASES = {
+    "one_cell": lambda: random_system(1, 0, 1),
+    "no_faces_33": lambda: random_system(33, 0, 2),
+    "chain_70": lambda: W.laplace(70, 1, 1, seed=3),           # 70 wavefronts of one row
+    "plane_31x33": lambda: W.laplace(31, 33, 1, seed=4),       # wavefronts of 1 to 31 rows
+    "grid_7pt": lambda: W.convdiff(17, 13, 11, seed=5),
+    "rows_of_45": lambda: random_system(300, 9000, 6),         # longer than any chunk
+    "rows_of_20": lambda: random_system(2500, 25000, 7, symm=True),
+    "wide_4_lanes": lambda: random_system(160_000, 900_000, 8, near=4000),
+    "wide_1_lane": lambda: random_system(310_000, 1_700_000, 9, near=9000),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("backward", [False, True])
+def test_sweeps_bit_exact(cuda, orc, name, backward):
+    torch = cuda
+    s = CASES[name]()
+    A = capi.DeviceMatrix(s)
+    x0 = np.random.default_rng(s.n).standard_normal(s.n)
+    b = torch.tensor(s.b, device="cuda")
+    for sweeps in ((1, 2) if s.n > 100_000 else (1, 4, 5, 9)):
+        x = torch.tensor(x0, device="cuda")
+        A.gauss_seidel(x, b, sweeps, backward=backward)
+        assert np.array_equal(x.cpu().numpy(), orc.gs(s, x0, s.b, sweeps, backward=backward)), sweeps
+    A.close()
+
+
+@pytest.mark.parametrize("pattern", [0xFFFFFFFFFFFFFFFF, 0x7FF8000000000000, 0x7FF0000000000000])
+def test_nan_and_inf_inputs(cuda, orc, pattern):
+    """A NaN that looks like a missing value, another NaN and an infinity
+    spread as in the oracle, and no wait runs out on them."""
+    torch = cuda
+    s = W.laplace(9, 8, 7, seed=1, permute=True)
+    bad = np.array([pattern], dtype=np.uint64).view(np.float64)[0]
+    A = capi.DeviceMatrix(s)
+    for where in ("b", "x"):
+        x0 = np.random.default_rng(2).standard_normal(s.n)
+        b = s.b.copy()
+        (b if where == "b" else x0)[s.n // 2] = bad
+        x = torch.tensor(x0, device="cuda")
+        A.gauss_seidel(x, torch.tensor(b, device="cuda"), 2)
+        assert np.array_equal(x.cpu().numpy(), orc.gs(s, x0, b, 2), equal_nan=True)
+    A.close()

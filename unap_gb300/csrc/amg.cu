@@ -168,6 +168,13 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
     }
     UNAP_CK(cudaStreamSynchronize(s));
     phase(3);
+    // the Gauss-Seidel levels' vectors
+    for (int k = 0; k < L; ++k)
+        if (!isCheby(k) && (params.nPre > 0 || params.nPost > 0) &&
+            (params.precision == 0 || lv[(size_t)k].n <= kFlowRows32))
+            lv[(size_t)k].sweeps.init((size_t)lv[(size_t)k].n,
+                                      params.precision == 1 ? sizeof(float) : sizeof(double),
+                                      std::min(std::max(params.nPre, params.nPost), 4));
     // row-packed copies of the levels the cluster tail may run (in the
     // precision of the V-cycle)
     for (int k = 0; k < L; ++k) {
@@ -219,7 +226,7 @@ size_t AmgHierarchy::deviceBytes() const
         if (l.own) b += l.own->deviceBytes();
         b += l.childStart.bytes() + l.child.bytes() + l.cmap.bytes() + l.x.bytes() + l.b.bytes() +
              l.r.bytes() + l.xf.bytes() + l.bf.bytes() + l.rf.bytes() + l.pack.bytes() +
-             l.t.bytes() + l.tf.bytes();
+             l.t.bytes() + l.tf.bytes() + l.sweeps.bytes();
     }
     return b;
 }
@@ -317,6 +324,11 @@ std::vector<double> AmgHierarchy::eigenvalues() const
     return v;
 }
 
+void AmgHierarchy::check() const
+{
+    for (auto& l : lv) l.sweeps.check();
+}
+
 int AmgHierarchy::tailFirst(size_t elemBytes) const
 {
     const int L = nLevels() - 1;
@@ -409,9 +421,9 @@ void AmgHierarchy::sweep(const Exec& ex, int k, const Level& Lk, const Rows<T>& 
         // register window by mean row length (measured per level on 256^3)
         const bool wide = mode == 3 || (mode == 1 && 2.0 * Lk.nf > 12.5 * Lk.n);
         gs_sweep_packed<T>(ex, Lk, P, Rk.diag, x, b, backward, xIsZero, wide, g);
-    }
-    else
+    } else {
         gs_sweep<T>(ex, Lk, Rk, x, b, backward, xIsZero, g);
+    }
 }
 
 template <class T>
@@ -453,7 +465,7 @@ ChebTailArgs<T> AmgHierarchy::chebTailArgs(int k)
 }
 
 template <class T>
-void AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
+const T* AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
 {
     const int L = nLevels() - 1;
     T* x = X<T>(k);
@@ -462,17 +474,17 @@ void AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
     if (k == curTail && k < L) {
         launch_tail<T>(ex, k, g);
         if (profOut) UNAP_CK(cudaEventRecordWithFlags((*profOut)[(size_t)k], ex.s, cudaEventRecordExternal));
-        return;
+        return x;
     }
     if (k == chebTail) {
         launch_cheb_tail<T>(ex, chebTailArgs<T>(k), g);
         if (profOut) UNAP_CK(cudaEventRecordWithFlags((*profOut)[(size_t)k], ex.s, cudaEventRecordExternal));
-        return;
+        return x;
     }
     if (k == L) {
         k_dense_apply<T>(ex, nc, Minv.p, b, denseGather, x, g);
         if (profOut) UNAP_CK(cudaEventRecordWithFlags((*profOut)[(size_t)k], ex.s, cudaEventRecordExternal));
-        return;
+        return x;
     }
     const Level& Lk = *lv[(size_t)k].L;
     Rows<T> Rk = rowsT<T>(Lk);
@@ -480,6 +492,7 @@ void AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
     const bool cheb = isCheby(k);
     const Lv& V = lv[(size_t)k];
     const int deg = params.chebyDegree;
+    T* cur = x;  // the level's iterate: the sweeps leave it in one of their vectors
     if (cheb) {
         // pre-smoothing from x = 0 (w shares the residual's buffer); the
         // first step of a coarse level ran inside the restriction
@@ -492,12 +505,15 @@ void AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
         for (int j = 1; j < deg; ++j)
             k_cheb_step<T>(ex, Rk, chebBuf<T>(k, j - 1), chebBuf<T>(k, j), b, r, (T)V.d1[j],
                            (T)V.d2[j], 0, g);
-    } else if (params.nPre > 0) {
+    } else if (params.nPre > 0 && !flows(k)) {
         for (int s = 0; s < params.nPre; ++s) sweep<T>(ex, k, Lk, Rk, x, b, false, s == 0, g);
+    } else if (params.nPre > 0) {
+        cur = flow_gs<T>(ex, Lk, Rk, V.sweeps, nullptr, b, params.nPre, false, true, nullptr,
+                         nullptr, g);
     } else {
         k_fill<T>(ex, Lk.n, x, T(0));
     }
-    k_residual<T>(ex, Rk, x, b, r, RSpec{}, g);
+    k_residual<T>(ex, Rk, cur, b, r, RSpec{}, g);
     const Lv& C = lv[(size_t)k + 1];
     if (isCheby(k + 1))
         k_restrict_cheb_zero<T>(ex, C.n, C.childStart.p, C.child.p, r, B<T>(k + 1),
@@ -505,26 +521,38 @@ void AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
                                 (T)C.Rth, g);
     else
         k_restrict<T>(ex, C.n, C.childStart.p, C.child.p, r, B<T>(k + 1), g);
-    vcycle_level<T>(ex, k + 1, g);
+    const T* e = vcycle_level<T>(ex, k + 1, g);
     if (cheb) {
         // post-smoothing from x + P e: the prolongation writes the buffer the
         // chain starts from
         T* prev = (deg % 2 == 0) ? x : Tmp<T>(k);
         if (prev == x)
-            k_prolong_add<T>(ex, Lk.n, C.cmap.p, X<T>(k + 1), x, g);
+            k_prolong_add<T>(ex, Lk.n, C.cmap.p, e, x, g);
         else
-            k_prolong_add_to<T>(ex, Lk.n, C.cmap.p, X<T>(k + 1), x, prev, g);
+            k_prolong_add_to<T>(ex, Lk.n, C.cmap.p, e, x, prev, g);
         for (int j = 0; j < deg; ++j) {
             T* out = chebBuf<T>(k, j);
             k_cheb_step<T>(ex, Rk, prev, out, b, r, j == 0 ? (T)V.Rth : (T)V.d1[j],
                            j == 0 ? T(0) : (T)V.d2[j], j == 0 ? 1 : 0, g);
             prev = out;
         }
-    } else {
-        k_prolong_add<T>(ex, Lk.n, C.cmap.p, X<T>(k + 1), x, g);
+    } else if (!flows(k)) {
+        k_prolong_add<T>(ex, Lk.n, C.cmap.p, e, x, g);
         for (int s = 0; s < params.nPost; ++s) sweep<T>(ex, k, Lk, Rk, x, b, true, false, g);
+    } else if (params.nPost > 0) {
+        k_prolong_add<T>(ex, Lk.n, C.cmap.p, e, cur, g);
+        // the finest FP64 level's result is the caller's vector
+        T* last = k == 0 && std::is_same<T, double>::value ? x : nullptr;
+        cur = flow_gs<T>(ex, Lk, Rk, V.sweeps, cur, b, params.nPost, true, false,
+                         cur == last ? nullptr : last, cur == last ? last : nullptr, g);
+    } else if (cur == x) {
+        k_prolong_add<T>(ex, Lk.n, C.cmap.p, e, x, g);
+    } else {
+        k_prolong_add_to<T>(ex, Lk.n, C.cmap.p, e, cur, x, g);
+        cur = x;
     }
     if (profOut) UNAP_CK(cudaEventRecordWithFlags((*profOut)[(size_t)k], ex.s, cudaEventRecordExternal));
+    return cur;
 }
 
 template <class T>
@@ -720,8 +748,7 @@ void AmgHierarchy::vcycle(const Exec& ex, const double* r, double* z, Gate g)
     if (params.precision == 1) {
         // a Chebyshev finest level converts r inside its first step
         if (!isCheby(0)) k_d2f(ex, lv[0].n, r, lv[0].bf.p);
-        vcycle_level<float>(ex, 0, g);
-        k_f2d(ex, lv[0].n, lv[0].xf.p, z);
+        k_f2d(ex, lv[0].n, vcycle_level<float>(ex, 0, g), z);
     } else {
         vcycle_level<double>(ex, 0, g);
     }
@@ -742,17 +769,16 @@ static double time_smoother(AmgHierarchy& H, cudaStream_t s, int k, int reps, do
     k_fill<T>(ex, V.n, b.p, T(1));
     k_fill<T>(ex, V.n, w.p, T(0));
     const bool cheb = H.isCheby(k);
+    FlowRing ring;
+    if (!cheb && H.flows(k)) ring.init((size_t)V.n, sizeof(T), 1);
     auto run = [&]() {
         if (cheb)
             k_cheb_step<T>(ex, R, x.p, t.p, b.p, w.p, (T)V.d1[1 % H.params.chebyDegree],
                            (T)V.d2[1 % H.params.chebyDegree], 0, Gate{});
-        else if (V.pack.rec.p && packed_sweeps() != 0 && R.wide)
-            gs_sweep_packed<T>(ex, Lk, V.pack, R.diag, x.p, b.p, false, false,
-                               packed_sweeps() == 3 ||
-                                   (packed_sweeps() == 1 && 2.0 * Lk.nf > 12.5 * Lk.n),
-                               Gate{});
+        else if (H.flows(k))
+            flow_gs<T>(ex, Lk, R, ring, x.p, b.p, 1, false, false, nullptr, nullptr, Gate{});
         else
-            gs_sweep<T>(ex, Lk, R, x.p, b.p, false, false, Gate{});
+            H.sweep<T>(ex, k, Lk, R, x.p, b.p, false, false, Gate{});
     };
     run();
     cudaEvent_t e0, e1;
@@ -766,9 +792,10 @@ static double time_smoother(AmgHierarchy& H, cudaStream_t s, int k, int reps, do
     UNAP_CK(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    ring.check();
     if (bytes)
         *bytes = cheb ? cheb_bytes(V.n, Lk.nf, fp32, true) : sweep_bytes(V.n, V.n, Lk.nf, fp32);
-    if (launches) *launches = cheb ? 1 : Lk.nWave;
+    if (launches) *launches = cheb || H.flows(k) ? 1 : Lk.nWave;
     return (double)ms / std::max(reps, 1);
 }
 
@@ -833,6 +860,7 @@ int AmgHierarchy::profile(cudaStream_t s, int reps, double* ms, int maxOut)
     UNAP_CK(cudaEventElapsedTime(&t, e0, e1));
     if (maxOut > 0) ms[0] = (double)t / std::max(reps, 1);
     UNAP_CK(cudaStreamSynchronize(s));
+    check();
     cudaGraphExecDestroy(ge);
     cudaGraphDestroy(gr);
     int written = 1;

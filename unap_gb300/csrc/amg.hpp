@@ -6,6 +6,7 @@
 
 #include "cheby.hpp"
 #include "engine.hpp"
+#include "flow.hpp"
 #include "tail.hpp"
 
 namespace unapgpu {
@@ -96,6 +97,7 @@ public:
         DevArray<float> xf, bf, rf;
         DevArray<double> t;  // second Chebyshev iterate (FP64 V-cycle)
         DevArray<float> tf;  // second Chebyshev iterate (FP32 V-cycle)
+        FlowRing sweeps;  // Gauss-Seidel sweeps of the V-cycle
         PackedRows pack;  // row-packed copy for the cluster tail (coarse levels)
         double lam = 0;   // Chebyshev: eigenvalue estimate and coefficients
         double Rth = 0, d1[kChebyMaxDegree] = {}, d2[kChebyMaxDegree] = {};
@@ -116,6 +118,22 @@ public:
         return params.smoother == 1 && k >= params.chebyFrom && k < nLevels() - 1;
     }
     std::vector<double> eigenvalues() const;
+    // throws when a wait of a sweep ran out (after synchronizing)
+    void check() const;
+
+    // Level k's sweeps are one launch each (flow_gs) in FP64 and on FP32
+    // levels of up to kFlowRows32 rows; above that an FP32 wavefront alone
+    // fills the GPU and launches per wavefront, chained by programmatic
+    // dependent launch, read the matrix faster (one sweep at 16,777,216 rows:
+    // 273 us by launches, 358 us in one; 7,760,664 rows: 294 and 305;
+    // 1,894,123 rows: 113 and 94; 453,513 rows: 88 and 54).  A forced form of
+    // the launches (set_packed_sweeps other than 1) applies to every level.
+    static constexpr int kFlowRows32 = 1 << 21;
+    bool flows(int k) const { return lv[(size_t)k].sweeps.sweeps > 0 && packed_sweeps() == 1; }
+    // launches per wavefront, in place on x
+    template <class T>
+    void sweep(const Exec& ex, int k, const Level& Lk, const Rows<T>& Rk, T* x, const T* b,
+               bool backward, bool xIsZero, Gate g);
 
 private:
     void setupCheby(cudaStream_t s);
@@ -126,13 +144,11 @@ private:
     template <class T>
     T* chebBuf(int k, int j);
     Matrix& A;
+    // returns the address of level k's result
     template <class T>
-    void vcycle_level(const Exec& ex, int k, Gate g);
+    const T* vcycle_level(const Exec& ex, int k, Gate g);
     template <class T>
     void launch_tail(const Exec& ex, int t, Gate g);
-    template <class T>
-    void sweep(const Exec& ex, int k, const Level& Lk, const Rows<T>& Rk, T* x, const T* b,
-               bool backward, bool xIsZero, Gate g);
     int curTail = -1;
     // first level of the Chebyshev cluster tail (launch_cheb_tail), -1: none
     int chebTail = -1;
@@ -159,6 +175,7 @@ public:
     {
         H.vcycle(ex, r, w, g);
     }
+    void check() const override { H.check(); }
     bool appendSteps(std::vector<Step>& out, std::vector<LevelRows>& lv, const double* r,
                      double* w, int, bool* dotFused) override
     {

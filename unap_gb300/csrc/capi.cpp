@@ -3,6 +3,7 @@
 // report failure through num_iterations = -1 / res_norm = NaN, the
 // unap_cuda_* calls return a negative status; the message is kept for
 // unap_cuda_last_error().
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -594,11 +595,15 @@ int unap_cuda_gauss_seidel(long int handle, double* x, const double* b, int nSwe
         k_to_internal<double>(ex, A.n(), A.L->d_perm.p, x, h->s1.p);
         k_to_internal<double>(ex, A.n(), A.L->d_perm.p, b, h->s2.p);
         Rows<double> R = rows64(*A.L);
-        for (int k = 0; k < nSweeps; ++k)
-            gs_sweep<double>(ex, *A.L, R, h->s1.p, h->s2.p, backward != 0, false, Gate{});
-        k_to_reference<double>(ex, A.n(), A.L->d_perm.p, h->s1.p, x);
+        // up to four sweeps a launch, each following the one before
+        const int per = std::min(nSweeps, 4);
+        if (h->sweeps.sweeps < per) h->sweeps.init((size_t)A.n(), sizeof(double), per);
+        const double* y = flow_gs<double>(ex, *A.L, R, h->sweeps, h->s1.p, h->s2.p, nSweeps,
+                                          backward != 0, false, nullptr, nullptr, Gate{});
+        k_to_reference<double>(ex, A.n(), A.L->d_perm.p, y, x);
         UNAP_CK(cudaGetLastError());
         UNAP_CK(cudaStreamSynchronize(A.stream));
+        h->sweeps.check();
     });
 }
 
@@ -667,9 +672,20 @@ extern "C" int unap_cuda_profile_kernels(long int handle, int reps, double* ms)
         if (L.sweepable) {
             ms[1] = timeit([&] { dic->apply(ex, a.p, b.p, nullptr, 0, nullptr, FIN_NONE, Gate{}); });
             ms[2] = timeit([&] { dilu->apply(ex, a.p, b.p, nullptr, 0, nullptr, FIN_NONE, Gate{}); });
-            ms[3] = timeit([&] { gs_sweep<double>(ex, L, R, b.p, a.p, false, false, Gate{}); });
-            ms[4] = timeit([&] { gs_sweep<double>(ex, L, R, b.p, a.p, true, false, Gate{}); });
-            ms[6] = timeit([&] { gs_sweep<float>(ex, L, R32, bf.p, af.p, false, false, Gate{}); });
+            FlowRing ring;
+            ring.init((size_t)n, sizeof(double), 1);
+            auto sweep = [&](bool backward) {
+                flow_gs<double>(ex, L, R, ring, b.p, a.p, 1, backward, false, nullptr, nullptr,
+                                Gate{});
+            };
+            ms[3] = timeit([&] { sweep(false); });
+            ms[4] = timeit([&] { sweep(true); });
+            ms[6] = timeit([&] {
+                flow_gs<float>(ex, L, R32, ring, bf.p, af.p, 1, false, false, nullptr, nullptr,
+                               Gate{});
+            });
+            UNAP_CK(cudaStreamSynchronize(ex.s));
+            ring.check();
         }
         ms[5] = timeit([&] { k_spmv<float>(ex, R32, af.p, bf.p, nullptr, RSpec{}, Gate{}); });
         ms[7] = timeit([&] { k_residual<double>(ex, R, a.p, b.p, c.p, RSpec{}, Gate{}); });

@@ -170,6 +170,7 @@ int unap_cuda_amg_vcycle(long int amg, const double* r, double* z)
         k_to_reference<double>(ex, n, A.L->d_perm.p, zi.p, z);
         UNAP_CK(cudaGetLastError());
         UNAP_CK(cudaStreamSynchronize(A.stream));
+        h->H->check();
     });
 }
 

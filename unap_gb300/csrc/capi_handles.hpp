@@ -4,6 +4,7 @@
 #include <memory>
 
 #include "engine.hpp"
+#include "flow.hpp"
 
 namespace unapgpu {
 
@@ -18,6 +19,7 @@ struct MatHandle {
     bool hasValues = false;
     std::unique_ptr<Matrix> M;
     DevArray<double> s1, s2;  // scratch for single-kernel entry points
+    FlowRing sweeps;          // and for Gauss-Seidel sweeps
     Matrix& get();
     int n() const;
     void setValues(const double* diag, const double* upper, const double* lower);

@@ -346,6 +346,7 @@ void Krylov::readState()
 {
     UNAP_CK(cudaMemcpyAsync(h_st, d_st, sizeof(KState), cudaMemcpyDeviceToHost, ex.s));
     UNAP_CK(cudaStreamSynchronize(ex.s));
+    P->check();
 }
 
 // PCG.cpp:97-180 with the vector work fused into four kernels (plus the

@@ -59,6 +59,8 @@ public:
     // its reciprocal diagonal in internal order, for whole-solve launches
     virtual int lduType() const { return -1; }
     virtual const double* lduRD() const { return nullptr; }
+    // throws when a wait of an apply() ran out (after synchronizing with it)
+    virtual void check() const {}
 };
 
 std::unique_ptr<Precond> make_ldu_precond(int type, Matrix& A);  // 1 Diag, 2 DIC, 3 DILU, else none

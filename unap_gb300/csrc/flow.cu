@@ -1,0 +1,435 @@
+// Wavefront sweeps as one launch (see flow.hpp).
+//
+// A sweep's rows are cut into tasks of at most 32 rows, one warp each: rows
+// of one SELL slice and of one wavefront, so a task's rows are independent.
+// Warps take tasks from a counter in dependency order (forward: ascending
+// rows, backward: descending).  A task's rows depend only on rows of tasks
+// taken before it, by warps that are running or done, so whatever part of
+// the grid is resident, the waits end: no co-residency is assumed.
+//
+// A row waits for its neighbours by value.  The output vector is filled with
+// 0xff bytes before the launch (a NaN that no row writes: a result with that
+// pattern is written as the default NaN), a row's value is one 4- or 8-byte
+// relaxed store, and a reader loads until it sees something else.  The store
+// carries its own flag, so no fence, barrier or launch stands between two
+// wavefronts: a dependent row costs one store-to-load hop through L2 (0.33
+// us) and its own arithmetic, where a launch per wavefront cost 3 to 6 us.
+// Old and new values live in different vectors, so no row overwrites what
+// another still reads, and several sweeps run in one launch, each following
+// the one before by its own waits.
+//
+// Every wait is bounded: after kSpinLimit polls, or once another wait of the
+// same ring gave up, it sets the ring's error word and goes on with what it
+// has; the host turns that into an error (FlowRing::check).
+#include <algorithm>
+
+#include "device_common.cuh"
+#include "flow.hpp"
+
+namespace unapgpu {
+
+namespace {
+
+constexpr int kFlowThreads = 128;
+constexpr int kStreams = kFlowThreads / 32;  // a task counter for each warp of a CTA
+static_assert(kFlowHeader >= kStreams * kFlowCounterBytes, "a counter per stream");
+constexpr int kSpinLimit = 1 << 23;  // polls; one is 0.3 us or more
+
+// ---- values that say whether they are there -------------------------------
+__device__ __forceinline__ float ld_flow(const float* p)
+{
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_flow(const double* p)
+{
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool absent(float v) { return __float_as_uint(v) == 0xffffffffu; }
+__device__ __forceinline__ bool absent(double v) { return __double_as_longlong(v) == -1ll; }
+__device__ __forceinline__ void st_flow(float* p, float v)
+{
+    if (absent(v)) v = __uint_as_float(0x7fffffffu);
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_flow(double* p, double v)
+{
+    if (absent(v)) v = __longlong_as_double(0x7ff8000000000000ll);
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+
+// One more poll of a wait: true when the wait has to be given up.
+__device__ __forceinline__ bool give_up(int& spins, int* err)
+{
+    if ((++spins & 0xfff) == 0) {
+        if (spins >= kSpinLimit) *(volatile int*)err = 1;
+        if (*(volatile int*)err) return true;
+    }
+    return false;
+}
+
+// Loads at(k) for the entries in `need` (one bit each) until every value is
+// there; all lanes of the warp call it.
+template <class T, int CK, class At>
+__device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], int* err)
+{
+    int spins = 0;
+    for (;;) {
+#pragma unroll
+        for (int k = 0; k < CK; ++k)
+            if (need >> k & 1u) v[k] = ld_flow(at(k));
+#pragma unroll
+        for (int k = 0; k < CK; ++k)
+            if ((need >> k & 1u) && !absent(v[k])) need &= ~(1u << k);
+        if (!__any_sync(0xffffffffu, need != 0)) return;
+        if (give_up(spins, err)) return;
+    }
+}
+
+// A task far ahead of the rows that are being computed would poll for long:
+// until a row two wavefronts before its own is there, the whole warp polls
+// that one address, with pauses.
+template <class T>
+__device__ __forceinline__ void wait_near(const T* p, int* err)
+{
+    int spins = 0;
+    while (absent(ld_flow(p))) {
+        __nanosleep(64);
+        if (give_up(spins, err)) return;
+    }
+}
+
+// The next task of this warp.  Warp w of every CTA takes the tasks w, w +
+// kStreams, ... from a counter of its own (starting at -1).  As every CTA
+// serves every counter, whichever CTAs are resident, no task is left behind.
+// One counter hands out a task every 0.65 ns at best, and eight that share
+// an L2 slice no more (0.60 ns, 32 bytes apart); 4 KB apart they give one
+// every 0.09 ns.
+__device__ __forceinline__ int take(unsigned* counters)
+{
+    const unsigned w = threadIdx.x >> 5;
+    int t = 0;
+    if ((threadIdx.x & 31) == 0)
+        t = (int)((atomicAdd(counters + (kFlowCounterBytes / 4) * w, 1u) + 1u) * kStreams + w);
+    return t;
+}
+
+template <class T>
+struct GsArgs {
+    Rows<T> A;
+    const int4* task;
+    const int2* near;
+    int nTasks, nSweeps, firstFromZero;
+    const T* in;
+    T* out;         // sweep s writes out + s * stride ...
+    long long stride;
+    T* last;        // ... and the last one here
+    T* copy;        // and here, or null
+    const T* b;
+    unsigned* counter;
+    int* err;
+};
+
+// G lanes a row, K entries a lane, so that a row is loaded whole before its
+// turn and its neighbours are asked for at once; with G > 1 the products meet
+// in shared memory and one lane takes their ordered sum (a chain of FP64
+// additions of 32 ns each on this GPU).  Lane i + (32 / G) g of the warp
+// holds entries g, g + G, ... of row i of the task: the lanes of one g read
+// consecutive rows.
+template <class T, int G, int K, bool BWD>
+__global__ void __launch_bounds__(kFlowThreads)
+    flow_gs_kernel(const __grid_constant__ GsArgs<T> a, Gate gate)
+{
+    if (gate_closed(gate)) return;
+    constexpr int RW = 32 / G;      // rows of a task
+    constexpr int W = G * K;        // entries of a row held at once
+    constexpr int P = W + 1;        // row pitch of the products
+    __shared__ T prod[kFlowThreads / 32][G == 1 ? 1 : RW * P];
+    T* pw = prod[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int row = lane % RW, g = lane / RW;
+    const int total = a.nTasks * a.nSweeps;
+    for (;;) {
+        const int t = __shfl_sync(0xffffffffu, take(a.counter), 0);
+        if (t >= total) return;
+        const int s = a.nSweeps == 1 ? 0 : t / a.nTasks;
+        int q = t - s * a.nTasks;
+        if (BWD) q = a.nTasks - 1 - q;
+        const int4 D = ldg(a.task + q);
+        const int2 nr = ldg(a.near + q);
+        const int r = D.x + row;
+        const bool on = row < D.y;
+        T* out = s == a.nSweeps - 1 ? a.last : a.out + s * a.stride;
+        const T* in = s == 0 ? a.in : a.out + (s - 1) * a.stride;
+        const int base = D.z + row;
+        int info = 0;
+        T d = T(1), acc = T(0);
+        if (on) {
+            info = ldg(a.A.rowInfo + r);
+            d = ldg(a.A.diag + r);
+            acc = __ldcg(a.b + r);
+        }
+        int c[K];
+        T v[K], xv[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const bool has = on && k * G + g < D.w;
+            c[k] = has ? ldg(a.A.col + base + 32 * (k * G + g)) : 0;
+            v[k] = has ? ldg(a.A.val + base + 32 * (k * G + g)) : T(0);
+        }
+        const int nLow = info >> 16;
+        const int jEnd = !BWD && s == 0 && a.firstFromZero ? nLow : info & 0xffff;
+        if ((BWD ? nr.y : nr.x) >= 0) wait_near(out + (BWD ? nr.y : nr.x), a.err);
+        for (int j0 = 0;;) {
+            unsigned need = 0;
+            auto at = [&](int k) {
+                const int j = j0 + k * G + g;
+                return ((BWD ? j >= nLow : j < nLow) ? (const T*)out : in) + c[k];
+            };
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int j = j0 + k * G + g;
+                xv[k] = T(0);
+                if (j < jEnd) {
+                    if ((BWD ? j >= nLow : j < nLow) || s > 0)
+                        need |= 1u << k;
+                    else
+                        xv[k] = *at(k);
+                }
+            }
+            wait_values<T, K>(need, at, xv, a.err);
+            if (G == 1) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) xv[k] = v[k] * xv[k];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    if (j0 + k >= D.w) break;
+                    const T less = acc - xv[k];
+                    acc = j0 + k < jEnd ? less : acc;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; ++k) pw[row * P + k * G + g] = v[k] * xv[k];
+                __syncwarp();
+            }
+            if (G > 1 && g == 0) {
+                // the reference's order: entry after entry
+                const int m = min(jEnd - j0, W);
+                const T* p = pw + row * P;
+                int j = 0;
+                for (; j + 4 <= m; j += 4) {
+                    const T p0 = p[j], p1 = p[j + 1], p2 = p[j + 2], p3 = p[j + 3];
+                    acc -= p0;
+                    acc -= p1;
+                    acc -= p2;
+                    acc -= p3;
+                }
+                for (; j < m; ++j) acc -= p[j];
+            }
+            if (G > 1) __syncwarp();
+            j0 += W;
+            if (j0 >= D.w || !__any_sync(0xffffffffu, j0 < jEnd)) break;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int j = j0 + k * G + g;
+                c[k] = j < jEnd ? ldg(a.A.col + base + 32 * j) : 0;
+                v[k] = j < jEnd ? ldg(a.A.val + base + 32 * j) : T(0);
+            }
+        }
+        if (on && g == 0) {
+            acc = acc / d;
+            st_flow(out + r, acc);
+            if (a.copy && s == a.nSweeps - 1) a.copy[r] = acc;  // as above
+        }
+    }
+}
+
+void tick()
+{
+    if (!capturing()) count_launches(1);
+}
+
+int sm_count()
+{
+    static int cached = 0;
+    if (!cached) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        cached = n > 0 ? n : 152;
+    }
+    return cached;
+}
+
+// fills in where a task's slice starts and how many entries its rows hold
+__global__ void task_slices_kernel(int n, const int* __restrict__ sliceOff, int4* task)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int r = task[i].x;
+    const int o = sliceOff[r >> 5];
+    task[i].z = o + (r & 31);
+    task[i].w = (sliceOff[(r >> 5) + 1] - o) / 32;
+}
+
+// Lanes a row of a Gauss-Seidel sweep.  A row is one ordered sum: with a lane
+// a row its entries' loads wait for one another in chunks, with more lanes
+// they are all in flight at once, but a warp holds fewer rows.  Rows of 8 or
+// fewer entries fit one lane.  One sweep of the levels of a 128^3 Laplacian's
+// hierarchy, us at 1 / 4 / 8 lanes: FP64, 453,513 rows 127 / 184 / -, 215,841
+// rows 161 / 151 / 184, 103,381 rows 166 / 147 / 123, 23,973 rows 149 / 119 /
+// 96, 2,718 rows 127 / 95 / 69; FP32, 965,724 rows 55 / 86 / -, 453,513 rows
+// 67 / 54 / -, 103,381 rows 93 / 54 / 70, 23,973 rows 86 / 53 / 64.
+int sweep_lanes(int n, double len, bool fp64)
+{
+    if (len <= 8.5) return 1;
+    if (fp64 && n <= 150000) return 8;
+    return n <= (fp64 ? 300000 : 600000) ? 4 : 1;
+}
+
+int flow_grid(long long tasks)
+{
+    constexpr int W = kFlowThreads / 32;
+    return (int)std::max(1LL, std::min((tasks + W - 1) / W, 12LL * sm_count()));
+}
+
+}  // namespace
+
+FlowRing::FlowRing(FlowRing&& o) noexcept
+    : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), err(o.err)
+{
+    o.err = nullptr;
+}
+
+FlowRing::~FlowRing() { pinned_block_free(err); }
+
+void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves)
+{
+    sweeps = std::max(1, std::min(sweepsPerHalf, kFlowMaxSweeps));
+    stride = (n * elemBytes + 255) / 256 * 256;
+    half = kFlowHeader + stride * (size_t)sweeps;
+    mem.alloc((size_t)halves * half);
+    if (!err) err = static_cast<int*>(pinned_block_alloc(64));
+    *err = 0;
+}
+
+int FlowRing::other(const void* p) const
+{
+    const unsigned char* q = static_cast<const unsigned char*>(p);
+    return q >= mem.p && q < mem.p + half ? 1 : 0;
+}
+
+void FlowRing::check() const
+{
+    if (err && *(volatile int*)err) {
+        *(volatile int*)err = 0;
+        throw CudaError("wavefront sweep: a wait for a neighbouring row ran out");
+    }
+}
+
+void flow_tasks(Level& L, cudaStream_t s)
+{
+    if (!L.sweepable) return;
+    const double len = L.n ? 2.0 * L.nf / L.n : 0.0;
+    for (SweepTasks& S : L.tasks) {
+        if (S.lanes > 1 && S.lanes != sweep_lanes(L.n, len, true) &&
+            S.lanes != sweep_lanes(L.n, len, false))
+            continue;
+        const int rows = 32 / S.lanes;
+        std::vector<int4> t;
+        std::vector<int2> near;
+        t.reserve((size_t)(L.n / rows + L.nWave + 2));
+        near.reserve(t.capacity());
+        for (int w = 0; w < L.nWave; ++w) {
+            const int r0 = L.waveStart[(size_t)w], r1 = L.waveStart[(size_t)w + 1];
+            // a row at the same relative place of wavefront v
+            auto beside = [&](int v, int r) {
+                if (v < 0 || v >= L.nWave) return -1;
+                const int a = L.waveStart[(size_t)v], m = L.waveStart[(size_t)v + 1] - a;
+                return m > 0 ? a + (int)((long long)(r - r0) * m / (r1 - r0)) : -1;
+            };
+            for (int r = r0; r < r1;) {
+                const int e = std::min(r1, (r / rows + 1) * rows);
+                t.push_back(make_int4(r, e - r, 0, 0));
+                near.push_back(make_int2(beside(w - 2, r), beside(w + 2, r)));
+                r = e;
+            }
+        }
+        S.n = (int)t.size();
+        S.task.upload(t, s);
+        S.near.upload(near, s);
+        if (S.n) {
+            task_slices_kernel<<<div_up(S.n, 256), 256, 0, s>>>(S.n, L.d_sliceOff.p, S.task.p);
+            UNAP_CK(cudaGetLastError());
+        }
+        UNAP_CK(cudaStreamSynchronize(s));
+    }
+}
+
+template <class T, bool BWD>
+static void launch_gs(const Exec& ex, int wide, int lanes, const GsArgs<T>& a, Gate g)
+{
+    const int grid = flow_grid((long long)a.nTasks * a.nSweeps);
+    if (lanes == 8)
+        flow_gs_kernel<T, 8, 4, BWD><<<grid, kFlowThreads, 0, ex.s>>>(a, g);
+    else if (lanes == 4)
+        flow_gs_kernel<T, 4, 6, BWD><<<grid, kFlowThreads, 0, ex.s>>>(a, g);
+    else if (wide)
+        flow_gs_kernel<T, 1, 16, BWD><<<grid, kFlowThreads, 0, ex.s>>>(a, g);
+    else
+        flow_gs_kernel<T, 1, 8, BWD><<<grid, kFlowThreads, 0, ex.s>>>(a, g);
+}
+
+template <class T>
+T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& ring, const T* in,
+           const T* b, int nSweeps, bool backward, bool xIsZero, T* last, T* copy, Gate g)
+{
+    const int lanes = L.n ? sweep_lanes(L.n, 2.0 * L.nf / L.n, sizeof(T) == 8) : 1;
+    const SweepTasks& S = L.tasks[lanes == 8 ? 2 : lanes == 4 ? 1 : 0];
+    T* cur = const_cast<T*>(in);
+    const size_t vecBytes = (size_t)L.n * sizeof(T);
+    for (int done = 0; done < nSweeps;) {
+        const int h = ring.other(cur);
+        const int m = std::min(nSweeps - done, ring.sweeps);
+        const bool end = done + m == nSweeps;
+        GsArgs<T> a;
+        a.A = A;
+        a.task = S.task.p;
+        a.near = S.near.p;
+        a.nTasks = S.n;
+        a.nSweeps = m;
+        a.firstFromZero = done == 0 && xIsZero ? 1 : 0;
+        a.in = cur;
+        a.out = reinterpret_cast<T*>(ring.vec(h, 0));
+        a.stride = (long long)(ring.stride / sizeof(T));
+        a.last = end && last ? last : reinterpret_cast<T*>(ring.vec(h, m - 1));
+        a.copy = end ? copy : nullptr;
+        a.b = b;
+        a.counter = ring.counter(h);
+        a.err = ring.err;
+        const int own = end && last ? m - 1 : m;  // vectors of the ring this launch writes
+        UNAP_CK(cudaMemsetAsync(ring.counter(h), 0xff, kFlowHeader + ring.stride * (size_t)own, ex.s));
+        if (own < m) UNAP_CK(cudaMemsetAsync(last, 0xff, vecBytes, ex.s));
+        tick();
+        if (backward)
+            launch_gs<T, true>(ex, A.wide, lanes, a, g);
+        else
+            launch_gs<T, false>(ex, A.wide, lanes, a, g);
+        UNAP_CK(cudaGetLastError());
+        cur = a.last;
+        done += m;
+    }
+    return cur;
+}
+
+template float* flow_gs<float>(const Exec&, const Level&, const Rows<float>&, const FlowRing&,
+                               const float*, const float*, int, bool, bool, float*, float*,
+                               Gate);
+template double* flow_gs<double>(const Exec&, const Level&, const Rows<double>&, const FlowRing&,
+                                 const double*, const double*, int, bool, bool, double*, double*,
+                                 Gate);
+
+}  // namespace unapgpu

@@ -1,0 +1,53 @@
+// Wavefront sweeps as one launch (implemented in flow.cu): Gauss-Seidel
+// sweeps of a level, with its rows as warp tasks taken in dependency order.
+#pragma once
+
+#include "kernels.hpp"
+
+namespace unapgpu {
+
+// Most sweeps of one flow_gs launch.
+constexpr int kFlowMaxSweeps = 16;
+// Task counters at the head of a half: four, this far apart.
+constexpr int kFlowCounterBytes = 4096;
+constexpr int kFlowHeader = 4 * kFlowCounterBytes;
+
+// Storage of one level's sweeps: one or two halves of `sweeps` vectors of n
+// elements, each half headed by the task counters of the launch that writes
+// it.  A launch reads its input from one half (or from elsewhere) and writes
+// the other; the written half is filled with 0xff bytes first.
+struct FlowRing {
+    DevArray<unsigned char> mem;
+    size_t stride = 0;   // bytes of one vector
+    size_t half = 0;     // bytes of one half
+    int sweeps = 0;      // vectors of one half
+    int* err = nullptr;  // pinned: set by a launch whose wait ran out
+    FlowRing() = default;
+    FlowRing(const FlowRing&) = delete;
+    FlowRing& operator=(const FlowRing&) = delete;
+    FlowRing(FlowRing&& o) noexcept;
+    ~FlowRing();
+    void init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves = 2);
+    size_t bytes() const { return mem.bytes(); }
+    // the half (0 or 1) that does not hold p
+    int other(const void* p) const;
+    unsigned* counter(int h) const { return reinterpret_cast<unsigned*>(mem.p + h * half); }
+    unsigned char* vec(int h, int i) const { return mem.p + h * half + kFlowHeader + i * stride; }
+    // throws when a wait of one of this ring's launches ran out (call after
+    // synchronizing with them)
+    void check() const;
+};
+
+// nSweeps Gauss-Seidel sweeps (forward, or backward in reverse cell order)
+// from `in`; xIsZero: in is zero (forward, the first sweep then reads only
+// its lower side, in may be null).  Returns the result's address: `last`
+// where it is given (n elements, not `in`), else one of the ring's vectors.
+// copy (optional, may be `in`): the result is written there too.
+template <class T>
+T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& ring, const T* in,
+           const T* b, int nSweeps, bool backward, bool xIsZero, T* last, T* copy, Gate g);
+
+// the level's task table, built with the level (build_level)
+void flow_tasks(Level& L, cudaStream_t s);
+
+}  // namespace unapgpu

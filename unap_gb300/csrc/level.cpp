@@ -4,7 +4,7 @@
 #include <cstring>
 #include <numeric>
 
-#include "unap_internal.hpp"
+#include "flow.hpp"
 
 namespace unapgpu {
 
@@ -30,7 +30,8 @@ size_t Level::deviceBytes() const
 {
     return d_perm.bytes() + d_iperm.bytes() + d_sliceOff.bytes() + d_rowInfo.bytes() +
            d_col.bytes() + d_val.bytes() + d_valT.bytes() + d_diag.bytes() + d_val32.bytes() +
-           d_diag32.bytes();
+           d_diag32.bytes() + tasks[0].bytes() + tasks[1].bytes() +
+           tasks[2].bytes();
 }
 
 namespace {
@@ -89,6 +90,7 @@ std::unique_ptr<Level> build_level(const HostLdu& A, const std::vector<int>* key
         A.n >= minCells) {
         if (auto D = build_level_device(A, key, s, wavefronts)) {
             D->version = next_version();
+            flow_tasks(*D, s);
             return D;
         }
     }
@@ -252,6 +254,7 @@ std::unique_ptr<Level> build_level(const HostLdu& A, const std::vector<int>* key
     L->d_col.upload(col, s);
     UNAP_CK(cudaStreamSynchronize(s));  // host vectors die here
     update_level_values(*L, A, s);
+    if (!identityOrder) flow_tasks(*L, s);
     return L;
 }
 

@@ -1,4 +1,5 @@
 // The reference's MGSolver on the device (see mg.hpp).
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -288,9 +289,14 @@ void MgSolver::smooth(int slot, int k, double* xk, const double* bk, int nSweeps
         }
         return;
     }
-    const Level& L = *lv[(size_t)k].L;
-    Rows<double> R = rows64(L);
-    for (int s = 0; s < nSweeps; ++s) gs_sweep<double>(ex, L, R, xk, bk, false, false, Gate{});
+    // all of a level's sweeps in one launch (a coarse level c takes nPost + c
+    // of them), each following the one before at a wavefront's distance
+    Lv& K = lv[(size_t)k];
+    const Level& L = *K.L;
+    const int per = std::min(nSweeps, kFlowMaxSweeps);
+    if (K.sweeps.sweeps < per) K.sweeps.init((size_t)K.n, sizeof(double), per);
+    flow_gs<double>(ex, L, rows64(L), K.sweeps, xk, bk, nSweeps, false, false, nullptr, xk,
+                    Gate{});
 }
 
 void MgSolver::scaling(int k, double* field, const double* source, double* Acf, int sfSlot)
@@ -399,6 +405,7 @@ SolveStats MgSolver::solveDevice(double* x_ref, const double* b_ref)
             UNAP_CK(cudaGetLastError());
             UNAP_CK(cudaMemcpyAsync(h_st, d_st, sizeof(KState), cudaMemcpyDeviceToHost, ex.s));
             UNAP_CK(cudaStreamSynchronize(ex.s));
+            for (auto& K : lv) K.sweeps.check();
             if (h_st->done) break;
         }
     } else {

@@ -6,6 +6,7 @@
 
 #include "amg.hpp"
 #include "cheby.hpp"
+#include "flow.hpp"
 #include "small_solve.hpp"
 
 namespace unapgpu {
@@ -47,6 +48,7 @@ private:
         DevArray<int> childStart, child, cmap;  // transfer into this level (k >= 1)
         DevArray<double> corr, src, acf, pre, rD, w, p;
         DevArray<double> dfac, pfac;  // coarsest DIC/DILU factor
+        FlowRing sweeps;              // Gauss-Seidel sweeps
     };
     Matrix& A;
     std::vector<Lv> lv;  // lv[0] finest, lv[k] coarse level k-1 of the reference

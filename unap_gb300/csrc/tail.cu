@@ -19,13 +19,14 @@ namespace unapgpu {
 
 namespace {
 
-// per V-cycle precision (0 FP64, 1 FP32), measured on the 256^3 log-normal
-// hierarchy: FP32 per-wavefront launches of the row-packed sweep (with
-// programmatic dependent launch) beat the cluster tail on every level, so it
-// is off; FP64 launches are slower and the tail still wins from ~100k rows
 std::atomic<int> g_packedSweeps{1};
 
-std::atomic<long long> g_tailRows[2] = {{1ll << 21}, {8192}};
+// per V-cycle precision (0 FP64, 1 FP32), Gauss-Seidel levels of a 128^3
+// Laplacian, two sweeps before and after.  FP64: one launch per sweep
+// (flow_gs) beats the tail on every level (V-cycle 4.61 ms without it, 5.79
+// with it up to 2^21 rows), so it is off; FP32: the tail still wins up to
+// 8,192 rows (2.36 ms against 2.42 without it)
+std::atomic<long long> g_tailRows[2] = {{0}, {8192}};
 std::atomic<long long> g_singleRows[2] = {{8192}, {8192}};
 
 constexpr int kStaticSmem =

@@ -233,6 +233,19 @@ struct HostLdu {
     void validate();
 };
 
+// Rows of a sweep in tasks of one warp: task t is task[t].y rows from
+// task[t].x on, of one SELL slice and one wavefront; their entry 0 starts at
+// task[t].z and they hold up to task[t].w entries.  near[t] names a row two
+// wavefronts before (x, forward sweeps) and after (y, backward), or -1.
+struct SweepTasks {
+    int lanes;  // lanes a row: tasks of up to 32 / lanes rows
+    int n = 0;
+    DevArray<int4> task;
+    DevArray<int2> near;
+    SweepTasks(int l) : lanes(l) {}
+    size_t bytes() const { return task.bytes() + near.bytes(); }
+};
+
 // Per-matrix topology on the device (shared by FP64 and FP32 values).
 struct Level {
     int n = 0, nf = 0;
@@ -251,6 +264,8 @@ struct Level {
     int maxRowLen = 0;
     DevArray<int> d_perm, d_iperm;
     DevArray<int> d_sliceOff, d_rowInfo, d_col;
+    // sweeps (flow.hpp), sweepable levels only
+    SweepTasks tasks[3] = {1, 4, 8};
     // FP64 values
     DevArray<double> d_val, d_valT, d_diag;
     // FP32 values (mixed precision); filled on demand
