@@ -1,4 +1,4 @@
-"""Gauss-Seidel sweeps in one launch: rows wait for their neighbours by value.
+"""Gauss-Seidel sweeps and DIC/DILU in one launch: rows wait for their neighbours by value.
 
 Bit-identical to the oracle's sweeps (the same entry order and roundings, so
 the tolerance is zero) at the sizes where the launch can go wrong: single
@@ -59,6 +59,19 @@ def test_sweeps_bit_exact(cuda, orc, name, backward):
     A.close()
 
 
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_preconditioners_bit_exact(cuda, orc, name):
+    torch = cuda
+    s = CASES[name]()
+    A = capi.DeviceMatrix(s)
+    r = np.random.default_rng(s.n + 1).standard_normal(s.n)
+    for t in (2, 3):
+        w = torch.zeros(s.n, dtype=torch.float64, device="cuda")
+        A.precondition(t, torch.tensor(r, device="cuda"), w)
+        assert np.array_equal(w.cpu().numpy(), orc.precond(t, s, r)[0], equal_nan=True), t
+    A.close()
+
+
 @pytest.mark.parametrize("pattern", [0xFFFFFFFFFFFFFFFF, 0x7FF8000000000000, 0x7FF0000000000000])
 def test_nan_and_inf_inputs(cuda, orc, pattern):
     """A NaN that looks like a missing value, another NaN and an infinity
@@ -74,4 +87,7 @@ def test_nan_and_inf_inputs(cuda, orc, pattern):
         x = torch.tensor(x0, device="cuda")
         A.gauss_seidel(x, torch.tensor(b, device="cuda"), 2)
         assert np.array_equal(x.cpu().numpy(), orc.gs(s, x0, b, 2), equal_nan=True)
+        if where == "b":
+            A.precondition(2, torch.tensor(b, device="cuda"), x)
+            assert np.array_equal(x.cpu().numpy(), orc.precond(2, s, b)[0], equal_nan=True)
     A.close()

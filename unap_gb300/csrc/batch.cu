@@ -20,6 +20,7 @@
 
 #include "batch.hpp"
 #include "device_common.cuh"
+#include "flow.hpp"
 
 namespace unapgpu {
 
@@ -211,16 +212,17 @@ const double* BatchSolver::factor(Matrix& A, int precond)
     if (it != factors.end() && it->second.version == A.L->version) return it->second.rD.p;
     Fac f;
     f.version = A.L->version;
-    f.rD.alloc((size_t)A.n());
     if (precond == 1) {
         std::vector<double> h((size_t)A.n());
         for (int i = 0; i < A.n(); ++i) h[(size_t)i] = 1.0 / A.host.diag[(size_t)A.L->perm[(size_t)i]];
         f.rD.upload(h, stream);
     } else {
-        DevArray<double> dfac((size_t)A.n());
-        Exec ex{stream, device_max_blocks()};
-        dic_factor(ex, *A.L, precond == 3, dfac.p, f.rD.p);
+        DicFlow D;
+        D.init(*A.L);
+        flow_dic_factor(Exec{stream, device_max_blocks()}, *A.L, precond == 3, D);
         UNAP_CK(cudaStreamSynchronize(stream));
+        D.check();
+        f.rD = std::move(D.rD);
     }
     UNAP_CK(cudaStreamSynchronize(stream));
     auto& slot = factors[k];

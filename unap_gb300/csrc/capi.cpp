@@ -577,6 +577,7 @@ int unap_cuda_precondition(long int handle, int precond, const double* r, double
         k_to_reference<double>(ex, A.n(), A.L->d_perm.p, h->s2.p, w);
         UNAP_CK(cudaGetLastError());
         UNAP_CK(cudaStreamSynchronize(A.stream));
+        P->check();
     });
 }
 

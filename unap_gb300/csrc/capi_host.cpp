@@ -261,12 +261,15 @@ int unap_cuda_precond_rD(long int handle, int precond, double* rD)
         if (!A.L->sweepable)
             throw std::invalid_argument("DIC/DILU need faces oriented lowerAddr < upperAddr and sorted by owner");
         Exec ex{A.stream, device_max_blocks()};
-        DevArray<double> dfac((size_t)n), ri((size_t)n), ro((size_t)n);
-        dic_factor(ex, *A.L, precond == 3, dfac.p, ri.p);
-        k_to_reference<double>(ex, n, A.L->d_perm.p, ri.p, ro.p);
+        DevArray<double> ro((size_t)n);
+        DicFlow D;
+        D.init(*A.L);
+        flow_dic_factor(ex, *A.L, precond == 3, D);
+        k_to_reference<double>(ex, n, A.L->d_perm.p, D.rD.p, ro.p);
         UNAP_CK(cudaMemcpyAsync(rD, ro.p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost,
                                 A.stream));
         UNAP_CK(cudaStreamSynchronize(A.stream));
+        D.check();
     });
 }
 

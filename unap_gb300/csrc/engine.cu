@@ -12,6 +12,7 @@
 
 #include "engine.hpp"
 #include "batch.hpp"
+#include "flow.hpp"
 
 namespace unapgpu {
 
@@ -205,21 +206,19 @@ public:
             throw std::invalid_argument(
                 "DIC/DILU need faces oriented lowerAddr < upperAddr and sorted by owner, "
                 "and a matrix built with wavefronts");
-        Exec ex;
-        ex.s = A.stream;
-        ex.maxBlocks = device_max_blocks();
-        dfac.alloc((size_t)L.n);
-        rD.alloc((size_t)L.n);
-        dic_factor(ex, L, dilu, dfac.p, rD.p);
-        UNAP_CK(cudaGetLastError());
+        Exec ex{A.stream, device_max_blocks()};
+        D.init(L);
+        flow_dic_factor(ex, L, dilu, D);
         UNAP_CK(cudaStreamSynchronize(A.stream));
+        D.check();
     }
     bool fusesDot() const override { return true; }
     void apply(const Exec& ex, const double* r, double* w, const RedPool* pool, int site,
                KState* st, int fin, Gate g) override
     {
-        dic_apply(ex, L, dilu, rD.p, r, w, pool, site, st, fin, g);
+        flow_dic_apply(ex, L, D, r, w, pool, site, st, fin, g);
     }
+    void check() const override { D.check(); }
     bool appendSteps(std::vector<Step>& out, std::vector<LevelRows>& lv, const double* r,
                      double* w, int slot, bool* dotFused) override
     {
@@ -234,7 +233,7 @@ public:
             s.r1 = L.waveStart[k + 1];
             s.a = r;
             s.c = w;
-            s.e = rD.p;
+            s.e = D.rD.p;
             s.d = dilu ? A.val : A.valT;
             // DIC/DILU apply: 40 N + 32 F over both sweeps, half each
             s.bytes = 0.5 * ((s.r1 - s.r0) * 40.0 + (double)(s.r1 - s.r0) / L.n * L.nf * 32.0);
@@ -249,7 +248,7 @@ public:
             s.r1 = L.waveStart[k + 1];
             s.a = r;
             s.c = w;
-            s.e = rD.p;
+            s.e = D.rD.p;
             s.red = slot;
             s.f0 = firstBwd ? 0 : 1;
             firstBwd = false;
@@ -261,10 +260,10 @@ public:
         return true;
     }
     int lduType() const override { return dilu ? 3 : 2; }
-    const double* lduRD() const override { return rD.p; }
+    const double* lduRD() const override { return D.rD.p; }
     const Level& L;
     bool dilu;
-    DevArray<double> dfac, rD;
+    DicFlow D;
 };
 
 }  // namespace
@@ -346,7 +345,7 @@ void Krylov::readState()
 {
     UNAP_CK(cudaMemcpyAsync(h_st, d_st, sizeof(KState), cudaMemcpyDeviceToHost, ex.s));
     UNAP_CK(cudaStreamSynchronize(ex.s));
-    P->check();
+    if (P) P->check();
 }
 
 // PCG.cpp:97-180 with the vector work fused into four kernels (plus the

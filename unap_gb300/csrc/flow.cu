@@ -247,6 +247,177 @@ __global__ void __launch_bounds__(kFlowThreads)
     }
 }
 
+// d_c = D_c - sum over lower-side faces (asc) of (c1 c2) / d_l
+// (lduDICPrecond.cpp:15-42, lduDILUPrecond.cpp:15-43), rD = 1 / d, and every
+// entry times its row's rD: the first product of the sweeps' rD coef w, taken
+// once here instead of in every application (7 FP64 operations a 7-point row
+// and sweep instead of 10, on a pipe of 0.525 T operations/s).  c2 is also
+// the lower-side coefficient of the forward sweep.
+template <int CK>
+__global__ void __launch_bounds__(kFlowThreads)
+    flow_factor_kernel(Rows<double> A, const int4* task, const int2* near, int nTasks,
+                       const double* c1, const double* c2, double* d, double* rD, double* f,
+                       unsigned* counter, int* err)
+{
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        const int q = __shfl_sync(0xffffffffu, take(counter), 0);
+        if (q >= nTasks) return;
+        const int4 D = ldg(task + q);
+        const int wait = ldg(near + q).x;
+        const int r = D.x + lane;
+        const bool on = lane < D.y;
+        const int base = D.z + lane;
+        int len = 0, nLow = 0;
+        double acc = 1.0;
+        if (on) {
+            const int info = ldg(A.rowInfo + r);
+            len = info & 0xffff;
+            nLow = info >> 16;
+            acc = ldg(A.diag + r);
+        }
+        const int most = __reduce_max_sync(0xffffffffu, nLow);
+        for (int j0 = 0; j0 < most; j0 += CK) {
+            int c[CK];
+            double v[CK], xv[CK];
+            unsigned need = 0;
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                const int e = base + 32 * (j0 + k);
+                const bool has = j0 + k < nLow;
+                c[k] = has ? ldg(A.col + e) : 0;
+                v[k] = has ? ldg(c1 + e) * ldg(c2 + e) : 0.0;
+                xv[k] = 1.0;
+                if (has) need |= 1u << k;
+            }
+            if (j0 == 0 && wait >= 0) wait_near(d + wait, err);
+            wait_values<double, CK>(need, [&](int k) { return (const double*)d + c[k]; }, xv, err);
+#pragma unroll
+            for (int k = 0; k < CK; ++k)
+                if (j0 + k < most) xv[k] = v[k] / xv[k];
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                if (j0 + k >= most) break;
+                const double less = acc - xv[k];
+                acc = j0 + k < nLow ? less : acc;
+            }
+        }
+        if (on) {
+            st_flow(d + r, acc);
+            const double rd = 1.0 / acc;
+            rD[r] = rd;
+            for (int j = 0; j < len; ++j) {
+                const int e = base + 32 * j;
+                f[e] = rd * (j < nLow ? ldg(c2 + e) : ldg(A.val + e));
+            }
+        }
+    }
+}
+
+struct DicArgs {
+    Rows<double> A;
+    const int4* task;
+    const int2* near;
+    int nTasks;
+    const double* f;
+    const double* rD;
+    const double* r;
+    double* wf;    // forward sweep's vector
+    double* w;
+    double* part;  // partial of w.r per task, or null
+    unsigned* counter;
+    int* err;
+};
+
+// w = M^-1 r (lduDICPrecond.cpp:45-77, lduDILUPrecond.cpp:46-86): the forward
+// sweep's tasks, then the backward sweep's.  forward: wf_c = rD_c r_c, then
+// wf_c -= (rD_c coef) wf_l over the lower entries in face order; backward:
+// w_c = wf_c, then w_c -= (rD_c upper) w_u over the upper entries from the
+// last (DIC's face loop in reverse).  Bound by the chain of wavefronts (a
+// hop and up to four FP64 operations each) up to some 10^5 rows, by the FP64
+// pipe above.
+template <int CK>
+__global__ void __launch_bounds__(kFlowThreads) flow_dic_kernel(const __grid_constant__ DicArgs a,
+                                                                Gate g)
+{
+    if (gate_closed(g)) return;
+    const int lane = threadIdx.x & 31;
+    const Rows<double>& A = a.A;
+    for (;;) {
+        const int t = __shfl_sync(0xffffffffu, take(a.counter), 0);
+        if (t >= 2 * a.nTasks) return;
+        const bool bwd = t >= a.nTasks;
+        const int q = bwd ? 2 * a.nTasks - 1 - t : t;
+        const int4 D = ldg(a.task + q);
+        const int2 nr = ldg(a.near + q);
+        const int r = D.x + lane;
+        const bool on = lane < D.y;
+        // entry k of the sweep is entry first + k * step of the storage
+        int cnt = 0, first = 0;
+        const int step = bwd ? -32 : 32;
+        double acc = 0.0, rr = 0.0;
+        if (on) {
+            const int info = ldg(A.rowInfo + r);
+            const int len = info & 0xffff, nLow = info >> 16;
+            const int base = D.z + lane;
+            cnt = bwd ? len - nLow : nLow;
+            first = bwd ? base + 32 * (len - 1) : base;
+            rr = __ldcg(a.r + r);
+            if (!bwd) acc = ldg(a.rD + r) * rr;
+        }
+        const int most = __reduce_max_sync(0xffffffffu, cnt);
+        double* out = bwd ? a.w : a.wf;
+        const int wait = bwd ? nr.y : nr.x;
+        int j0 = 0;
+        do {
+            // slot CK is the backward sweep's own starting value
+            int c[CK];
+            double v[CK], xv[CK + 1];
+            unsigned need = 0;
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                const int e = first + step * (j0 + k);
+                const bool has = j0 + k < cnt;
+                c[k] = has ? ldg(A.col + e) : 0;
+                v[k] = has ? ldg(a.f + e) : 0.0;
+                xv[k] = 0.0;
+                if (has) need |= 1u << k;
+            }
+            xv[CK] = 0.0;
+            if (bwd && on && j0 == 0) need |= 1u << CK;
+            if (j0 == 0 && wait >= 0) wait_near(out + wait, a.err);
+            wait_values<double, CK + 1>(
+                need, [&](int k) { return k == CK ? a.wf + r : (const double*)out + c[k]; }, xv,
+                a.err);
+            if (bwd && j0 == 0) acc = xv[CK];
+#pragma unroll
+            for (int k = 0; k < CK; ++k) xv[k] = v[k] * xv[k];
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                if (j0 + k >= most) break;
+                const double less = acc - xv[k];
+                acc = j0 + k < cnt ? less : acc;
+            }
+            j0 += CK;
+        } while (j0 < most);
+        if (on) st_flow(out + r, acc);
+        if (bwd && a.part) {
+            const double s = warp_sum(on ? acc * rr : 0.0);
+            if (lane == 0) a.part[q] = s;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) flow_sum_kernel(int n, const double* __restrict__ part,
+                                                          RSpec red, Gate g)
+{
+    if (gate_closed(g)) return;
+    double v[1] = {0.0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        v[0] += part[i];
+    reduce_launch<1>(v, red, [&](const double (&t)[1]) { apply_fin(red.st, red.fin, t, 1); });
+}
+
 void tick()
 {
     if (!capturing()) count_launches(1);
@@ -431,5 +602,60 @@ template float* flow_gs<float>(const Exec&, const Level&, const Rows<float>&, co
 template double* flow_gs<double>(const Exec&, const Level&, const Rows<double>&, const FlowRing&,
                                  const double*, const double*, int, bool, bool, double*, double*,
                                  Gate);
+
+void DicFlow::init(const Level& L)
+{
+    rD.alloc((size_t)L.n);
+    f.alloc((size_t)L.nEntries);
+    part.alloc((size_t)std::max(L.tasks[0].n, 1));
+    ring.init((size_t)L.n, sizeof(double), 1);
+}
+
+void flow_dic_factor(const Exec& ex, const Level& L, bool dilu, DicFlow& D)
+{
+    if (L.n <= 0) return;
+    Rows<double> A = rows64(L);
+    // DIC: upper * upper; DILU: upper * lower.  On the lower side of a row the
+    // face's upper coefficient is valT and its lower coefficient is val; the
+    // forward sweep reads upper (DIC) or lower (DILU) there.
+    const double* c1 = A.valT;
+    const double* c2 = dilu ? A.val : A.valT;
+    double* d = reinterpret_cast<double*>(D.ring.vec(0, 0));
+    UNAP_CK(cudaMemsetAsync(D.ring.counter(0), 0xff, kFlowHeader + D.ring.stride, ex.s));
+    tick();
+    flow_factor_kernel<4><<<flow_grid(L.tasks[0].n), kFlowThreads, 0, ex.s>>>(
+        A, L.tasks[0].task.p, L.tasks[0].near.p, L.tasks[0].n, c1, c2, d, D.rD.p, D.f.p,
+        D.ring.counter(0), D.ring.err);
+    UNAP_CK(cudaGetLastError());
+}
+
+void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const double* r, double* w,
+                    const RedPool* pool, int site, KState* st, int fin, Gate g)
+{
+    if (L.n <= 0) return;
+    DicArgs a;
+    a.A = rows64(L);
+    a.task = L.tasks[0].task.p;
+    a.near = L.tasks[0].near.p;
+    a.nTasks = L.tasks[0].n;
+    a.f = D.f.p;
+    a.rD = D.rD.p;
+    a.r = r;
+    a.wf = reinterpret_cast<double*>(D.ring.vec(1, 0));
+    a.w = w;
+    a.part = pool ? D.part.p : nullptr;
+    a.counter = D.ring.counter(1);
+    a.err = D.ring.err;
+    UNAP_CK(cudaMemsetAsync(a.counter, 0xff, kFlowHeader + D.ring.stride, ex.s));
+    UNAP_CK(cudaMemsetAsync(w, 0xff, (size_t)L.n * sizeof(double), ex.s));
+    tick();
+    flow_dic_kernel<4><<<flow_grid(2LL * L.tasks[0].n), kFlowThreads, 0, ex.s>>>(a, g);
+    if (pool) {
+        tick();
+        flow_sum_kernel<<<ex.grid(div_up(L.tasks[0].n, 4)), kBlock, 0, ex.s>>>(
+            L.tasks[0].n, D.part.p, pool->site(site, st, fin), g);
+    }
+    UNAP_CK(cudaGetLastError());
+}
 
 }  // namespace unapgpu

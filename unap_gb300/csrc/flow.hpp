@@ -1,4 +1,5 @@
 // Wavefront sweeps as one launch (implemented in flow.cu): Gauss-Seidel
+// sweeps, the DIC/DILU factorisation and the DIC/DILU forward and backward
 // sweeps of a level, with its rows as warp tasks taken in dependency order.
 #pragma once
 
@@ -46,6 +47,22 @@ struct FlowRing {
 template <class T>
 T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& ring, const T* in,
            const T* b, int nSweeps, bool backward, bool xIsZero, T* last, T* copy, Gate g);
+
+// DIC / DILU.  rD: the factored diagonal's reciprocal; f: every entry times
+// its row's reciprocal (rD coef on the lower side, rD upper on the upper
+// side); part: partial sums of w.r, one per task; ring: the factored diagonal
+// and the forward sweep's vector.
+struct DicFlow {
+    DevArray<double> rD, f, part;
+    FlowRing ring;
+    void init(const Level& L);
+    void check() const { ring.check(); }
+};
+// factors the level's matrix (DIC, or DILU); check() once it is done
+void flow_dic_factor(const Exec& ex, const Level& L, bool dilu, DicFlow& D);
+// w = M^-1 r; with a pool, w.r is reduced into `site` and finalized with fin
+void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const double* r, double* w,
+                    const RedPool* pool, int site, KState* st, int fin, Gate g);
 
 // the level's task table, built with the level (build_level)
 void flow_tasks(Level& L, cudaStream_t s);

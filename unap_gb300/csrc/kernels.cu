@@ -233,170 +233,6 @@ void gs_sweep(const Exec& ex, const Level& L, const Rows<T>& A, T* x, const T* b
     }
 }
 
-// --------------------------------------------------------------------------
-// DIC / DILU
-// --------------------------------------------------------------------------
-
-// lduDICPrecond::calcReciprocalD (lduDICPrecond.cpp:15-42) and the DILU
-// variant (lduDILUPrecond.cpp:15-43) on one wavefront:
-// dfac_c = D_c - sum over lower-side faces (asc) of (c1 c2) / dfac_l
-__global__ void __launch_bounds__(kBlock) factor_kernel(Rows<double> A, const double* c1,
-                                                        const double* c2, double* dfac, int r0,
-                                                        int r1)
-{
-    for (int r = r0 + blockIdx.x * blockDim.x + threadIdx.x; r < r1;
-         r += gridDim.x * blockDim.x) {
-        const int info = ldg(A.rowInfo + r);
-        const int nLow = info >> 16;
-        const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
-        double d = ldg(A.diag + r);
-        for (int j = 0; j < nLow; ++j) {
-            const int e = base + 32 * j;
-            d -= ldg(c1 + e) * ldg(c2 + e) / dfac[ldg(A.col + e)];
-        }
-        dfac[r] = d;
-    }
-}
-
-__global__ void recip_kernel(int n, const double* __restrict__ d, double* __restrict__ rD)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        rD[i] = 1.0 / d[i];
-}
-
-void dic_factor(const Exec& ex, const Level& L, bool dilu, double* dfac, double* rD)
-{
-    Rows<double> A = rows64(L);
-    // DIC: upper * upper; DILU: upper * lower.  On the lower side of a row the
-    // face's upper coefficient is valT and its lower coefficient is val.
-    const double* c1 = A.valT;
-    const double* c2 = dilu ? A.val : A.valT;
-    for (int w = 0; w < L.nWave; ++w) {
-        int r0 = L.waveStart[w], r1 = L.waveStart[w + 1];
-        if (r1 > r0) tick(), factor_kernel<<<ex.grid(r1 - r0), kBlock, 0, ex.s>>>(A, c1, c2, dfac, r0, r1);
-    }
-    if (L.n) tick(), recip_kernel<<<ex.grid(L.n), kBlock, 0, ex.s>>>(L.n, dfac, rD);
-}
-
-// forward sweep (lduDICPrecond.cpp:63-71; DILU in losort order,
-// lduDILUPrecond.cpp:70-80): w_c = rD_c r_c - sum_low (rD_c coef) w_l
-template <int CK>
-__global__ void __launch_bounds__(kBlock) dic_fwd_kernel(Rows<double> A, const double* coef,
-                                                         const double* __restrict__ rD,
-                                                         const double* rr, double* w, int r0,
-                                                         int r1, Gate g)
-{
-    // Programmatic dependent launch: the next wavefront's kernel may launch
-    // now.  Before griddepcontrol.wait this kernel reads only the matrix and
-    // rD (written at factorisation); r, w and the solver state after it.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int r = r0 + blockIdx.x * blockDim.x + threadIdx.x;
-    int nLow = 0, base = 0;
-    double rd = 0.0;
-    int c[CK];
-    double v[CK];
-    if (r < r1) {
-        nLow = ldg(A.rowInfo + r) >> 16;
-        base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
-        rd = ldg(rD + r);
-#pragma unroll
-        for (int k = 0; k < CK; ++k) {
-            const int e = base + 32 * k;
-            c[k] = k < nLow ? ldg(A.col + e) : r;
-            v[k] = k < nLow ? ldg(coef + e) : 0.0;
-        }
-    }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (gate_closed(g) || r >= r1) return;
-    // lduDICPrecond.cpp:65-71: w = rD r, then w_u -= (rD_u coef) w_l in face order
-    double acc = rd * rr[r];
-#pragma unroll
-    for (int k = 0; k < CK; ++k)
-        if (k < nLow) acc -= rd * v[k] * w[c[k]];
-    for (int j = CK; j < nLow; ++j) {
-        const int e = base + 32 * j;
-        acc -= rd * ldg(coef + e) * w[ldg(A.col + e)];
-    }
-    w[r] = acc;
-}
-
-// backward sweep (lduDICPrecond.cpp:73-76): faces in reverse order,
-// w_c -= (rD_c upper) w_u; sums w.r for the PCG/PBiCGStab dot product
-__global__ void __launch_bounds__(kBlock) dic_bwd_kernel(Rows<double> A,
-                                                         const double* __restrict__ rD,
-                                                         const double* rr, double* w, int r0,
-                                                         int r1, RSpec red, Gate g)
-{
-    // programmatic dependent launch: launch the next wavefront now, wait for
-    // this one's inputs before reading anything the chain writes
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (gate_closed(g)) return;
-    double v[1] = {0.0};
-    for (int r = r0 + blockIdx.x * blockDim.x + threadIdx.x; r < r1;
-         r += gridDim.x * blockDim.x) {
-        const int info = ldg(A.rowInfo + r);
-        const int len = info & 0xffff;
-        const int nLow = info >> 16;
-        const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
-        const double rd = ldg(rD + r);
-        double acc = w[r];
-        for (int j = len - 1; j >= nLow; --j) {
-            const int e = base + 32 * j;
-            acc -= rd * ldg(A.val + e) * w[ldg(A.col + e)];
-        }
-        w[r] = acc;
-        v[0] += acc * rr[r];
-    }
-    if (red.blockPart) reduce_and_finalize<1>(v, red);
-}
-
-// wavefronts of up to this many rows launch one-warp CTAs (spread over more
-// SMs, as for the Gauss-Seidel wavefronts)
-constexpr int kDicSmallRows = 100000;
-
-void dic_apply(const Exec& ex, const Level& L, bool dilu, const double* rD, const double* r,
-               double* w, const RedPool* pool, int site, KState* st, int fin, Gate g)
-{
-    Rows<double> A = rows64(L);
-    const double* coef = dilu ? A.val : A.valT;  // DIC uses upper on the lower side
-    const int W = L.nWave;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.stream = ex.s;
-    cfg.attrs = at;
-    cfg.numAttrs = wave_pdl() ? 1 : 0;
-    for (int k = 0; k < W; ++k) {
-        const int r0 = L.waveStart[k], r1 = L.waveStart[k + 1];
-        if (r1 <= r0) continue;
-        const int threads = (r1 - r0) <= kDicSmallRows ? 32 : kBlock;
-        cfg.gridDim = dim3((unsigned)div_up(r1 - r0, threads));
-        cfg.blockDim = dim3((unsigned)threads);
-        tick();
-        UNAP_CK(cudaLaunchKernelEx(&cfg, dic_fwd_kernel<4>, A, coef, rD, r, w, r0, r1, g));
-    }
-    // backward: one launch slot per non-empty wavefront
-    int nonEmpty = 0;
-    for (int k = 0; k < W; ++k) nonEmpty += L.waveStart[k + 1] > L.waveStart[k];
-    int slot = 0;
-    for (int k = W - 1; k >= 0; --k) {
-        const int r0 = L.waveStart[k], r1 = L.waveStart[k + 1];
-        if (r1 <= r0) continue;
-        RSpec red;
-        if (pool) red = pool->site(site, st, slot == nonEmpty - 1 ? fin : FIN_STORE, slot, nonEmpty);
-        const int threads = (r1 - r0) <= kDicSmallRows ? 32 : kBlock;
-        int grid = div_up(r1 - r0, threads);
-        if (red.blockPart && grid > red.maxBlocks) grid = red.maxBlocks;
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3((unsigned)threads);
-        tick();
-        UNAP_CK(cudaLaunchKernelEx(&cfg, dic_bwd_kernel, A, rD, r, w, r0, r1, red, g));
-        ++slot;
-    }
-}
-
 __global__ void __launch_bounds__(kBlock) diag_apply_kernel(int n, const double* __restrict__ rD,
                                                             const double* __restrict__ r,
                                                             double* __restrict__ w, RSpec red,

@@ -48,14 +48,6 @@ template <class T>
 void gs_sweep(const Exec& ex, const Level& L, const Rows<T>& A, T* x, const T* b, bool backward,
               bool xIsZero, Gate g);
 
-// DIC (dilu=false) or DILU factorisation: rD = 1 / factored diagonal.
-void dic_factor(const Exec& ex, const Level& L, bool dilu, double* dfac, double* rD);
-
-// w = M^-1 r for M = DIC/DILU with rD; with a reduction spec, sums w.r over
-// all wavefronts (backward sweep launches) and finalizes on the last one.
-void dic_apply(const Exec& ex, const Level& L, bool dilu, const double* rD, const double* r,
-               double* w, const RedPool* pool, int site, KState* st, int fin, Gate g);
-
 // w = rD * r (Diag) or w = r (rD == nullptr); sums w.r.
 void diag_apply(const Exec& ex, int n, const double* rD, const double* r, double* w, RSpec red,
                 Gate g);

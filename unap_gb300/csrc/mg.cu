@@ -187,15 +187,14 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
     if (nC > 0) {
         Lv& C = lv[(size_t)nC];
         const bool symm = C.L->symm;
-        C.dfac.alloc((size_t)C.n);
-        C.pfac.alloc((size_t)C.n);
-        dic_factor(ex, *C.L, !symm, C.dfac.p, C.pfac.p);
+        C.dic.init(*C.L);
+        flow_dic_factor(ex, *C.L, !symm, C.dic);
         coarseWork.alloc((size_t)8 * C.n);
         static_assert(sizeof(SmallSystem) % 8 == 0, "SmallSystem layout");
         SmallSystem S{};
         S.A = rows64(*C.L);
         S.nWave = C.L->nWave;
-        S.rD = C.pfac.p;
+        S.rD = C.dic.rD.p;
         S.method = symm ? 0 : 1;
         S.precond = symm ? 2 : 3;
         S.tol = 0.0;
@@ -225,6 +224,7 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
     UNAP_CK(cudaEventCreate(&ev0));
     UNAP_CK(cudaEventCreate(&ev1));
     UNAP_CK(cudaStreamSynchronize(s));
+    lv.back().dic.check();
 }
 
 MgSolver::~MgSolver()

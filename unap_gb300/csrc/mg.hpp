@@ -47,7 +47,7 @@ private:
         int n = 0;
         DevArray<int> childStart, child, cmap;  // transfer into this level (k >= 1)
         DevArray<double> corr, src, acf, pre, rD, w, p;
-        DevArray<double> dfac, pfac;  // coarsest DIC/DILU factor
+        DicFlow dic;                  // coarsest DIC/DILU factor
         FlowRing sweeps;              // Gauss-Seidel sweeps
     };
     Matrix& A;
