@@ -571,6 +571,7 @@ int unap_cuda_precondition(long int handle, int precond, const double* r, double
         order_after_default_stream(A.stream);
         Exec ex{A.stream, device_max_blocks()};
         h->ensureScratch();
+        StreamAllocScope scope(A.stream, workspace_pool());
         auto P = make_ldu_precond(precond, A);
         k_to_internal<double>(ex, A.n(), A.L->d_perm.p, r, h->s1.p);
         P->apply(ex, h->s1.p, h->s2.p, nullptr, 0, nullptr, FIN_NONE, Gate{});
@@ -618,6 +619,7 @@ int unap_cuda_krylov_solve(long int handle, int method, int precond, double tol,
             throw std::invalid_argument("method 0 (PCG) or 1 (PBiCGStab)");
         if (precond < 0 || precond > 3)
             throw std::invalid_argument("precond 0 (none), 1 (Diag), 2 (DIC) or 3 (DILU)");
+        StreamAllocScope scope(A.stream, workspace_pool());
         auto P = make_ldu_precond(precond, A);
         Krylov K(A, P.get(), method == 1 ? Method::PBiCGStab : Method::PCG);
         order_after_default_stream(A.stream);

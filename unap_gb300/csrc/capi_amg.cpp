@@ -164,6 +164,7 @@ int unap_cuda_amg_vcycle(long int amg, const double* r, double* z)
         order_after_default_stream(A.stream);
         Exec ex{A.stream, device_max_blocks()};
         const int n = A.n();
+        StreamAllocScope scope(A.stream, workspace_pool());
         DevArray<double> ri((size_t)n), zi((size_t)n);
         k_to_internal<double>(ex, n, A.L->d_perm.p, r, ri.p);
         h->H->vcycle(ex, ri.p, zi.p, Gate{});

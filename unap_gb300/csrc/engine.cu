@@ -33,6 +33,41 @@ cudaStream_t& thread_alloc_stream()
     static thread_local cudaStream_t s = nullptr;
     return s;
 }
+cudaMemPool_t& thread_alloc_pool()
+{
+    static thread_local cudaMemPool_t p = nullptr;
+    return p;
+}
+namespace {
+std::mutex g_workspaceMutex;
+std::map<int, cudaMemPool_t> g_workspacePools;  // by device
+std::map<int, int> g_matrices;                  // matrices alive, by device
+}  // namespace
+cudaMemPool_t workspace_pool()
+{
+    int dev = 0;
+    UNAP_CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_workspaceMutex);
+    cudaMemPool_t& p = g_workspacePools[dev];
+    if (!p) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        UNAP_CK(cudaMemPoolCreate(&p, &props));
+        unsigned long long keep = 1ull << 30;
+        UNAP_CK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    return p;
+}
+void trim_workspace_pool()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> lk(g_workspaceMutex);
+    auto it = g_workspacePools.find(dev);
+    if (it != g_workspacePools.end() && it->second) cudaMemPoolTrimTo(it->second, 0);
+}
 void keep_pool_memory()
 {
     static std::mutex m;
@@ -83,12 +118,23 @@ void order_after_default_stream(cudaStream_t s)
 {
     // an event on the legacy default stream, waited for by s: everything
     // issued before the call to the legacy stream (and so to every blocking
-    // stream) is done before s runs the call's kernels
-    cudaEvent_t e;
-    UNAP_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    // stream) is done before s runs the call's kernels.  The event is this
+    // thread's own, one per device; recording it again while another stream
+    // still waits for its last record does not change that wait.
+    struct Events {
+        std::map<int, cudaEvent_t> byDevice;
+        ~Events()
+        {
+            for (auto& e : byDevice) cudaEventDestroy(e.second);
+        }
+    };
+    static thread_local Events events;
+    int dev = 0;
+    UNAP_CK(cudaGetDevice(&dev));
+    cudaEvent_t& e = events.byDevice[dev];
+    if (!e) UNAP_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     UNAP_CK(cudaEventRecord(e, cudaStreamLegacy));
     UNAP_CK(cudaStreamWaitEvent(s, e, 0));
-    UNAP_CK(cudaEventDestroy(e));  // released once it has completed
 }
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 const char* last_error() { return g_last_error.c_str(); }
@@ -107,11 +153,20 @@ Matrix::Matrix(HostLdu&& h, cudaStream_t s, bool wavefronts) : host(std::move(h)
     }
     host.validate();
     L = build_level(host, nullptr, false, stream, wavefronts);
+    std::lock_guard<std::mutex> lk(g_workspaceMutex);
+    ++g_matrices[device];
+    counted = true;
 }
 
 Matrix::~Matrix()
 {
     L.reset();
+    if (counted) {
+        std::lock_guard<std::mutex> lk(g_workspaceMutex);
+        auto it = g_workspacePools.find(device);
+        if (--g_matrices[device] == 0 && it != g_workspacePools.end() && it->second)
+            cudaMemPoolTrimTo(it->second, 0);
+    }
     if (ownsStream && stream) cudaStreamDestroy(stream);
 }
 
@@ -306,7 +361,8 @@ Krylov::Krylov(Matrix& A_, Precond* P_, Method m) : A(A_), P(P_), method(m)
         s.alloc(N);
         t.alloc(N);
     }
-    UNAP_CK(gated_malloc((void**)&d_st, sizeof(KState)));
+    state.alloc(1);
+    d_st = state.p;
     h_st = static_cast<KState*>(pinned_block_alloc(sizeof(KState)));
     // partial buffers for one CTA per 256 rows (row kernels launch that many)
     pool.init(S_NSITES, std::max(ex.maxBlocks, div_up(n, kBlock)), std::max(1, A.L->nWave) + 1,
@@ -319,7 +375,6 @@ Krylov::~Krylov()
 {
     if (graphExec) cudaGraphExecDestroy(graphExec);
     if (graph) cudaGraphDestroy(graph);
-    if (d_st) gated_free(d_st);
     pinned_block_free(h_st);
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);

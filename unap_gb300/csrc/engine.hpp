@@ -32,6 +32,7 @@ public:
     cudaStream_t stream;
     bool ownsStream = false;
     int device = 0;  // the GPU the matrix was built on (current at construction)
+    bool counted = false;
     int n() const { return host.n; }
     // replace the coefficients (same addressing)
     void setValues(const double* diag, const double* upper, const double* lower);
@@ -98,7 +99,8 @@ private:
     int n;
     DevArray<double> x, b, r, z, p, q, r0, y, Ay, s, t, zz;
     DevArray<double> hx_ref;  // staging for host solves
-    KState* d_st = nullptr;
+    DevArray<KState> state;
+    KState* d_st = nullptr;   // state.p
     KState* h_st = nullptr;   // pinned
     RedPool pool;
     cudaGraph_t graph = nullptr;

@@ -72,10 +72,18 @@ struct CaptureGate {
     CaptureGate() : lk(capture_gate()) { thread_in_capture() = true; }
     ~CaptureGate() { thread_in_capture() = false; }
 };
+// what the workspace pool holds goes back to the driver (the current device)
+void trim_workspace_pool();
 inline cudaError_t gated_malloc(void** p, size_t bytes)
 {
     AllocGate g;
-    return cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        trim_workspace_pool();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 inline cudaError_t gated_free(void* p)
 {
@@ -102,15 +110,29 @@ inline cudaError_t gated_free_host(void* p)
 // slot workers: one stream each).  The pool keeps freed memory for reuse
 // instead of returning it to the driver at each synchronization.
 cudaStream_t& thread_alloc_stream();
+cudaMemPool_t& thread_alloc_pool();  // null: the device's default pool
 void keep_pool_memory();
+// The library's own pool for the workspaces of a call that returns
+// synchronized (a preconditioner's or Krylov solver's vectors): it keeps up
+// to 1 GiB of freed blocks, so a small call does not pay for cudaMalloc and
+// the device-wide wait of cudaFree, and gives them back when no matrix is
+// left or an allocation fails.
+cudaMemPool_t workspace_pool();
 struct StreamAllocScope {
     cudaStream_t prev;
-    explicit StreamAllocScope(cudaStream_t s) : prev(thread_alloc_stream())
+    cudaMemPool_t prevPool;
+    explicit StreamAllocScope(cudaStream_t s, cudaMemPool_t pool = nullptr)
+        : prev(thread_alloc_stream()), prevPool(thread_alloc_pool())
     {
-        keep_pool_memory();
+        if (!pool) keep_pool_memory();
         thread_alloc_stream() = s;
+        thread_alloc_pool() = pool;
     }
-    ~StreamAllocScope() { thread_alloc_stream() = prev; }
+    ~StreamAllocScope()
+    {
+        thread_alloc_stream() = prev;
+        thread_alloc_pool() = prevPool;
+    }
     StreamAllocScope(const StreamAllocScope&) = delete;
     StreamAllocScope& operator=(const StreamAllocScope&) = delete;
 };
@@ -167,7 +189,11 @@ struct DevArray {
         if (s) {
             if (thread_in_capture())
                 throw std::logic_error("device allocation inside a stream capture");
-            UNAP_CK(cudaMallocAsync((void**)&p, count * sizeof(T), s));
+            if (thread_alloc_pool())
+                UNAP_CK(cudaMallocFromPoolAsync((void**)&p, count * sizeof(T),
+                                                thread_alloc_pool(), s));
+            else
+                UNAP_CK(cudaMallocAsync((void**)&p, count * sizeof(T), s));
             as = s;
             async = true;
         } else {
