@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kFlowThreads)
     if (gate_closed(gate)) return;
     constexpr int RW = 32 / G;      // rows of a task
     constexpr int W = G * K;        // entries of a row held at once
-    constexpr int P = W + 1;        // row pitch of the products
+    constexpr int P = W + 5;        // row pitch of the products
     __shared__ T prod[kFlowThreads / 32][G == 1 ? 1 : RW * P];
     T* pw = prod[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -219,15 +219,23 @@ __global__ void __launch_bounds__(kFlowThreads)
                 // the reference's order: entry after entry
                 const int m = min(jEnd - j0, W);
                 const T* p = pw + row * P;
+                T p0 = p[0], p1 = p[1], p2 = p[2], p3 = p[3];
                 int j = 0;
                 for (; j + 4 <= m; j += 4) {
-                    const T p0 = p[j], p1 = p[j + 1], p2 = p[j + 2], p3 = p[j + 3];
+                    // the next four (a row's pitch leaves room for them)
+                    const T n0 = p[j + 4], n1 = p[j + 5], n2 = p[j + 6], n3 = p[j + 7];
                     acc -= p0;
                     acc -= p1;
                     acc -= p2;
                     acc -= p3;
+                    p0 = n0;
+                    p1 = n1;
+                    p2 = n2;
+                    p3 = n3;
                 }
-                for (; j < m; ++j) acc -= p[j];
+                if (j < m) acc -= p0;
+                if (j + 1 < m) acc -= p1;
+                if (j + 2 < m) acc -= p2;
             }
             if (G > 1) __syncwarp();
             j0 += W;
@@ -391,7 +399,10 @@ __global__ void __launch_bounds__(kFlowThreads) flow_dic_kernel(const __grid_con
                 a.err);
             if (bwd && j0 == 0) acc = xv[CK];
 #pragma unroll
-            for (int k = 0; k < CK; ++k) xv[k] = v[k] * xv[k];
+            for (int k = 0; k < CK; ++k) {
+                if (j0 + k >= most) break;
+                xv[k] = v[k] * xv[k];
+            }
 #pragma unroll
             for (int k = 0; k < CK; ++k) {
                 if (j0 + k >= most) break;
@@ -623,7 +634,7 @@ void flow_dic_factor(const Exec& ex, const Level& L, bool dilu, DicFlow& D)
     double* d = reinterpret_cast<double*>(D.ring.vec(0, 0));
     UNAP_CK(cudaMemsetAsync(D.ring.counter(0), 0xff, kFlowHeader + D.ring.stride, ex.s));
     tick();
-    flow_factor_kernel<4><<<flow_grid(L.tasks[0].n), kFlowThreads, 0, ex.s>>>(
+    flow_factor_kernel<8><<<flow_grid(L.tasks[0].n), kFlowThreads, 0, ex.s>>>(
         A, L.tasks[0].task.p, L.tasks[0].near.p, L.tasks[0].n, c1, c2, d, D.rD.p, D.f.p,
         D.ring.counter(0), D.ring.err);
     UNAP_CK(cudaGetLastError());
@@ -649,7 +660,7 @@ void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const doub
     UNAP_CK(cudaMemsetAsync(a.counter, 0xff, kFlowHeader + D.ring.stride, ex.s));
     UNAP_CK(cudaMemsetAsync(w, 0xff, (size_t)L.n * sizeof(double), ex.s));
     tick();
-    flow_dic_kernel<4><<<flow_grid(2LL * L.tasks[0].n), kFlowThreads, 0, ex.s>>>(a, g);
+    flow_dic_kernel<8><<<flow_grid(2LL * L.tasks[0].n), kFlowThreads, 0, ex.s>>>(a, g);
     if (pool) {
         tick();
         flow_sum_kernel<<<ex.grid(div_up(L.tasks[0].n, 4)), kBlock, 0, ex.s>>>(
