@@ -20,7 +20,6 @@
 
 #include "batch.hpp"
 #include "device_common.cuh"
-#include "flow.hpp"
 
 namespace unapgpu {
 
@@ -203,31 +202,29 @@ BatchSolver::BatchSolver(cudaStream_t s) : stream(s) {}
 
 BatchSolver::~BatchSolver() = default;
 
-const double* BatchSolver::factor(Matrix& A, int precond)
+const DicFlow& BatchSolver::factor(Matrix& A, int precond)
 {
     // reciprocal diagonal for Diag (1/D), DIC or DILU, cached per matrix and
     // coefficient version
     Key k{&A, precond};
     auto it = factors.find(k);
-    if (it != factors.end() && it->second.version == A.L->version) return it->second.rD.p;
+    if (it != factors.end() && it->second.version == A.L->version) return it->second.D;
     Fac f;
     f.version = A.L->version;
     if (precond == 1) {
         std::vector<double> h((size_t)A.n());
         for (int i = 0; i < A.n(); ++i) h[(size_t)i] = 1.0 / A.host.diag[(size_t)A.L->perm[(size_t)i]];
-        f.rD.upload(h, stream);
+        f.D.rD.upload(h, stream);
     } else {
-        DicFlow D;
-        D.init(*A.L);
-        flow_dic_factor(Exec{stream, device_max_blocks()}, *A.L, precond == 3, D);
+        f.D.init(*A.L);
+        flow_dic_factor(Exec{stream, device_max_blocks()}, *A.L, precond == 3, f.D);
         UNAP_CK(cudaStreamSynchronize(stream));
-        D.check();
-        f.rD = std::move(D.rD);
+        f.D.check();
     }
     UNAP_CK(cudaStreamSynchronize(stream));
     auto& slot = factors[k];
     slot = std::move(f);
-    return slot.rD.p;
+    return slot.D;
 }
 
 void BatchSolver::forget(const Matrix* A)
@@ -330,8 +327,8 @@ void BatchSolver::solveSmall(const std::vector<BatchItem>& items, const std::vec
         total += (size_t)items[(size_t)i].A->n();
         nMax = std::max(nMax, items[(size_t)i].A->n());
     }
-    // workspace: internal x, b and 8 work vectors per system (reused)
-    if (ws.n < total * 10) ws.alloc(total * 10);
+    // workspace: internal x, b and the work vectors of each system (reused)
+    if (ws.n < total * (2 + kTeamWorkBicg)) ws.alloc(total * (2 + kTeamWorkBicg));
     std::vector<SmallSystem> sys((size_t)m);
     std::vector<PermJob> in((size_t)2 * m), outJobs((size_t)m);
     std::vector<std::vector<int>> waves;
@@ -344,14 +341,18 @@ void BatchSolver::solveSmall(const std::vector<BatchItem>& items, const std::vec
         double* xi = ws.p + off;
         double* bi = xi + n;
         double* wk = bi + n;
-        off += (size_t)n * 10;
+        off += (size_t)n * (2 + kTeamWorkBicg);
         SmallSystem& S = sys[(size_t)j];
         S = SmallSystem{};
         S.A = rows64(*A.L);
         S.nWave = A.L->nWave;
         waveDev[(size_t)j].upload(A.L->waveStart, stream);
         S.waveStart = waveDev[(size_t)j].p;
-        S.rD = (it.precond >= 1 && it.precond <= 3) ? factor(A, it.precond) : nullptr;
+        if (it.precond >= 1 && it.precond <= 3) {
+            const DicFlow& D = factor(A, it.precond);
+            S.rD = D.rD.p;
+            if (it.precond >= 2) small_sweeps(S, *A.L, D);
+        }
         S.method = it.method == 1 ? 1 : 0;
         S.precond = (it.precond >= 1 && it.precond <= 3) ? it.precond : 0;
         S.tol = it.tol;
@@ -385,6 +386,10 @@ void BatchSolver::solveSmall(const std::vector<BatchItem>& items, const std::vec
                             cudaMemcpyDeviceToHost, stream));
     UNAP_CK(cudaStreamSynchronize(stream));
     UNAP_CK(cudaGetLastError());
+    for (int i : idx) {
+        const BatchItem& it = items[(size_t)i];
+        if (it.precond >= 2 && it.precond <= 3) factor(*it.A, it.precond).check();
+    }
     for (int j = 0; j < m; ++j) {
         SolveStats& s = out[(size_t)idx[(size_t)j]];
         s.nIter = res[(size_t)j].nIter;

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "engine.hpp"
+#include "flow.hpp"
 #include "small_solve.hpp"
 
 namespace unapgpu {
@@ -34,7 +35,7 @@ public:
     int lastLargeMode = -1;     // systems above the whole-solve size: 1 one
                                 // group launch, 0 one after another, -1 none
 
-    // drop the cached preconditioner diagonals of a matrix that is going away
+    // drop the cached preconditioners of a matrix that is going away
     void forget(const Matrix* A);
 
 private:
@@ -48,16 +49,16 @@ private:
     };
     struct Fac {
         int version = -1;
-        DevArray<double> rD;
+        DicFlow D;  // rD alone for Diag
     };
     cudaStream_t stream;
-    std::map<Key, Fac> factors;       // preconditioner diagonals per matrix
+    std::map<Key, Fac> factors;       // preconditioners per matrix
     DevArray<double> ws;              // internal-order x, b and work vectors
     DevArray<SmallSystem> dSys;
     DevArray<SmallResult> results;
     std::vector<DevArray<int>> waveDev;
     DevArray<unsigned char> dIn, dOut;  // gather / scatter job lists
-    const double* factor(Matrix& A, int precond);
+    const DicFlow& factor(Matrix& A, int precond);
     // the systems idx in one whole-solve launch (largeGroup: systems above
     // the whole-solve size, clusters of 16 only); *tunedMs = the chosen
     // shape's capped trial time (timed now or cached with the shape), left

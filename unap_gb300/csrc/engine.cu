@@ -316,6 +316,7 @@ public:
     }
     int lduType() const override { return dilu ? 3 : 2; }
     const double* lduRD() const override { return D.rD.p; }
+    const DicFlow* dicFlow() const override { return &D; }
     const Level& L;
     bool dilu;
     DicFlow D;
@@ -591,7 +592,7 @@ SolveStats Krylov::solveTeam(double* x_ref, const double* b_ref)
     const Level& L = *A.L;
     const size_t N = (size_t)n;
     if (!teamWork.p) {
-        teamWork.alloc(N * (method == Method::PBiCGStab ? 8 : 3));
+        teamWork.alloc(N * (method == Method::PBiCGStab ? kTeamWorkBicg : kTeamWorkPcg));
         teamWaves.upload(L.waveStart, ex.s);
         teamSys.alloc(sizeof(SmallSystem) + sizeof(SmallResult));
     }
@@ -603,6 +604,7 @@ SolveStats Krylov::solveTeam(double* x_ref, const double* b_ref)
     S.nWave = L.nWave;
     S.precond = P->lduType();
     S.rD = S.precond ? P->lduRD() : nullptr;
+    if (const DicFlow* D = P->dicFlow()) small_sweeps(S, L, *D);
     S.method = method == Method::PBiCGStab ? 1 : 0;
     S.tol = tol;
     S.relTol = relTol;
@@ -632,6 +634,7 @@ SolveStats Krylov::solveTeam(double* x_ref, const double* b_ref)
     UNAP_CK(cudaMemcpyAsync(&R, dR, sizeof(R), cudaMemcpyDeviceToHost, ex.s));
     UNAP_CK(cudaStreamSynchronize(ex.s));
     UNAP_CK(cudaGetLastError());
+    P->check();
     SolveStats out;
     float ms = 0;
     UNAP_CK(cudaEventElapsedTime(&ms, ev0, ev1));

@@ -10,6 +10,8 @@
 
 namespace unapgpu {
 
+struct DicFlow;
+
 struct SolveStats {
     int nIter = 0;
     double initRes = 0, finalRes = 0, trueRes = -1;
@@ -60,6 +62,8 @@ public:
     // its reciprocal diagonal in internal order, for whole-solve launches
     virtual int lduType() const { return -1; }
     virtual const double* lduRD() const { return nullptr; }
+    // DIC/DILU: its sweep data (null otherwise)
+    virtual const DicFlow* dicFlow() const { return nullptr; }
     // throws when a wait of an apply() ran out (after synchronizing with it)
     virtual void check() const {}
 };

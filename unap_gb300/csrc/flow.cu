@@ -23,8 +23,8 @@
 // has; the host turns that into an error (FlowRing::check).
 #include <algorithm>
 
-#include "device_common.cuh"
 #include "flow.hpp"
+#include "flow_values.cuh"
 
 namespace unapgpu {
 
@@ -33,74 +33,6 @@ namespace {
 constexpr int kFlowThreads = 128;
 constexpr int kStreams = kFlowThreads / 32;  // a task counter for each warp of a CTA
 static_assert(kFlowHeader >= kStreams * kFlowCounterBytes, "a counter per stream");
-constexpr int kSpinLimit = 1 << 23;  // polls; one is 0.3 us or more
-
-// ---- values that say whether they are there -------------------------------
-__device__ __forceinline__ float ld_flow(const float* p)
-{
-    float v;
-    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ double ld_flow(const double* p)
-{
-    double v;
-    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ bool absent(float v) { return __float_as_uint(v) == 0xffffffffu; }
-__device__ __forceinline__ bool absent(double v) { return __double_as_longlong(v) == -1ll; }
-__device__ __forceinline__ void st_flow(float* p, float v)
-{
-    if (absent(v)) v = __uint_as_float(0x7fffffffu);
-    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
-}
-__device__ __forceinline__ void st_flow(double* p, double v)
-{
-    if (absent(v)) v = __longlong_as_double(0x7ff8000000000000ll);
-    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-}
-
-// One more poll of a wait: true when the wait has to be given up.
-__device__ __forceinline__ bool give_up(int& spins, int* err)
-{
-    if ((++spins & 0xfff) == 0) {
-        if (spins >= kSpinLimit) *(volatile int*)err = 1;
-        if (*(volatile int*)err) return true;
-    }
-    return false;
-}
-
-// Loads at(k) for the entries in `need` (one bit each) until every value is
-// there; all lanes of the warp call it.
-template <class T, int CK, class At>
-__device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], int* err)
-{
-    int spins = 0;
-    for (;;) {
-#pragma unroll
-        for (int k = 0; k < CK; ++k)
-            if (need >> k & 1u) v[k] = ld_flow(at(k));
-#pragma unroll
-        for (int k = 0; k < CK; ++k)
-            if ((need >> k & 1u) && !absent(v[k])) need &= ~(1u << k);
-        if (!__any_sync(0xffffffffu, need != 0)) return;
-        if (give_up(spins, err)) return;
-    }
-}
-
-// A task far ahead of the rows that are being computed would poll for long:
-// until a row two wavefronts before its own is there, the whole warp polls
-// that one address, with pauses.
-template <class T>
-__device__ __forceinline__ void wait_near(const T* p, int* err)
-{
-    int spins = 0;
-    while (absent(ld_flow(p))) {
-        __nanosleep(64);
-        if (give_up(spins, err)) return;
-    }
-}
 
 // The next task of this warp.  Warp w of every CTA takes the tasks w, w +
 // kStreams, ... from a counter of its own (starting at -1).  As every CTA
@@ -486,6 +418,16 @@ FlowRing::FlowRing(FlowRing&& o) noexcept
     o.err = nullptr;
 }
 
+FlowRing& FlowRing::operator=(FlowRing&& o) noexcept
+{
+    mem = std::move(o.mem);
+    stride = o.stride;
+    half = o.half;
+    sweeps = o.sweeps;
+    std::swap(err, o.err);
+    return *this;
+}
+
 FlowRing::~FlowRing() { pinned_block_free(err); }
 
 void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves)
@@ -667,6 +609,16 @@ void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const doub
             L.tasks[0].n, D.part.p, pool->site(site, st, fin), g);
     }
     UNAP_CK(cudaGetLastError());
+}
+
+void small_sweeps(SmallSystem& S, const Level& L, const DicFlow& D)
+{
+    S.rD = D.rD.p;
+    S.f = D.f.p;
+    S.task = L.tasks[0].task.p;
+    S.near = L.tasks[0].near.p;
+    S.nTasks = L.tasks[0].n;
+    S.err = D.ring.err;
 }
 
 }  // namespace unapgpu

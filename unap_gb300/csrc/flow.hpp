@@ -4,6 +4,7 @@
 #pragma once
 
 #include "kernels.hpp"
+#include "small_solve.hpp"
 
 namespace unapgpu {
 
@@ -27,6 +28,7 @@ struct FlowRing {
     FlowRing(const FlowRing&) = delete;
     FlowRing& operator=(const FlowRing&) = delete;
     FlowRing(FlowRing&& o) noexcept;
+    FlowRing& operator=(FlowRing&& o) noexcept;
     ~FlowRing();
     void init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves = 2);
     size_t bytes() const { return mem.bytes(); }
@@ -64,6 +66,8 @@ void flow_dic_factor(const Exec& ex, const Level& L, bool dilu, DicFlow& D);
 void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const double* r, double* w,
                     const RedPool* pool, int site, KState* st, int fin, Gate g);
 
+// the DIC/DILU fields of a whole-solve system (the level's and D's arrays)
+void small_sweeps(SmallSystem& S, const Level& L, const DicFlow& D);
 // the level's task table, built with the level (build_level)
 void flow_tasks(Level& L, cudaStream_t s);
 

@@ -189,12 +189,12 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
         const bool symm = C.L->symm;
         C.dic.init(*C.L);
         flow_dic_factor(ex, *C.L, !symm, C.dic);
-        coarseWork.alloc((size_t)8 * C.n);
+        coarseWork.alloc((size_t)kTeamWorkBicg * C.n);
         static_assert(sizeof(SmallSystem) % 8 == 0, "SmallSystem layout");
         SmallSystem S{};
         S.A = rows64(*C.L);
         S.nWave = C.L->nWave;
-        S.rD = C.dic.rD.p;
+        small_sweeps(S, *C.L, C.dic);
         S.method = symm ? 0 : 1;
         S.precond = symm ? 2 : 3;
         S.tol = 0.0;
@@ -406,6 +406,7 @@ SolveStats MgSolver::solveDevice(double* x_ref, const double* b_ref)
             UNAP_CK(cudaMemcpyAsync(h_st, d_st, sizeof(KState), cudaMemcpyDeviceToHost, ex.s));
             UNAP_CK(cudaStreamSynchronize(ex.s));
             for (auto& K : lv) K.sweeps.check();
+            lv.back().dic.check();
             if (h_st->done) break;
         }
     } else {

@@ -15,13 +15,20 @@
 // the launch are read from L2 (ld.global.cg), so every CTA of the cluster
 // sees the other CTAs' rows after the barrier.
 //
+// DIC/DILU sweeps.  With C = 1 a barrier separates the wavefronts.  With
+// C > 1 a cluster barrier and the L2 round trip after it cost 1.8 us a
+// wavefront, so rows wait for their neighbours by value instead (flow.cu):
+// the sweeps' vectors are filled with 0xff bytes a barrier earlier, warp w of
+// CTA q takes every (C x warps)-th task from w C + q on, and both sweeps of an
+// application run without a barrier between their wavefronts.
+//
 // Rows are computed with the same per-row formulas as the multi-block
 // kernels, so SpMV and preconditioner applications are bit-identical to
 // them.  A dot product is the fixed block tree of each CTA; with C > 1 the
 // C block sums are exchanged through distributed shared memory and added in
 // rank order, identically in every CTA, so every CTA takes the same
 // branches.
-#include "device_common.cuh"
+#include "flow_values.cuh"
 #include "small_solve.hpp"
 
 namespace unapgpu {
@@ -116,26 +123,24 @@ __device__ void team_spmv(const Team<C>& T, const Rows<double>& A, const double*
 }
 
 // Row data of a DIC/DILU sweep that does not depend on the sweep's previous
-// wavefronts: the row's reciprocal, its starting value (r forward, w
-// backward) and its first kPre entries (forward: lower entries in order;
-// backward: upper entries from the last).  A thread loads them for its row
-// of the next wavefront while it computes the current one, so a wavefront
-// costs one dependent round trip (the gather of finished neighbours) and a
-// barrier.
+// wavefronts: the row's starting value (rD r forward, w backward) and its
+// first kPre scaled entries (forward: lower entries in order; backward:
+// upper entries from the last).  A thread loads them for its row of the next
+// wavefront while it computes the current one, so a wavefront costs one
+// dependent round trip (the gather of finished neighbours) and a barrier.
 constexpr int kPre = 4;
 
 struct RowPre {
     int i;       // row, -1: none
     int lo, hi;  // entries [lo, hi) of the row
     int base;
-    double rd, a0;
+    double a0;
     int c[kPre];
     double v[kPre];
 };
 
-template <int C, bool FWD>
-__device__ __forceinline__ void sweep_pre(const SmallSystem& S, const double* coef,
-                                          const double* src, int i, RowPre& P)
+template <bool FWD>
+__device__ __forceinline__ void sweep_pre(const SmallSystem& S, const double* src, int i, RowPre& P)
 {
     P.i = i;
     if (i < 0) return;
@@ -143,8 +148,7 @@ __device__ __forceinline__ void sweep_pre(const SmallSystem& S, const double* co
     const int info = A.rowInfo[i];
     const int len = info & 0xffff, nLow = info >> 16;
     P.base = A.sliceOff[i >> 5] + (i & 31);
-    P.rd = S.rD[i];
-    P.a0 = ldv<C>(src + i);
+    P.a0 = FWD ? S.rD[i] * src[i] : src[i];
     P.lo = FWD ? 0 : nLow;
     P.hi = FWD ? nLow : len;
 #pragma unroll
@@ -153,38 +157,37 @@ __device__ __forceinline__ void sweep_pre(const SmallSystem& S, const double* co
         const bool on = k < P.hi - P.lo;
         const int e = P.base + 32 * j;
         P.c[k] = on ? A.col[e] : i;
-        P.v[k] = on ? coef[e] : 0.0;
+        P.v[k] = on ? S.f[e] : 0.0;
     }
 }
 
 // lduDICPrecond.cpp:57-76 / lduDILUPrecond.cpp:60-85 for one row, in the
-// reference's order: forward acc = rD r, then acc -= rD coef w[l] over the
-// lower entries in face order; backward acc = w, then acc -= rD upper w[u]
+// reference's order: forward acc = rD r, then acc -= (rD coef) w[l] over the
+// lower entries in face order; backward acc = w, then acc -= (rD upper) w[u]
 // over the upper entries from the last
-template <int C, bool FWD>
-__device__ __forceinline__ double sweep_row(const SmallSystem& S, const double* coef,
-                                            const RowPre& P, const double* w)
+template <bool FWD>
+__device__ __forceinline__ double sweep_row(const SmallSystem& S, const RowPre& P, const double* w)
 {
-    double acc = FWD ? P.rd * P.a0 : P.a0;
+    double acc = P.a0;
     const int cnt = P.hi - P.lo;
     double xv[kPre];
 #pragma unroll
-    for (int k = 0; k < kPre; ++k) xv[k] = k < cnt ? ldv<C>(w + P.c[k]) : 0.0;
+    for (int k = 0; k < kPre; ++k) xv[k] = k < cnt ? w[P.c[k]] : 0.0;
 #pragma unroll
     for (int k = 0; k < kPre; ++k)
-        if (k < cnt) acc -= P.rd * P.v[k] * xv[k];
+        if (k < cnt) acc -= P.v[k] * xv[k];
     for (int k = kPre; k < cnt; ++k) {
         const int j = FWD ? P.lo + k : P.hi - 1 - k;
         const int e = P.base + 32 * j;
-        acc -= P.rd * coef[e] * ldv<C>(w + S.A.col[e]);
+        acc -= S.f[e] * w[S.A.col[e]];
     }
     return acc;
 }
 
 // one sweep over the wavefronts (forward: 0 .. nWave-1, backward: reverse)
-template <int C, bool FWD>
-__device__ __noinline__ void team_sweep(const Team<C>& T, const SmallSystem& S, const double* coef,
-                           const double* src, double* w)
+template <bool FWD>
+__device__ __noinline__ void cta_sweep(const Team<1>& T, const SmallSystem& S, const double* src,
+                                       double* w)
 {
     const int nW = S.nWave;
     if (nW <= 0) return;
@@ -193,7 +196,7 @@ __device__ __noinline__ void team_sweep(const Team<C>& T, const SmallSystem& S, 
     auto hi = [&](int q) { return S.waveStart[FWD ? q + 1 : nW - q]; };
     int r0 = lo(0), r1 = hi(0);
     RowPre cur;
-    sweep_pre<C, FWD>(S, coef, src, r0 + T.g < r1 ? r0 + T.g : -1, cur);
+    sweep_pre<FWD>(S, src, r0 + T.g < r1 ? r0 + T.g : -1, cur);
     for (int q = 0; q < nW; ++q) {
         int n0 = 0, n1 = 0;
         if (q + 1 < nW) {
@@ -201,12 +204,12 @@ __device__ __noinline__ void team_sweep(const Team<C>& T, const SmallSystem& S, 
             n1 = hi(q + 1);
         }
         RowPre nxt;
-        sweep_pre<C, FWD>(S, coef, src, n0 + T.g < n1 ? n0 + T.g : -1, nxt);
-        if (cur.i >= 0) w[cur.i] = sweep_row<C, FWD>(S, coef, cur, w);
+        sweep_pre<FWD>(S, src, n0 + T.g < n1 ? n0 + T.g : -1, nxt);
+        if (cur.i >= 0) w[cur.i] = sweep_row<FWD>(S, cur, w);
         for (int i = r0 + T.g + T.stride; i < r1; i += T.stride) {
             RowPre more;
-            sweep_pre<C, FWD>(S, coef, src, i, more);
-            w[i] = sweep_row<C, FWD>(S, coef, more, w);
+            sweep_pre<FWD>(S, src, i, more);
+            w[i] = sweep_row<FWD>(S, more, w);
         }
         T.sync();
         cur = nxt;
@@ -215,10 +218,97 @@ __device__ __noinline__ void team_sweep(const Team<C>& T, const SmallSystem& S, 
     }
 }
 
-// w = M^-1 r (unapMatrixPrecond.cpp, lduDiagPrecond.cpp:44-73,
-// lduDICPrecond.cpp:45-77, lduDILUPrecond.cpp:46-86)
+// both sweeps of a cluster, by value (flow_dic_kernel's arithmetic); wf and w
+// hold 0xff bytes on entry
 template <int C>
-__device__ void team_precond(const Team<C>& T, const SmallSystem& S, const double* r, double* w)
+__device__ __noinline__ void cluster_sweeps(const SmallSystem& S, const double* r, double* wf,
+                                            double* w)
+{
+    constexpr int CK = 6;
+    const int lane = (int)threadIdx.x & 31;
+    const int slot = (int)(threadIdx.x >> 5) * C + (int)(blockIdx.x % C);
+    const int step = C * (int)(blockDim.x >> 5);
+    const Rows<double>& A = S.A;
+    const int nT = S.nTasks;
+    for (int t = slot; t < 2 * nT; t += step) {
+        const bool bwd = t >= nT;
+        const int q = bwd ? 2 * nT - 1 - t : t;
+        const int4 D = ldg(S.task + q);
+        const int2 nr = ldg(S.near + q);
+        const int i = D.x + lane;
+        const bool on = lane < D.y;
+        int cnt = 0, first = 0;
+        const int dir = bwd ? -32 : 32;
+        double acc = 0.0;
+        if (on) {
+            const int info = ldg(A.rowInfo + i);
+            const int len = info & 0xffff, nLow = info >> 16;
+            cnt = bwd ? len - nLow : nLow;
+            first = D.z + lane + (bwd ? 32 * (len - 1) : 0);
+            if (!bwd) acc = ldg(S.rD + i) * __ldcg(r + i);
+        }
+        const int most = __reduce_max_sync(0xffffffffu, cnt);
+        double* out = bwd ? w : wf;
+        const int wait = bwd ? nr.y : nr.x;
+        int j0 = 0;
+        do {
+            int c[CK];
+            double v[CK], xv[CK + 1];
+            unsigned need = 0;
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                const int e = first + dir * (j0 + k);
+                const bool has = j0 + k < cnt;
+                c[k] = has ? ldg(A.col + e) : 0;
+                v[k] = has ? ldg(S.f + e) : 0.0;
+                xv[k] = 0.0;
+                if (has) need |= 1u << k;
+            }
+            xv[CK] = 0.0;
+            if (bwd && on && j0 == 0) need |= 1u << CK;
+            if (j0 == 0 && wait >= 0) wait_near(out + wait, S.err);
+            wait_values<double, CK + 1>(
+                need, [&](int k) { return k == CK ? wf + i : (const double*)out + c[k]; }, xv,
+                S.err);
+            if (bwd && j0 == 0) acc = xv[CK];
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                if (j0 + k >= most) break;
+                xv[k] = v[k] * xv[k];
+            }
+#pragma unroll
+            for (int k = 0; k < CK; ++k) {
+                if (j0 + k >= most) break;
+                const double less = acc - xv[k];
+                acc = j0 + k < cnt ? less : acc;
+            }
+            j0 += CK;
+        } while (j0 < most);
+        if (on) st_flow(out + i, acc);
+    }
+}
+
+// the value of a row that is not there yet
+__device__ __forceinline__ double no_value() { return __longlong_as_double(-1ll); }
+
+// marks this thread's row i of the vectors of the next application; a team
+// barrier stands between this and the application
+template <int C>
+__device__ __forceinline__ void clear_row(const SmallSystem& S, double* wf, double* w, int i)
+{
+    if constexpr (C > 1) {
+        if (S.precond < 2) return;
+        wf[i] = no_value();
+        w[i] = no_value();
+    }
+}
+
+// w = M^-1 r (unapMatrixPrecond.cpp, lduDiagPrecond.cpp:44-73,
+// lduDICPrecond.cpp:45-77, lduDILUPrecond.cpp:46-86); with C > 1 the rows of
+// wf and w were cleared before
+template <int C>
+__device__ void team_precond(const Team<C>& T, const SmallSystem& S, const double* r, double* wf,
+                             double* w)
 {
     const Rows<double>& A = S.A;
     const int n = A.n;
@@ -228,8 +318,13 @@ __device__ void team_precond(const Team<C>& T, const SmallSystem& S, const doubl
         T.sync();
         return;
     }
-    team_sweep<C, true>(T, S, S.precond == 3 ? A.val : A.valT, r, w);
-    team_sweep<C, false>(T, S, A.val, w, w);
+    if constexpr (C == 1) {
+        cta_sweep<true>(T, S, r, w);
+        cta_sweep<false>(T, S, w, w);
+    } else {
+        cluster_sweeps<C>(S, r, wf, w);
+        T.sync();
+    }
 }
 
 template <int C>
@@ -240,15 +335,19 @@ __device__ void team_pcg(Team<C>& T, const SmallSystem& S, SmallResult& R)
     double* p = S.work;
     double* w = S.work + n;
     double* r = S.work + 2 * n;
+    double* wf = S.work + 3 * n;
     team_spmv(T, S.A, x, w);
-    for (int i = T.g; i < n; i += T.stride) r[i] = ldv<C>(S.b + i) - ldv<C>(w + i);
+    for (int i = T.g; i < n; i += T.stride) {
+        r[i] = ldv<C>(S.b + i) - ldv<C>(w + i);
+        clear_row<C>(S, wf, w, i);
+    }
     T.sync();
     R.initRes = sqrt(team_dot(T, n, r, r)) + SMALL_D;
     R.finalRes = R.initRes;
     double wArA = 1.0e37, wArAold;
     for (;;) {
         wArAold = wArA;
-        team_precond(T, S, r, w);
+        team_precond(T, S, r, wf, w);
         wArA = team_dot(T, n, w, r);
         if (!(fabs(wArA) > SMALL_D)) {
             R.singular = 1;
@@ -265,6 +364,7 @@ __device__ void team_pcg(Team<C>& T, const SmallSystem& S, SmallResult& R)
         for (int i = T.g; i < n; i += T.stride) {
             x[i] = ldv<C>(x + i) + alpha * ldv<C>(p + i);
             r[i] = ldv<C>(r + i) - alpha * ldv<C>(w + i);
+            clear_row<C>(S, wf, w, i);
         }
         T.sync();
         R.finalRes = sqrt(team_dot(T, n, r, r)) + SMALL_D;
@@ -287,11 +387,13 @@ __device__ void team_bicgstab(Team<C>& T, const SmallSystem& S, SmallResult& R)
     double* s = S.work + 5 * n;
     double* z = S.work + 6 * n;
     double* t = S.work + 7 * n;
+    double* wf = S.work + 8 * n;
     team_spmv(T, S.A, x, y);
     for (int i = T.g; i < n; i += T.stride) {
         const double ri = ldv<C>(S.b + i) - ldv<C>(y + i);
         r[i] = ri;
         r0[i] = ri;
+        clear_row<C>(S, wf, y, i);
     }
     T.sync();
     R.initRes = sqrt(team_dot(T, n, r, r)) + SMALL_D;
@@ -312,10 +414,13 @@ __device__ void team_bicgstab(Team<C>& T, const SmallSystem& S, SmallResult& R)
                 p[i] = ldv<C>(r + i) + beta * (ldv<C>(p + i) - omega * ldv<C>(Ay + i));
         }
         T.sync();
-        team_precond(T, S, p, y);
+        team_precond(T, S, p, wf, y);
         team_spmv(T, S.A, y, Ay);
         alpha = rA0rA / team_dot(T, n, r0, Ay);
-        for (int i = T.g; i < n; i += T.stride) s[i] = ldv<C>(r + i) - alpha * ldv<C>(Ay + i);
+        for (int i = T.g; i < n; i += T.stride) {
+            s[i] = ldv<C>(r + i) - alpha * ldv<C>(Ay + i);
+            clear_row<C>(S, wf, z, i);
+        }
         T.sync();
         R.finalRes = sqrt(team_dot(T, n, s, s)) + SMALL_D;
         if (check_conv(R.finalRes, R.initRes, S.tol, S.relTol, R.nIter + 1, S.minIter)) {
@@ -325,7 +430,7 @@ __device__ void team_bicgstab(Team<C>& T, const SmallSystem& S, SmallResult& R)
             R.nIter++;
             return;
         }
-        team_precond(T, S, s, z);
+        team_precond(T, S, s, wf, z);
         team_spmv(T, S.A, z, t);
         const double tAtA = team_dot(T, n, t, t);
         omega = team_dot(T, n, t, s);
@@ -333,6 +438,7 @@ __device__ void team_bicgstab(Team<C>& T, const SmallSystem& S, SmallResult& R)
         for (int i = T.g; i < n; i += T.stride) {
             x[i] = ldv<C>(x + i) + (alpha * ldv<C>(y + i) + omega * ldv<C>(z + i));
             r[i] = ldv<C>(s + i) - omega * ldv<C>(t + i);
+            clear_row<C>(S, wf, y, i);
         }
         T.sync();
         R.finalRes = sqrt(team_dot(T, n, r, r)) + SMALL_D;

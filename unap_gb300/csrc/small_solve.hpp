@@ -13,6 +13,9 @@ struct TeamShape {
     int cluster = 1;
 };
 
+// work vectors of a whole solve
+constexpr int kTeamWorkPcg = 4, kTeamWorkBicg = 9;
+
 struct SmallResult {
     int nIter, converged, singular, pad;
     double initRes, finalRes;
@@ -23,6 +26,11 @@ struct SmallSystem {
     const int* waveStart;       // device, nWave + 1
     int nWave;
     const double* rD;           // 1/D (Diag) or factored reciprocal (DIC/DILU)
+    const double* f;            // DIC/DILU: entries times their row's rD (DicFlow)
+    const int4* task;           // the level's sweep tasks (SweepTasks, a lane a row)
+    const int2* near;
+    int nTasks;
+    int* err;                   // set when a sweep's wait ran out
     int method;                 // 0 PCG, 1 PBiCGStab
     int precond;                // 0 none, 1 Diag, 2 DIC, 3 DILU
     double tol, relTol;
@@ -30,7 +38,7 @@ struct SmallSystem {
     int zeroX;                  // start from x = 0
     double* x;
     const double* b;
-    double* work;               // 8 n doubles
+    double* work;               // kTeamWorkPcg n or kTeamWorkBicg n doubles
     SmallResult* result;        // may be null
 };
 
