@@ -334,7 +334,14 @@ void MgSolver::vcycle()
         Lv& N = lv[(size_t)c + 2];
         k_restrict<double>(ex, N.n, N.childStart.p, N.child.p, C.src.p, N.src.p, Gate{});
     }
-    if (L >= 0) launch_small_krylov(ex.s, coarseSys.p, 1, nullptr);
+    if (L >= 0) {
+        // one CTA with a thread a row: its barriers and block sums, a few tens
+        // an iteration, cost less with fewer warps (the idle warps' zeros do
+        // not change a sum)
+        const int nc = lv[(size_t)L + 1].n;
+        launch_small_krylov(ex.s, coarseSys.p, 1, nullptr,
+                            nc <= 128 ? 128 : nc <= 256 ? 256 : kSmallBlock);
+    }
     for (int c = L - 1; c >= 0; --c) {
         Lv& C = lv[(size_t)c + 1];
         Lv& N = lv[(size_t)c + 2];
