@@ -548,10 +548,10 @@ int unap_cuda_set_matrix_wavefronts(int on);
  * in the reference. */
 int unap_cuda_set_cheby_chunk(int entries);
 /* Chebyshev V-cycles run their coarse levels of at most `rows` rows (and
- * every level below them, at most 8 above the coarsest) in one
- * thread-block-cluster launch instead of a launch per step (0: never).
- * Results are identical.  Returns the previous value; applies to AMG
- * handles created afterwards.  No counterpart in the reference. */
+ * every level below them) in one launch instead of a launch per step
+ * (default 60000; 0: never).  Results are identical.  Returns the previous
+ * value; applies to AMG handles created afterwards.  No counterpart in the
+ * reference. */
 int unap_cuda_set_cheby_tail_rows(int rows);
 
 /* Coarse-level tail of the AMG V-cycle (per-step executor), set for the FP64

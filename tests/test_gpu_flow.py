@@ -91,3 +91,30 @@ def test_nan_and_inf_inputs(cuda, orc, pattern):
             A.precondition(2, torch.tensor(b, device="cuda"), x)
             assert np.array_equal(x.cpu().numpy(), orc.precond(2, s, b)[0], equal_nan=True)
     A.close()
+
+
+@pytest.mark.parametrize("degree", [1, 3, 4])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_chebyshev_tail_long_rows(cuda, precision, degree):
+    """The Chebyshev tail from level 1 on a hierarchy whose rows are longer
+    than the entries a task holds at once: the bits of a launch per step."""
+    torch = cuda
+    s = random_system(3000, 60000, 11, symm=True)
+    s.upper = s.upper * 0 - np.abs(s.upper)
+    s.diag = W._fast_row_abs_sum(s.n, s.lower_addr, s.upper_addr, s.upper, s.upper) + 0.1
+    A = capi.DeviceMatrix(s)
+    r = torch.tensor(np.random.default_rng(3).standard_normal(s.n), device="cuda")
+    out = []
+    for rows in (0, 1 << 30):
+        old = capi.set_cheby_tail_rows(rows)
+        try:
+            G = capi.DeviceAmg(A, n_coarsest=70, precision=precision, smoother=1,
+                               cheby_degree=degree)
+        finally:
+            capi.set_cheby_tail_rows(old)
+        z = torch.zeros_like(r)
+        G.vcycle(r, z)
+        out.append(z.cpu().numpy())
+        G.close()
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+    A.close()

@@ -189,15 +189,20 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
     if (params.smoother == 1) setupCheby(s);
     tail_cluster_size();  // function attributes and the cluster query, outside any capture
     // the Chebyshev levels of at most cheby_tail_rows() rows, and all below,
-    // in one cluster launch
-    if (params.smoother == 1 && cheby_tail_rows() > 0 && cheby_tail_cluster() > 0) {
+    // in one launch
+    if (params.smoother == 1 && cheby_tail_rows() > 0) {
         for (int k = std::max(1, params.chebyFrom); k < L; ++k)
-            if (lv[(size_t)k].n <= cheby_tail_rows() && L - k <= kChebTailMaxLevels) {
+            if (lv[(size_t)k].n <= cheby_tail_rows() &&
+                cheb_flow_stages(L - k, params.chebyDegree) <= kChebTailMaxStages) {
                 chebTail = k;
                 break;
             }
-        if (chebTail > 0)
-            chebTailPart.alloc((size_t)nc * (size_t)((nc + kDenseChunk - 1) / kDenseChunk));
+        if (chebTail > 0) {
+            if (params.precision == 1)
+                buildChebTail<float>(s);
+            else
+                buildChebTail<double>(s);
+        }
     }
     phase(5);
     setupSeconds =
@@ -220,7 +225,7 @@ std::vector<int> AmgHierarchy::levelWavefronts() const
 
 size_t AmgHierarchy::deviceBytes() const
 {
-    size_t b = Minv.bytes();
+    size_t b = Minv.bytes() + tail32.bytes() + tail64.bytes();
     for (size_t k = 0; k < lv.size(); ++k) {
         const Lv& l = lv[k];
         if (l.own) b += l.own->deviceBytes();
@@ -327,6 +332,8 @@ std::vector<double> AmgHierarchy::eigenvalues() const
 void AmgHierarchy::check() const
 {
     for (auto& l : lv) l.sweeps.check();
+    tail32.check();
+    tail64.check();
 }
 
 int AmgHierarchy::tailFirst(size_t elemBytes) const
@@ -426,42 +433,29 @@ void AmgHierarchy::sweep(const Exec& ex, int k, const Level& Lk, const Rows<T>& 
     }
 }
 
+template <>
+ChebFlow<float>& AmgHierarchy::chebFlow<float>()
+{
+    return tail32;
+}
+template <>
+ChebFlow<double>& AmgHierarchy::chebFlow<double>()
+{
+    return tail64;
+}
+
 template <class T>
-ChebTailArgs<T> AmgHierarchy::chebTailArgs(int k)
+void AmgHierarchy::buildChebTail(cudaStream_t s)
 {
     const int L = nLevels() - 1;
-    ChebTailArgs<T> a{};
-    a.nLev = L - k;
-    a.deg = params.chebyDegree;
-    for (int l = 0; l < a.nLev; ++l) {
-        const int kk = k + l;
-        Lv& V = lv[(size_t)kk];
-        ChebTailLevel<T>& t = a.lev[l];
-        t.A = rowsT<T>(*V.L);
-        t.childStart = V.childStart.p;
-        t.child = V.child.p;
-        t.cmap = V.cmap.p;
-        t.x = X<T>(kk);
-        t.b = B<T>(kk);
-        t.w = R<T>(kk);
-        t.cb[0] = chebBuf<T>(kk, 0);
-        t.cb[1] = chebBuf<T>(kk, 1);
-        t.post = (params.chebyDegree % 2 == 0) ? X<T>(kk) : Tmp<T>(kk);
-        t.Rth = (T)V.Rth;
-        for (int j = 0; j < kChebyMaxDegree; ++j) {
-            t.d1[j] = (T)V.d1[j];
-            t.d2[j] = (T)V.d2[j];
-        }
+    std::vector<ChebFlowLevel<T>> lev;
+    for (int k = chebTail; k < L; ++k) {
+        const Lv& V = lv[(size_t)k];
+        lev.push_back({rowsT<T>(*V.L), V.childStart.p, V.child.p, V.cmap.p, V.Rth, V.d1, V.d2});
     }
-    a.nc = nc;
-    a.cChildStart = lv[(size_t)L].childStart.p;
-    a.cChild = lv[(size_t)L].child.p;
-    a.cCmap = lv[(size_t)L].cmap.p;
-    a.cb = B<T>(L);
-    a.cx = X<T>(L);
-    a.Minv = Minv.p;
-    a.part = chebTailPart.p;
-    return a;
+    const Lv& C = lv[(size_t)L];
+    chebFlow<T>().build(lev, params.chebyDegree, R<T>(chebTail - 1), nc, C.childStart.p, C.child.p,
+                        C.cmap.p, Minv.p, X<T>(chebTail), s);
 }
 
 template <class T>
@@ -477,7 +471,7 @@ const T* AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
         return x;
     }
     if (k == chebTail) {
-        launch_cheb_tail<T>(ex, chebTailArgs<T>(k), g);
+        chebFlow<T>().launch(ex, g);
         if (profOut) UNAP_CK(cudaEventRecordWithFlags((*profOut)[(size_t)k], ex.s, cudaEventRecordExternal));
         return x;
     }
@@ -515,7 +509,9 @@ const T* AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
     }
     k_residual<T>(ex, Rk, cur, b, r, RSpec{}, g);
     const Lv& C = lv[(size_t)k + 1];
-    if (isCheby(k + 1))
+    if (k + 1 == chebTail)
+        ;  // the tail restricts
+    else if (isCheby(k + 1))
         k_restrict_cheb_zero<T>(ex, C.n, C.childStart.p, C.child.p, r, B<T>(k + 1),
                                 rowsT<T>(*C.L).diag, chebBuf<T>(k + 1, 0), R<T>(k + 1),
                                 (T)C.Rth, g);

@@ -150,11 +150,14 @@ private:
     template <class T>
     void launch_tail(const Exec& ex, int t, Gate g);
     int curTail = -1;
-    // first level of the Chebyshev cluster tail (launch_cheb_tail), -1: none
+    // first level of the Chebyshev tail (one launch, cheb_flow.cu), -1: none
     int chebTail = -1;
-    DevArray<double> chebTailPart;  // its coarsest chunk sums
+    ChebFlow<float> tail32;
+    ChebFlow<double> tail64;
     template <class T>
-    ChebTailArgs<T> chebTailArgs(int k);
+    ChebFlow<T>& chebFlow();
+    template <class T>
+    void buildChebTail(cudaStream_t s);
     std::vector<cudaEvent_t>* profIn = nullptr;   // per-level events (profiling)
     std::vector<cudaEvent_t>* profOut = nullptr;
     template <class T>

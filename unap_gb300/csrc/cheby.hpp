@@ -74,58 +74,55 @@ template <class T>
 void k_prolong_add_to(const Exec& ex, int n, const int* cmap, const T* coarse, const T* xin,
                       T* xout, Gate g);
 
-// ---- the coarse end of a Chebyshev V-cycle in one cluster launch --------
-constexpr int kChebTailMaxLevels = 8;
+// ---- the coarse end of a Chebyshev V-cycle in one launch (cheb_flow.cu) --
+constexpr int kChebTailRows = 60000;   // default of set_cheby_tail_rows
+constexpr int kChebTailMaxStages = 600;
+constexpr int kChebTailCtas = 8;       // CTAs of 128 threads an SM at most
 
 // one tail level: its matrix, the restriction into it (children of each
-// cell, ascending), the prolongation out of it (cmap: finer row -> cell),
-// its vectors (x, b, w = the residual buffer, the two buffers of the step
-// chain: step j writes cb[j & 1], the post-smoothing chain starting from
-// `post`) and Chebyshev coefficients
+// cell, ascending), the prolongation from it (finer row -> cell) and its
+// Chebyshev coefficients
 template <class T>
-struct ChebTailLevel {
+struct ChebFlowLevel {
     Rows<T> A;
     const int* childStart;
     const int* child;
     const int* cmap;
-    T* x;
-    T* b;
-    T* w;
-    T* cb[2];
-    T* post;
-    T Rth;
-    T d1[kChebyMaxDegree];
-    T d2[kChebyMaxDegree];
+    double Rth;
+    const double* d1;
+    const double* d2;
 };
 
+// stages of a tail of `levels` levels above the coarsest
+inline int cheb_flow_stages(int levels, int deg) { return levels * (2 * deg + 2) + 3; }
+
 template <class T>
-struct ChebTailArgs {
-    ChebTailLevel<T> lev[kChebTailMaxLevels];  // first tail level .. coarsest - 1
-    int nLev;
-    int deg;
-    int nc;                   // coarsest level
-    const int* cChildStart;   // restriction into it
-    const int* cChild;
-    const int* cCmap;         // prolongation out of it
-    T* cb;
-    T* cx;
-    const double* Minv;       // dense inverse, column-major
-    double* part;             // nc x ceil(nc / 64) chunk sums (scratch)
+struct ChebFlow {
+    DevArray<unsigned char> arena;   // task counters, then every stage's vectors
+    DevArray<unsigned char> stages;
+    int nStages = 0, nTasks = 0, nc = 0, grid = 0;
+    const double* M = nullptr;
+    double* part = nullptr;
+    int* err = nullptr;              // pinned: set when a wait ran out
+    ChebFlow() = default;
+    ChebFlow(const ChebFlow&) = delete;
+    ChebFlow& operator=(const ChebFlow&) = delete;
+    ~ChebFlow();
+    // levels in order, finest first; rIn: the residual of the level above
+    // the first; result: where the first level's iterate goes
+    void build(const std::vector<ChebFlowLevel<T>>& lev, int deg, const T* rIn, int nc,
+               const int* cChildStart, const int* cChild, const int* cCmap, const double* Minv,
+               T* result, cudaStream_t s);
+    void launch(const Exec& ex, Gate g) const;
+    void check() const;  // throws when a wait ran out (after synchronizing)
+    size_t bytes() const { return arena.bytes() + stages.bytes(); }
 };
 
-// One launch of a thread-block cluster (16 CTAs of 512 threads, else 8)
-// runs the V-cycle from a.lev[0] (its b, first iterate and w already set by
-// the fused restriction) down to the coarsest and back, bit-identical to the
-// per-step kernels.
-template <class T>
-void launch_cheb_tail(const Exec& ex, const ChebTailArgs<T>& a, Gate g);
 // Chebyshev V-cycles run their levels of at most `rows` rows (and every
 // level below them) in the tail launch; 0 turns it off.  Returns the
 // previous value; applies to hierarchies built afterwards.
 int set_cheby_tail_rows(int rows);
 int cheby_tail_rows();
-// cluster size the tail launches with on this device (0: none schedulable)
-int cheby_tail_cluster();
 
 // Rows per level below which Chebyshev-step launches use one-warp CTAs
 // (spread over more SMs); returns the previous value.
