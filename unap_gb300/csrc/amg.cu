@@ -79,32 +79,10 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
         lv[(size_t)k].own = build_level(c.A, &key, k == L, s, !isCheby(k));
         lv[(size_t)k].L = lv[(size_t)k].own.get();
         lv[(size_t)k].n = nC;
-        const Level& Cl = *lv[(size_t)k].L;
-        // restriction: children of every coarse cell, ascending finer cell
-        // index (the summation order of restrictField), in internal indices
-        std::vector<int> refStart((size_t)nC + 1, 0);
-        for (int i = 0; i < F.n; ++i) refStart[(size_t)c.restrictAddr[(size_t)i] + 1]++;
-        for (int C = 0; C < nC; ++C) refStart[(size_t)C + 1] += refStart[(size_t)C];
-        std::vector<int> refChild((size_t)F.n);
-        {
-            std::vector<int> pos(refStart.begin(), refStart.end() - 1);
-            for (int i = 0; i < F.n; ++i) refChild[(size_t)pos[(size_t)c.restrictAddr[(size_t)i]]++] = i;
-        }
-        std::vector<int> cs((size_t)nC + 1, 0), ch((size_t)F.n);
-        for (int Ci = 0; Ci < nC; ++Ci) {
-            int C = Cl.perm[(size_t)Ci];
-            int len = refStart[(size_t)C + 1] - refStart[(size_t)C];
-            cs[(size_t)Ci + 1] = cs[(size_t)Ci] + len;
-            for (int j = 0; j < len; ++j)
-                ch[(size_t)(cs[(size_t)Ci] + j)] = F.iperm[(size_t)refChild[(size_t)(refStart[(size_t)C] + j)]];
-        }
-        std::vector<int> cmap((size_t)F.n);
-        for (int i = 0; i < F.n; ++i) cmap[(size_t)i] = Cl.iperm[(size_t)c.restrictAddr[(size_t)F.perm[(size_t)i]]];
-        lv[(size_t)k].childStart.upload(cs, s);
-        lv[(size_t)k].child.upload(ch, s);
-        lv[(size_t)k].cmap.upload(cmap, s);
-        UNAP_CK(cudaStreamSynchronize(s));
+        transfer_maps(F, *lv[(size_t)k].L, c.restrictAddr, lv[(size_t)k].childStart,
+                      lv[(size_t)k].child, lv[(size_t)k].cmap, s);
     }
+    UNAP_CK(cudaStreamSynchronize(s));
     phase(1);
     // coarsest: dense FP64 inverse (identity internal order when L >= 1)
     const HostLdu& Ch = L ? coarse[(size_t)L - 1].A : A.host;

@@ -32,6 +32,15 @@ std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, const std::vecto
 bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, CoarseHost& out,
                               std::vector<double>& cw, int& nCoarse, cudaStream_t s);
 std::vector<double> mg_face_weights(const HostLdu& A);
+// Transfers between a level and the one its cells aggregate into (agg: cell
+// -> coarse cell, reference numbering), in internal rows: the children of
+// coarse row r are child[childStart[r] ..], ascending finer cell (the
+// summation order of restrictField), and cmap[i] is the coarse row of finer
+// row i.  Made by kernels on levels of at least device_setup_min_cells()
+// cells; agg has to live until the stream is synchronized.
+void transfer_maps(const Level& F, const Level& C, const std::vector<int>& agg,
+                   DevArray<int>& childStart, DevArray<int>& child, DevArray<int>& cmap,
+                   cudaStream_t s);
 
 struct AmgParams {
     int nCoarsest = 1000;

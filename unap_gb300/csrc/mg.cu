@@ -142,29 +142,9 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
         lv[(size_t)k].own = build_level(c.A, &key, false, s);
         lv[(size_t)k].L = lv[(size_t)k].own.get();
         lv[(size_t)k].n = c.A.n;
-        const Level& Cl = *lv[(size_t)k].L;
         const int nc = c.A.n;
-        std::vector<int> refStart((size_t)nc + 1, 0);
-        for (int i = 0; i < F.n; ++i) refStart[(size_t)c.restrictAddr[(size_t)i] + 1]++;
-        for (int C = 0; C < nc; ++C) refStart[(size_t)C + 1] += refStart[(size_t)C];
-        std::vector<int> refChild((size_t)F.n);
-        {
-            std::vector<int> pos(refStart.begin(), refStart.end() - 1);
-            for (int i = 0; i < F.n; ++i) refChild[(size_t)pos[(size_t)c.restrictAddr[(size_t)i]]++] = i;
-        }
-        std::vector<int> cs((size_t)nc + 1, 0), ch((size_t)F.n), cmap((size_t)F.n);
-        for (int Ci = 0; Ci < nc; ++Ci) {
-            int C = Cl.perm[(size_t)Ci];
-            int len = refStart[(size_t)C + 1] - refStart[(size_t)C];
-            cs[(size_t)Ci + 1] = cs[(size_t)Ci] + len;
-            for (int j = 0; j < len; ++j)
-                ch[(size_t)(cs[(size_t)Ci] + j)] = F.iperm[(size_t)refChild[(size_t)(refStart[(size_t)C] + j)]];
-        }
-        for (int i = 0; i < F.n; ++i) cmap[(size_t)i] = Cl.iperm[(size_t)c.restrictAddr[(size_t)F.perm[(size_t)i]]];
         Lv& K = lv[(size_t)k];
-        K.childStart.upload(cs, s);
-        K.child.upload(ch, s);
-        K.cmap.upload(cmap, s);
+        transfer_maps(F, *K.L, c.restrictAddr, K.childStart, K.child, K.cmap, s);
         K.corr.alloc((size_t)nc);
         K.src.alloc((size_t)nc);
         UNAP_CK(cudaStreamSynchronize(s));
