@@ -199,7 +199,7 @@ int unap_cuda_matrix_layout(long int handle, int* nWavefronts, int* perm, int* w
 /* Matrices (and AMG levels) of at least minCells cells build their device
  * structure (internal order, SELL-32 layout, values) with kernels instead
  * of host loops; minCells < 0 builds every one on the host.  Both give the
- * same structure bit for bit.  Default 32768; the previous value is
+ * same structure bit for bit.  Default 8192; the previous value is
  * returned through the (nullable) pointer.  No reference counterpart. */
 int unap_cuda_set_device_setup(long long minCells, long long* oldMinCells);
 

@@ -215,14 +215,13 @@ void coarse_coefficients(const HostLdu& fine, CoarseHost& c)
     C.validate();
 }
 
-std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, const std::vector<double>& weights,
+std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, std::vector<double> w,
                                            int nCoarsest, int maxLevels, int stopRule,
                                            cudaStream_t s)
 {
     if (maxLevels <= 0) maxLevels = 50;
     if (nCoarsest <= 0) nCoarsest = 50;
     std::vector<CoarseHost> levels;
-    std::vector<double> w = weights;
     while ((int)levels.size() < maxLevels - 1) {
         const HostLdu& fm = levels.empty() ? fine : levels.back().A;
         if (stopRule == 1 && fm.n <= nCoarsest) break;
@@ -263,7 +262,9 @@ std::vector<double> mg_face_weights(const HostLdu& A)
     for (int f = 0; f < A.nf; ++f) s += A.upper[(size_t)f] * A.upper[(size_t)f];
     double avg = std::sqrt(s);
     std::vector<double> w((size_t)A.nf);
-    for (int f = 0; f < A.nf; ++f) w[(size_t)f] = std::fabs(A.upper[(size_t)f]) / avg;
+    parallel_ranges(A.nf, 65536, [&](int f0, int f1) {
+        for (int f = f0; f < f1; ++f) w[(size_t)f] = std::fabs(A.upper[(size_t)f]) / avg;
+    });
     return w;
 }
 

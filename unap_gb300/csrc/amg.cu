@@ -58,7 +58,7 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
     };
     std::vector<double> w = mg_face_weights(A.host);
     std::vector<CoarseHost> coarse =
-        agglomerate_levels(A.host, w, params.nCoarsest, params.maxLevels, 1, s);
+        agglomerate_levels(A.host, std::move(w), params.nCoarsest, params.maxLevels, 1, s);
     phase(0);
     const int L = (int)coarse.size();
     lv.resize((size_t)L + 1);

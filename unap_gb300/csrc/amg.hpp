@@ -26,7 +26,7 @@ void coarse_coefficients(const HostLdu& fine, CoarseHost& c);
 // cells); stopRule 1: agglomerate until the coarsest has <= nCoarsest cells.
 // Levels of at least device_setup_min_cells() cells are agglomerated by
 // kernels on stream s (aggl_dev.cu), with the same result.
-std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, const std::vector<double>& weights,
+std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, std::vector<double> weights,
                                            int nCoarsest, int maxLevels, int stopRule,
                                            cudaStream_t s = 0);
 bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, CoarseHost& out,

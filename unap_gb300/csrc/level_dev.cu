@@ -302,6 +302,162 @@ __global__ void k_bfs_assign(Adj A, const int* __restrict__ F, int m, const int*
     }
 }
 
+// The three phases above for one BFS level after another, by one cluster
+// of kBfsCtas CTAs: a launch per phase, the scan and a read-back cost 48 us a
+// level and a hex grid has as many levels as its edges are long together
+// (9.6 ms at 508,200 cells), a level here about 8: three cluster barriers and
+// the phases' loads.  CTA q takes the q-th part of the frontier, so the ranks
+// of its discoveries follow those of the CTAs before it; their counts meet in
+// distributed shared memory.  Stops at an empty frontier, or at one of more
+// than `limit` cells, which all SMs expand faster.  state: {frontier size,
+// next rank, 1 when the frontier is in fb, 1 when ranks ran past n}.
+constexpr int kBfsCtas = 8;
+constexpr int kBfsThreads = 1024;
+constexpr int kBfsLimit = 32768;
+
+__device__ __forceinline__ void bfs_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kBfsThreads)
+    k_bfs_levels(Adj A, int* fa, int* fb, int* rank, unsigned long long* disc, int* won, int n,
+                 int limit, int* state)
+{
+    __shared__ int found;
+    const int q = (int)blockIdx.x;  // one cluster
+    int m = state[0], base = state[1], flip = state[2], bad = 0;
+    bfs_sync();  // everybody has read the state before anybody writes it
+    while (m > 0 && m <= limit && !bad) {
+        const int* F = flip ? fb : fa;
+        int* N = flip ? fa : fb;
+        const int part = (m + kBfsCtas - 1) / kBfsCtas;
+        const int lo = min(q * part, m), hi = min(lo + part, m);
+        // Vectors written in this launch are read from L2.  A thread's first
+        // cell with up to kHeld neighbours (nearly all of them) keeps these in
+        // registers with a bit for each unvisited one, so that the later
+        // phases read only disc.
+        constexpr int kHeld = 8;
+        const int mineP = lo + (int)threadIdx.x;
+        int nb[kHeld];
+        unsigned open = 0;
+        bool held = false;
+        if (mineP < hi) {
+            const int v = __ldcg(F + mineP), lowN = A.low(v), dg = A.deg(v);
+            held = dg <= kHeld;
+            if (held) {
+                int r[kHeld];
+#pragma unroll
+                for (int j = 0; j < kHeld; ++j) nb[j] = j < dg ? A.nbr(v, j, lowN) : v;
+#pragma unroll
+                for (int j = 0; j < kHeld; ++j) r[j] = j < dg ? __ldcg(rank + nb[j]) : 0;
+#pragma unroll
+                for (int j = 0; j < kHeld; ++j)
+                    if (r[j] < 0) {
+                        open |= 1u << j;
+                        atomicMin(&disc[nb[j]], claim_key(mineP, j));
+                    }
+            }
+        }
+        for (int p = held ? mineP + kBfsThreads : mineP; p < hi; p += kBfsThreads) {
+            const int v = __ldcg(F + p), lowN = A.low(v), dg = A.deg(v);
+            for (int j = 0; j < dg; ++j) {
+                const int w = A.nbr(v, j, lowN);
+                if (__ldcg(rank + w) < 0) atomicMin(&disc[w], claim_key(p, j));
+            }
+        }
+        bfs_sync();
+        if (held) {
+            unsigned long long d[kHeld];
+#pragma unroll
+            for (int j = 0; j < kHeld; ++j) d[j] = open >> j & 1u ? __ldcg(disc + nb[j]) : 0;
+#pragma unroll
+            for (int j = 0; j < kHeld; ++j)
+                if ((open >> j & 1u) && d[j] != claim_key(mineP, j)) open &= ~(1u << j);
+        }
+        int mine = 0;  // discoveries of this CTA's part
+        for (int p0 = lo; p0 < hi; p0 += kBfsThreads) {
+            const int p = p0 + (int)threadIdx.x;
+            int c = 0;
+            if (p == mineP && held) {
+                c = __popc(open);
+            } else if (p < hi) {
+                const int v = __ldcg(F + p), lowN = A.low(v), dg = A.deg(v);
+                for (int j = 0; j < dg; ++j) {
+                    const int w = A.nbr(v, j, lowN);
+                    c += (__ldcg(rank + w) < 0 && __ldcg(disc + w) == claim_key(p, j));
+                }
+            }
+            int tot;
+            const int ex = block_exclusive_scan(c, &tot);
+            if (p < hi) won[p] = mine + ex;
+            mine += tot;
+        }
+        if (threadIdx.x == 0) found = mine;
+        bfs_sync();
+        int before = 0, total = 0;
+        for (int k = 0; k < kBfsCtas; ++k) {
+            unsigned a = (unsigned)__cvta_generic_to_shared(&found), ra;
+            int t;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(k));
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(t) : "r"(ra) : "memory");
+            if (k < q) before += t;
+            total += t;
+        }
+        if (total > n - base) bad = 1;  // cannot happen: each cell is won once
+        if (held && !bad) {
+            int t = before + won[mineP];
+#pragma unroll
+            for (int j = 0; j < kHeld; ++j)
+                if (open >> j & 1u) {
+                    __stcg(rank + nb[j], base + t);
+                    __stcg(N + t, nb[j]);
+                    ++t;
+                }
+        }
+        for (int p = held ? mineP + kBfsThreads : mineP; p < hi && !bad; p += kBfsThreads) {
+            const int v = __ldcg(F + p), lowN = A.low(v), dg = A.deg(v);
+            int t = before + won[p];
+            for (int j = 0; j < dg; ++j) {
+                const int w = A.nbr(v, j, lowN);
+                if (__ldcg(rank + w) < 0 && __ldcg(disc + w) == claim_key(p, j)) {
+                    __stcg(rank + w, base + t);
+                    __stcg(N + t, w);
+                    ++t;
+                }
+            }
+        }
+        bfs_sync();
+        base += total;
+        m = total;
+        flip ^= 1;
+    }
+    if (q == 0 && threadIdx.x == 0) {
+        state[0] = m;
+        state[1] = base;
+        state[2] = flip;
+        state[3] = bad;
+    }
+}
+
+void bfs_levels(Adj A, int* fa, int* fb, int* rank, unsigned long long* disc, int* won, int n,
+                int* state, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kBfsCtas);
+    cfg.blockDim = dim3(kBfsThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kBfsCtas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    UNAP_CK(cudaLaunchKernelEx(&cfg, k_bfs_levels, A, fa, fb, rank, disc, won, n, kBfsLimit, state));
+}
+
 // smallest cell >= from that is unvisited (with needNbr != 0: and has at
 // least one neighbour), atomically minimised into *best
 __global__ void k_first_unvisited(Adj A, int from, int n, const int* rank, int needNbr, int* best)
@@ -551,7 +707,9 @@ struct Readback {
     }
 };
 
-std::atomic<long long> g_deviceMinCells{32768};
+// The hierarchy of a 508,200-cell log-normal system took 50.7 / 44.0 / 43.2 /
+// 44.4 / 48.7 ms to set up with this at 32768 / 16384 / 8192 / 4096 / 1024.
+std::atomic<long long> g_deviceMinCells{8192};
 
 }  // namespace
 
@@ -682,10 +840,27 @@ std::unique_ptr<Level> build_level_device(const HostLdu& A, const std::vector<in
             k_set<<<1, 1, 0, s>>>(rank + seed, nextRank);
             k_set<<<1, 1, 0, s>>>(fa.p, seed);
             ++nextRank;
-            int* F = fa.p;
-            int* G = fb.p;
-            int m = 1;
+            Scratch<int> state(4, s);
+            int m = 1, flip = 0;
             for (;;) {
+                int* F = flip ? fb.p : fa.p;
+                int* G = flip ? fa.p : fb.p;
+                if (m <= kBfsLimit / 2) {
+                    rb.h[0] = m;
+                    rb.h[1] = nextRank;
+                    rb.h[2] = flip;
+                    rb.h[3] = 0;
+                    UNAP_CK(cudaMemcpyAsync(state.p, rb.h, 4 * sizeof(int), cudaMemcpyHostToDevice, s));
+                    bfs_levels(adj, fa.p, fb.p, rank, disc.p, won.p, n, state.p, s);
+                    UNAP_CK(cudaMemcpyAsync(rb.h, state.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
+                    UNAP_CK(cudaStreamSynchronize(s));
+                    if (rb.h[3]) return nullptr;
+                    m = rb.h[0];
+                    nextRank = rb.h[1];
+                    flip = rb.h[2];
+                    if (m == 0) break;
+                    continue;
+                }
                 k_bfs_claim<<<grid_for(m), kThreads, 0, s>>>(adj, F, m, rank, disc.p);
                 k_bfs_count<<<grid_for(m), kThreads, 0, s>>>(adj, F, m, rank, disc.p, won.p);
                 exclusive_scan(won.p, won.p, m, s);
@@ -696,7 +871,7 @@ std::unique_ptr<Level> build_level_device(const HostLdu& A, const std::vector<in
                                                               disc.p, G);
                 nextRank += t;
                 m = t;
-                std::swap(F, G);
+                flip ^= 1;
             }
             UNAP_CK(cudaGetLastError());
             from = seed + 1;
@@ -714,7 +889,13 @@ std::unique_ptr<Level> build_level_device(const HostLdu& A, const std::vector<in
     L->d_perm.alloc((size_t)n);
     L->d_iperm.alloc((size_t)n);
     Scratch<int> ws((size_t)nWave + 1, s);
-    {
+    if (!wavefronts) {
+        // one range: the key order itself
+        UNAP_CK(cudaMemcpyAsync(L->d_perm.p, byKey.p, sizeof(int) * (size_t)n,
+                                cudaMemcpyDeviceToDevice, s));
+        k_set<<<1, 1, 0, s>>>(ws.p, 0);
+        k_set<<<1, 1, 0, s>>>(ws.p + 1, n);
+    } else {
         const long long nChunks = (n + kSplitChunk - 1) / kSplitChunk;
         Scratch<int> cnt((size_t)(nChunks * nWave), s), tot((size_t)nWave, s);
         UNAP_CK(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (size_t)(nChunks * nWave), s));
