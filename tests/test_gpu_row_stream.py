@@ -1,0 +1,41 @@
+"""Products over large levels: a warp walks over several slices, fetching ahead.
+
+The products are bit-identical to the oracle's (the same entry order and
+roundings, tolerance zero) at the sizes where the walk can go wrong: the last
+block of 256 rows and the last slice partly filled, rows longer than the eight
+entries held in registers, products of -0, rows without entries.  The dot
+products sum the same terms as the oracle's in another order: at most n eps =
+6e-11 of the sum of their magnitudes, so three iterations of a
+well-conditioned solve agree to 1e-9.
+"""
+import numpy as np
+import pytest
+
+from test_gpu_flow import random_system
+from unap_gb300 import capi
+
+pytestmark = pytest.mark.gpu
+
+LIMIT = 1 << 19  # rows from which FP64 levels are walked
+
+
+@pytest.mark.parametrize("n,per_row", [(LIMIT, 2.2), (LIMIT + 1, 3.0), (LIMIT + 31 * 256 + 45, 0.3),
+                                       (LIMIT - 1, 2.2)])
+@pytest.mark.parametrize("symm", [True, False])
+def test_products_and_dots(cuda, orc, n, per_row, symm):
+    torch = cuda
+    s = random_system(n, int(per_row * n), n % 97, symm=symm, near=9000)
+    A = capi.DeviceMatrix(s)
+    x = np.random.default_rng(n).standard_normal(n)
+    x[::5] = -0.0
+    y = torch.empty(n, dtype=torch.float64, device="cuda")
+    A.spmv(torch.tensor(x, device="cuda"), y)
+    want = orc.spmv(s, x)
+    assert np.array_equal(y.cpu().numpy().view(np.int64), want.view(np.int64))
+    z = torch.zeros(n, dtype=torch.float64, device="cuda")
+    A.krylov_solve(0 if symm else 1, 1, z, torch.tensor(s.b, device="cuda"),
+                   rel_tol=0.0, max_iter=3)
+    ref = (orc.pcg if symm else orc.pbicgstab)(s, 1, s.b, rel_tol=0.0, max_iter=3)
+    xr, _ = ref
+    assert np.abs(z.cpu().numpy() - xr).max() <= 1e-9 * np.abs(xr).max()
+    A.close()

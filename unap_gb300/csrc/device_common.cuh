@@ -60,24 +60,23 @@ __device__ __forceinline__ void block_sum(double (&v)[K])
 // launch's last block (ticket) sums them in block order into launch slot
 // r.slot; when r.fin asks for it, that block sums slots 0..nSlots-1 in order
 // and calls fin(t) on one thread.
+// Only the thread that wrote a partial fences it before the ticket.
 template <int K, class F>
-__device__ __forceinline__ void reduce_launch(double (&v)[K], const RSpec& r, F&& fin)
+__device__ __forceinline__ void reduce_partials(int nPart, const RSpec& r, F&& fin)
 {
-    block_sum<K>(v);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) r.blockPart[blockIdx.x * K + k] = v[k];
-    }
-    __threadfence();
     __shared__ int amLast;
-    if (threadIdx.x == 0) amLast = (atomicAdd(r.ticket, 1u) == gridDim.x - 1) ? 1 : 0;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        amLast = (atomicAdd(r.ticket, 1u) == gridDim.x - 1) ? 1 : 0;
+    }
     __syncthreads();
     if (!amLast) return;
     __threadfence();
     double s[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) s[k] = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+#pragma unroll(K == 1 ? 16 : 4)
+    for (int b = threadIdx.x; b < nPart; b += blockDim.x) {
 #pragma unroll
         for (int k = 0; k < K; ++k) s[k] += __ldcg(r.blockPart + b * K + k);
     }
@@ -98,6 +97,17 @@ __device__ __forceinline__ void reduce_launch(double (&v)[K], const RSpec& r, F&
         }
         __threadfence();
     }
+}
+
+template <int K, class F>
+__device__ __forceinline__ void reduce_launch(double (&v)[K], const RSpec& r, F&& fin)
+{
+    block_sum<K>(v);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) r.blockPart[blockIdx.x * K + k] = v[k];
+    }
+    reduce_partials<K>((int)gridDim.x, r, fin);
 }
 
 // solverPerformance::checkConvergence, unapMatrixTest.cpp:3-31

@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "device_common.cuh"
+#include "row_stream.hpp"
 
 namespace unapgpu {
 
@@ -72,6 +73,10 @@ void k_spmv(const Exec& ex, const Rows<T>& A, const T* x, T* y, const T* dotWith
             Gate g, bool fused)
 {
     if (A.n <= 0) return;
+    if (row_streams(A, red)) {
+        stream_spmv<T>(ex, A, x, y, dotWith, red, g, fused);
+        return;
+    }
     const T* dw = red.blockPart ? dotWith : nullptr;
     const dim3 grid = ex.rowGrid(A.n, red);
     tick();
@@ -108,6 +113,10 @@ template <class T>
 void k_residual(const Exec& ex, const Rows<T>& A, const T* x, const T* b, T* r, RSpec red, Gate g)
 {
     if (A.n <= 0) return;
+    if (row_streams(A, red) && !red.blockPart) {
+        stream_residual<T>(ex, A, x, b, r, g);
+        return;
+    }
     if (A.wide)
         tick(), residual_kernel<T, 16><<<ex.rowGrid(A.n, red), kBlock, 0, ex.s>>>(A, x, b, r, red, g);
     else
