@@ -1,4 +1,4 @@
-"""Products over large levels: a warp walks over several slices, fetching ahead.
+"""Products over large levels, where a warp walks over several slices, and in the caller's order.
 
 The products are bit-identical to the oracle's (the same entry order and
 roundings, tolerance zero) at the sizes where the walk can go wrong: the last
@@ -38,4 +38,20 @@ def test_products_and_dots(cuda, orc, n, per_row, symm):
     ref = (orc.pcg if symm else orc.pbicgstab)(s, 1, s.b, rel_tol=0.0, max_iter=3)
     xr, _ = ref
     assert np.abs(z.cpu().numpy() - xr).max() <= 1e-9 * np.abs(xr).max()
+    A.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 5000, 40_000, LIMIT - 1, LIMIT])
+@pytest.mark.parametrize("shift", [None, 0, 1, 32])
+def test_products_in_the_callers_order(cuda, orc, n, shift):
+    """y apart from x, x itself, or x moved by some entries."""
+    torch = cuda
+    s = random_system(n, int(2.2 * n) if n > 1 else 0, n % 89, near=min(n, 9000) if n > 1 else None)
+    A = capi.DeviceMatrix(s)
+    x = np.random.default_rng(n).standard_normal(n)
+    buf = torch.zeros(2 * n + 32, dtype=torch.float64, device="cuda")
+    buf[:n] = torch.tensor(x)
+    at = n if shift is None else min(shift, n)
+    A.spmv(buf[:n], buf[at:at + n])
+    assert np.array_equal(buf[at:at + n].cpu().numpy(), orc.spmv(s, x))
     A.close()

@@ -156,17 +156,20 @@ __device__ __forceinline__ T lds(const T* p)
 // the mixed-precision solve's FP64 outer loop, where GB300's FP64 pipe and
 // not the bytes bounds the SpMV; FM = false keeps the reference's separate
 // roundings.
-template <class T, int XL = XL_NC, bool ST = false, int CK = 8, bool FM = false>
-__device__ __forceinline__ T row_apply(const Rows<T>& A, int r, const T* x)
+// MAP: column c's entry is x[map[c]].
+template <class T, int XL = XL_NC, bool ST = false, int CK = 8, bool FM = false, bool MAP = false>
+__device__ __forceinline__ T row_apply(const Rows<T>& A, int r, const T* x,
+                                       const int* map = nullptr)
 {
+    auto at = [&](int c) { return MAP ? ldg(map + c) : c; };
     const int info = lds<ST>(A.rowInfo + r);
     const int len = info & 0xffff;
     const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
     T acc = T(0);
     if constexpr (FM)
-        acc = lds<ST>(A.diag + r) * ldx<XL>(x + r);
+        acc = lds<ST>(A.diag + r) * ldx<XL>(x + at(r));
     else
-        acc += lds<ST>(A.diag + r) * ldx<XL>(x + r);
+        acc += lds<ST>(A.diag + r) * ldx<XL>(x + at(r));
     for (int j0 = 0; j0 < len; j0 += CK) {
         int c[CK];
         T v[CK], xv[CK];
@@ -177,7 +180,7 @@ __device__ __forceinline__ T row_apply(const Rows<T>& A, int r, const T* x)
             v[k] = j0 + k < len ? lds<ST>(A.val + e) : T(0);
         }
 #pragma unroll
-        for (int k = 0; k < CK; ++k) xv[k] = ldx<XL>(x + c[k]);
+        for (int k = 0; k < CK; ++k) xv[k] = ldx<XL>(x + at(c[k]));
 #pragma unroll
         for (int k = 0; k < CK; ++k)
             if (j0 + k < len) {

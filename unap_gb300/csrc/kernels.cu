@@ -498,6 +498,47 @@ void k_to_reference(const Exec& ex, int n, const int* perm, const T* in, T* out)
     if (n > 0) tick(), to_reference_kernel<T><<<ex.grid(n), kBlock, 0, ex.s>>>(n, perm, in, out);
 }
 
+// y = A x in the caller's order: the row's position there is looked up where
+// the row is stored and, MAP, the columns' where they are gathered.
+template <class T, int CK, bool MAP>
+__global__ void __launch_bounds__(kBlock)
+    spmv_reference_kernel(Rows<T> A, const int* __restrict__ perm, const T* __restrict__ x, T* y)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= A.n) return;
+    const int at = ldg(perm + r);
+    y[at] = row_apply<T, XL_NC, true, CK, false, MAP>(A, r, x, perm);
+}
+
+// Below this many rows one launch looks up every column's position: the
+// lookups hit the caches and cost less than a launch that copies x into
+// internal order first.  A whole call, us, copy first against lookups: 16.7
+// and 13.6 at 20^3, 21.8 and 19.0 at 50^3, 36.9 and 33.4 at 80^3, 50.2 and
+// 52.5 at 100^3, 299 and 481 at 200^3.  (With the result scattered by a launch
+// of its own as well: 22.7 at 20^3, 384 at 200^3.)
+static constexpr int kLookupRows = 1 << 19;
+
+template <class T>
+void k_spmv_reference(const Exec& ex, const Rows<T>& A, const int* perm, const T* x, T* y, T* xi)
+{
+    if (A.n <= 0) return;
+    // an x that y overlaps is copied first
+    const bool apart = x + A.n <= y || y + A.n <= x;
+    const bool look = A.n < kLookupRows && apart;
+    if (!look) k_to_internal<T>(ex, A.n, perm, x, xi);
+    if (!look && row_streams(A, RSpec{})) {
+        stream_spmv_reference<T>(ex, A, perm, xi, y);
+        return;
+    }
+    tick();
+    auto f = look ? (A.wide ? spmv_reference_kernel<T, 16, true> : spmv_reference_kernel<T, 8, true>)
+                  : (A.wide ? spmv_reference_kernel<T, 16, false>
+                            : spmv_reference_kernel<T, 8, false>);
+    // up to one CTA of kBlock an SM: narrower ones, over more SMs
+    const int threads = A.n <= 152 * kBlock ? 64 : kBlock;
+    f<<<div_up(A.n, threads), threads, 0, ex.s>>>(A, perm, look ? x : xi, y);
+}
+
 // restrictField (unapMatrix.hpp:378-407) in gather form: children ascending
 template <class T>
 __global__ void restrict_kernel(int nc, const int* __restrict__ cs, const int* __restrict__ ch,
@@ -757,6 +798,7 @@ int device_max_blocks()
 #define INST(T)                                                                                   \
     template void k_spmv<T>(const Exec&, const Rows<T>&, const T*, T*, const T*, RSpec, Gate,      \
                             bool);                                                               \
+    template void k_spmv_reference<T>(const Exec&, const Rows<T>&, const int*, const T*, T*, T*); \
     template void k_residual<T>(const Exec&, const Rows<T>&, const T*, const T*, T*, RSpec, Gate); \
     template void k_gs_rows<T>(const Exec&, const Rows<T>&, T*, const T*, int, int, bool, Gate);   \
     template void gs_sweep<T>(const Exec&, const Level&, const Rows<T>&, T*, const T*, bool, bool, \

@@ -30,7 +30,7 @@ namespace unapgpu {
 
 namespace {
 
-enum Op : int { OP_SPMV, OP_RESIDUAL };
+enum Op : int { OP_SPMV, OP_SPMV_PERM, OP_RESIDUAL };
 
 template <class T>
 struct StreamArgs {
@@ -39,6 +39,7 @@ struct StreamArgs {
     const T* b;    // right-hand side, or the vector of the dot product (null: none)
     T* out;
     RSpec red;
+    const int* perm;  // OP_SPMV_PERM: where a row's result goes
 };
 
 // 0 + v
@@ -139,10 +140,12 @@ __global__ void __launch_bounds__(kBlock)
     for (int blk = blockIdx.x; blk < nBlocks; blk += gridDim.x, s += step) {
         const int r = 32 * s + lane;
         const bool on = r < a.A.n;
+        int to = r;
         T xv[K], xr = T(0), bb = T(0);
         if (on) {
             xr = ldg(a.x + r);
             if (a.b) bb = ldg(a.b + r);
+            if (OP == OP_SPMV_PERM) to = lds<true>(a.perm + r);
         }
 #pragma unroll
         for (int k = 0; k < K; ++k)
@@ -192,11 +195,10 @@ __global__ void __launch_bounds__(kBlock)
                 }
         }
         if (on) {
-            if constexpr (OP == OP_SPMV) {
-                a.out[r] = acc;
-            } else {
+            if constexpr (OP == OP_RESIDUAL)
                 a.out[r] = bb - acc;
-            }
+            else
+                a.out[to] = acc;
         }
         if constexpr (DOT) {
             double v = 0.0;
@@ -274,6 +276,13 @@ void stream_spmv(const Exec& ex, const Rows<T>& A, const T* x, T* y, const T* do
 }
 
 template <class T>
+void stream_spmv_reference(const Exec& ex, const Rows<T>& A, const int* perm, const T* x, T* y)
+{
+    StreamArgs<T> a{A, x, nullptr, y, RSpec{}, perm};
+    launch<T, OP_SPMV_PERM, false, false>(ex, a, Gate{});
+}
+
+template <class T>
 void stream_residual(const Exec& ex, const Rows<T>& A, const T* x, const T* b, T* r, Gate g)
 {
     StreamArgs<T> a{A, x, b, r, RSpec{}};
@@ -284,6 +293,7 @@ void stream_residual(const Exec& ex, const Rows<T>& A, const T* x, const T* b, T
     template bool row_streams<T>(const Rows<T>&, const RSpec&);                                   \
     template void stream_spmv<T>(const Exec&, const Rows<T>&, const T*, T*, const T*, RSpec, Gate, \
                                  bool);                                                           \
+    template void stream_spmv_reference<T>(const Exec&, const Rows<T>&, const int*, const T*, T*); \
     template void stream_residual<T>(const Exec&, const Rows<T>&, const T*, const T*, T*, Gate);
 UNAP_STREAM_INST(float)
 UNAP_STREAM_INST(double)

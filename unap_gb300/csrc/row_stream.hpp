@@ -23,6 +23,9 @@ bool row_streams(const Rows<T>& A, const RSpec& red);
 template <class T>
 void stream_spmv(const Exec& ex, const Rows<T>& A, const T* x, T* y, const T* dotWith, RSpec red,
                  Gate g, bool fused);
+// y = A x with y in the order that perm gives
+template <class T>
+void stream_spmv_reference(const Exec& ex, const Rows<T>& A, const int* perm, const T* x, T* y);
 // r = b - A x (k_residual without a reduction)
 template <class T>
 void stream_residual(const Exec& ex, const Rows<T>& A, const T* x, const T* b, T* r, Gate g);
