@@ -270,32 +270,53 @@ void AmgHierarchy::setupCheby(cudaStream_t s)
         if (isCheby(k)) nMax = std::max(nMax, (size_t)lv[(size_t)k].n);
     if (!nMax) return;
     DevArray<double> x(nMax), b(nMax), rD(nMax), rA(nMax), wA(nMax), pA(nMax);
-    DevArray<EigState> es(1);
+    DevArray<EigState> es(kEigSet);
     RedPool pool;
-    pool.init(2, ex.maxBlocks, 1, s);
-    for (int k = 0; k < L; ++k) {
-        if (!isCheby(k)) continue;
-        Lv& V = lv[(size_t)k];
-        const Level& Lk = *V.L;
-        const int n = V.n;
+    pool.init(2 * kEigSet, ex.maxBlocks, 1, s);
+    // as many levels at once as the largest one's vectors hold
+    for (int k = 0; k < L;) {
+        std::vector<int> set;
+        size_t rows = 0;
+        for (; k < L && (int)set.size() < kEigSet; ++k) {
+            if (!isCheby(k)) continue;
+            if (rows + (size_t)lv[(size_t)k].n > nMax) break;
+            rows += (size_t)lv[(size_t)k].n;
+            set.push_back(k);
+        }
+        if (set.empty()) continue;
         // eigenDiagPCG from x = 0 on b = the splitmix64 start vector, FP64
-        k_fill<double>(ex, n, x.p, 0.0);
-        k_eig_start(ex, n, Lk.d_perm.p, b.p);
-        k_reciprocal(ex, n, Lk.d_diag.p, rD.p);
-        EigState h{};
-        h.wArA = 1.0e37;  // GREAT, eigenDiagPCG.cpp:75
-        UNAP_CK(cudaMemcpyAsync(es.p, &h, sizeof(EigState), cudaMemcpyHostToDevice, s));
-        eig_diag_pcg(ex, rows64(Lk), rD.p, x.p, b.p, rA.p, wA.p, pA.p, es.p,
-                     pool.site(0, nullptr, FIN_RES_ONLY), pool.site(1, nullptr, FIN_RES_ONLY), 10);
-        k_eig_sturm(ex, es.p, 10);
-        UNAP_CK(cudaMemcpyAsync(&h, es.p, sizeof(EigState), cudaMemcpyDeviceToHost, s));
+        k_fill<double>(ex, (int)rows, x.p, 0.0);
+        std::vector<EigLevel> E;
+        std::vector<const double*> rhs;
+        size_t at = 0;
+        for (int j : set) {
+            const Level& Lj = *lv[(size_t)j].L;
+            const int n = lv[(size_t)j].n, i = (int)E.size();
+            k_eig_start(ex, n, Lj.d_perm.p, b.p + at);
+            k_reciprocal(ex, n, Lj.d_diag.p, rD.p + at);
+            E.push_back(EigLevel{rows64(Lj), rD.p + at, x.p + at, rA.p + at, wA.p + at, pA.p + at,
+                                 es.p + i, pool.site(2 * i, nullptr, FIN_RES_ONLY),
+                                 pool.site(2 * i + 1, nullptr, FIN_RES_ONLY)});
+            rhs.push_back(b.p + at);
+            at += (size_t)n;
+        }
+        std::vector<EigState> h(set.size(), EigState{});
+        for (EigState& e : h) e.wArA = 1.0e37;  // GREAT, eigenDiagPCG.cpp:75
+        const size_t bytes = h.size() * sizeof(EigState);
+        UNAP_CK(cudaMemcpyAsync(es.p, h.data(), bytes, cudaMemcpyHostToDevice, s));
+        eig_diag_pcg(ex, E.data(), (int)E.size(), rhs.data(), 10);
+        k_eig_sturm(ex, es.p, 10, (int)E.size());
+        UNAP_CK(cudaMemcpyAsync(h.data(), es.p, bytes, cudaMemcpyDeviceToHost, s));
         UNAP_CK(cudaStreamSynchronize(s));
-        V.lam = h.maxEig;
-        cheby_coeffs(V.lam, params.eigRatio, params.chebyDegree, &V.Rth, V.d1, V.d2);
-        if (params.precision == 1)
-            V.tf.alloc((size_t)n);
-        else
-            V.t.alloc((size_t)n);
+        for (size_t i = 0; i < set.size(); ++i) {
+            Lv& V = lv[(size_t)set[i]];
+            V.lam = h[i].maxEig;
+            cheby_coeffs(V.lam, params.eigRatio, params.chebyDegree, &V.Rth, V.d1, V.d2);
+            if (params.precision == 1)
+                V.tf.alloc((size_t)V.n);
+            else
+                V.t.alloc((size_t)V.n);
+        }
     }
     UNAP_CK(cudaStreamSynchronize(s));
 }

@@ -314,9 +314,10 @@ int unap_cuda_cheby_smooth_host(long int handle, double* x, const double* b, int
             EigState st{};
             st.wArA = 1.0e37;  // GREAT, eigenDiagPCG.cpp:75
             UNAP_CK(cudaMemcpyAsync(es.p, &st, sizeof st, cudaMemcpyHostToDevice, A.stream));
-            eig_diag_pcg(ex, R, rD.p, xi.p, bi.p, t.p, w.p, pA.p, es.p,
-                         pool.site(0, nullptr, FIN_RES_ONLY), pool.site(1, nullptr, FIN_RES_ONLY),
-                         10);
+            EigLevel E{R, rD.p, xi.p, t.p, w.p, pA.p, es.p, pool.site(0, nullptr, FIN_RES_ONLY),
+                       pool.site(1, nullptr, FIN_RES_ONLY)};
+            const double* rhs = bi.p;
+            eig_diag_pcg(ex, &E, 1, &rhs, 10);
             k_eig_sturm(ex, es.p, 10);
             UNAP_CK(cudaMemcpyAsync(&st, es.p, sizeof st, cudaMemcpyDeviceToHost, A.stream));
             UNAP_CK(cudaStreamSynchronize(A.stream));

@@ -25,19 +25,41 @@ std::atomic<int> g_chunk{0};
 constexpr int kChunk8Rows = 1 << 20;
 
 // ---- eigenDiagPCG::diagPCGLoops (eigenDiagPCG.cpp:48-238) ----------------
-__global__ void __launch_bounds__(kBlock) eig_wr_kernel(int n, const double* __restrict__ rD,
-                                                        const double* __restrict__ rA,
-                                                        double* __restrict__ wA, EigState* es,
-                                                        int it, RSpec red)
+// One launch for the same step of several levels: level k has nBlocks CTAs
+// from block0 on and reduces among them.  A step of a level of a hierarchy
+// takes microseconds whatever its size (launch, gathers, two trees of FP64
+// sums), so ten levels one after another took ten times as long: 110x66x70
+// setup took 5.6 ms for its estimates, this 2.7.
+struct EigSet {
+    int n = 0;
+    EigLevel lv[kEigSet];
+};
+static_assert(sizeof(EigSet) <= 4096);
+
+__device__ __forceinline__ const EigLevel& eig_level(const EigSet& S)
 {
+    int k = 0;
+    while (k + 1 < S.n && (int)blockIdx.x >= S.lv[k + 1].block0) ++k;
+    return S.lv[k];
+}
+
+#define EIG_ROWS(i, L)                                                                \
+    for (int i = ((int)blockIdx.x - L.block0) * blockDim.x + threadIdx.x; i < L.A.n; \
+         i += L.nBlocks * blockDim.x)
+
+__global__ void __launch_bounds__(kBlock) eig_wr_kernel(const __grid_constant__ EigSet S, int it)
+{
+    const EigLevel& L = eig_level(S);
+    EigState* es = L.es;
     if (es->broken) return;
     double v[1] = {0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double w = rD[i] * rA[i];
-        wA[i] = w;
-        v[0] += w * rA[i];
+    EIG_ROWS(i, L)
+    {
+        double w = L.rD[i] * L.rA[i];
+        L.wA[i] = w;
+        v[0] += w * L.rA[i];
     }
-    reduce_launch<1>(v, red, [&](const double (&t)[1]) {
+    reduce_ctas<1>(v, L.wr, (int)blockIdx.x - L.block0, L.nBlocks, [&](const double (&t)[1]) {
         es->wArAold = es->wArA;
         es->wArA = t[0];
         if (fabs(es->wArA) < VSMALL_D) {
@@ -51,50 +73,51 @@ __global__ void __launch_bounds__(kBlock) eig_wr_kernel(int n, const double* __r
     });
 }
 
-__global__ void eig_p_kernel(int n, const double* __restrict__ wA, double* __restrict__ pA,
-                             const EigState* es, int it)
+__global__ void eig_p_kernel(const __grid_constant__ EigSet S, int it)
 {
-    if (es->broken) return;
-    const double beta = es->beta;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        pA[i] = it == 0 ? wA[i] : wA[i] + beta * pA[i];
+    const EigLevel& L = eig_level(S);
+    if (L.es->broken) return;
+    const double beta = L.es->beta;
+    EIG_ROWS(i, L)
+    L.pA[i] = it == 0 ? L.wA[i] : L.wA[i] + beta * L.pA[i];
 }
 
-__global__ void __launch_bounds__(kBlock) eig_alpha_kernel(Rows<double> A,
-                                                           const double* __restrict__ pA,
-                                                           double* __restrict__ wA, EigState* es,
-                                                           int it, RSpec red)
+__global__ void __launch_bounds__(kBlock) eig_alpha_kernel(const __grid_constant__ EigSet S, int it)
 {
+    const EigLevel& L = eig_level(S);
+    EigState* es = L.es;
     if (es->broken) return;
     double v[1] = {0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
-        double w = row_apply<double>(A, i, pA);
-        wA[i] = w;
-        v[0] += w * pA[i];
+    EIG_ROWS(i, L)
+    {
+        double w = row_apply<double>(L.A, i, L.pA);
+        L.wA[i] = w;
+        v[0] += w * L.pA[i];
     }
-    reduce_launch<1>(v, red, [&](const double (&t)[1]) {
+    reduce_ctas<1>(v, L.al, (int)blockIdx.x - L.block0, L.nBlocks, [&](const double (&t)[1]) {
         es->wApA = t[0];
         es->alpha = es->wArA / es->wApA;
         es->alphas[it] = es->alpha;
     });
 }
 
-__global__ void eig_update_kernel(int n, double* __restrict__ x, double* __restrict__ rA,
-                                  const double* __restrict__ pA, const double* __restrict__ wA,
-                                  const EigState* es)
+__global__ void eig_update_kernel(const __grid_constant__ EigSet S)
 {
-    if (es->broken) return;
-    const double alpha = es->alpha;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        x[i] += alpha * pA[i];
-        rA[i] -= alpha * wA[i];
+    const EigLevel& L = eig_level(S);
+    if (L.es->broken) return;
+    const double alpha = L.es->alpha;
+    EIG_ROWS(i, L)
+    {
+        L.x[i] += alpha * L.pA[i];
+        L.rA[i] -= alpha * L.wA[i];
     }
 }
 
 // Lanczos tridiagonal + Sturm-sequence bisection to 1e-5 (k = 1), over the
 // iterations the diagonal PCG completed
-__global__ void eig_sturm_kernel(EigState* es, int nMax)
+__global__ void eig_sturm_kernel(EigState* all, int nMax)
 {
+    EigState* es = all + blockIdx.x;
     int nP = 0;
     while (nP < nMax && nP < 16 && es->alphas[nP] != 0.0) ++nP;
     if (nP < 2) {
@@ -291,29 +314,35 @@ int set_cheby_chunk(int entries)
     return g_chunk.exchange(entries);
 }
 
-void eig_diag_pcg(const Exec& ex, const Rows<double>& A, const double* rD, double* x,
-                  const double* b, double* rA, double* wA, double* pA, EigState* es,
-                  const RSpec& wr, const RSpec& al, int nIt)
+void eig_diag_pcg(const Exec& ex, EigLevel* lv, int count, const double* const* b, int nIt)
 {
-    const int n = A.n;
-    k_residual<double>(ex, A, x, b, rA, RSpec{}, Gate{});  // rA = b - A x
+    if (count < 1 || count > kEigSet) throw std::invalid_argument("too many levels at once");
+    EigSet S;
+    int blocks = 0;
+    for (int k = 0; k < count; ++k) {
+        EigLevel& L = S.lv[S.n++] = lv[k];
+        L.block0 = blocks;
+        L.nBlocks = ex.grid(L.A.n);
+        blocks += L.nBlocks;
+        k_residual<double>(ex, L.A, L.x, b[k], L.rA, RSpec{}, Gate{});  // rA = b - A x
+    }
     for (int it = 0; it < nIt; ++it) {
         tick();
-        eig_wr_kernel<<<ex.grid(n), kBlock, 0, ex.s>>>(n, rD, rA, wA, es, it, wr);
+        eig_wr_kernel<<<blocks, kBlock, 0, ex.s>>>(S, it);
         tick();
-        eig_p_kernel<<<ex.grid(n), kBlock, 0, ex.s>>>(n, wA, pA, es, it);
+        eig_p_kernel<<<blocks, kBlock, 0, ex.s>>>(S, it);
         tick();
-        eig_alpha_kernel<<<ex.grid(n), kBlock, 0, ex.s>>>(A, pA, wA, es, it, al);
+        eig_alpha_kernel<<<blocks, kBlock, 0, ex.s>>>(S, it);
         tick();
-        eig_update_kernel<<<ex.grid(n), kBlock, 0, ex.s>>>(n, x, rA, pA, wA, es);
+        eig_update_kernel<<<blocks, kBlock, 0, ex.s>>>(S);
     }
     UNAP_CK(cudaGetLastError());
 }
 
-void k_eig_sturm(const Exec& ex, EigState* es, int nMax)
+void k_eig_sturm(const Exec& ex, EigState* es, int nMax, int count)
 {
     tick();
-    eig_sturm_kernel<<<1, 1, 0, ex.s>>>(es, nMax);
+    eig_sturm_kernel<<<count, 1, 0, ex.s>>>(es, nMax);
     UNAP_CK(cudaGetLastError());
 }
 

@@ -26,19 +26,29 @@ struct EigState {
     double maxEig;
 };
 
-// eigenDiagPCG::diagPCGLoops: nIt (<= 16) diagonal-PCG iterations on
-// (x, b), x updated in place.  es must hold wArA = GREAT and zeros on entry;
-// a breakdown (|wArA| < VSMALL) sets es->broken and leaves the remaining
-// alphas 0.  rA, wA, pA: n-vector scratch; wr and al: two reduction sites.
-void eig_diag_pcg(const Exec& ex, const Rows<double>& A, const double* rD, double* x,
-                  const double* b, double* rA, double* wA, double* pA, EigState* es,
-                  const RSpec& wr, const RSpec& al, int nIt);
+// A level whose largest eigenvalue is estimated.  x: start, updated in place.
+// es must hold wArA = GREAT and zeros on entry.  rA, wA, pA: n-vector scratch;
+// wr and al: two reduction sites of its own.
+struct EigLevel {
+    Rows<double> A;
+    const double* rD;
+    double *x, *rA, *wA, *pA;
+    EigState* es;
+    RSpec wr, al;
+    int block0 = 0, nBlocks = 0;  // set by eig_diag_pcg
+};
+constexpr int kEigSet = 16;
+
+// eigenDiagPCG::diagPCGLoops on each of `count` (<= kEigSet) levels: nIt
+// (<= 16) diagonal-PCG iterations on (x, b).  A breakdown (|wArA| < VSMALL)
+// sets es->broken and leaves the remaining alphas 0.
+void eig_diag_pcg(const Exec& ex, EigLevel* lv, int count, const double* const* b, int nIt);
 
 // eigenDiagPCG::computeMaxEig (eigenDiagPCG.cpp:242-361) on one device
 // thread: es->maxEig = the largest eigenvalue of the Lanczos tridiagonal of
 // the iterations done (nonzero alphas, at most nMax <= 16) by Sturm-sequence
 // bisection to a band of 1e-5; 1 / alpha_0 after one iteration, 1 after none.
-void k_eig_sturm(const Exec& ex, EigState* es, int nMax);
+void k_eig_sturm(const Exec& ex, EigState* es, int nMax, int count = 1);
 
 // Start vector of the AMG levels' eigenvalue estimate: cell c (reference
 // numbering of its level) gets a uniform value in [-1, 1) from splitmix64.

@@ -61,13 +61,14 @@ __device__ __forceinline__ void block_sum(double (&v)[K])
 // r.slot; when r.fin asks for it, that block sums slots 0..nSlots-1 in order
 // and calls fin(t) on one thread.
 // Only the thread that wrote a partial fences it before the ticket.
+// nCta CTAs arrive with nPart partials between them.
 template <int K, class F>
-__device__ __forceinline__ void reduce_partials(int nPart, const RSpec& r, F&& fin)
+__device__ __forceinline__ void reduce_partials(int nPart, int nCta, const RSpec& r, F&& fin)
 {
     __shared__ int amLast;
     if (threadIdx.x == 0) {
         __threadfence();
-        amLast = (atomicAdd(r.ticket, 1u) == gridDim.x - 1) ? 1 : 0;
+        amLast = (atomicAdd(r.ticket, 1u) == (unsigned)nCta - 1) ? 1 : 0;
     }
     __syncthreads();
     if (!amLast) return;
@@ -99,15 +100,23 @@ __device__ __forceinline__ void reduce_partials(int nPart, const RSpec& r, F&& f
     }
 }
 
+// this CTA is the blk-th of nCta
 template <int K, class F>
-__device__ __forceinline__ void reduce_launch(double (&v)[K], const RSpec& r, F&& fin)
+__device__ __forceinline__ void reduce_ctas(double (&v)[K], const RSpec& r, int blk, int nCta,
+                                            F&& fin)
 {
     block_sum<K>(v);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) r.blockPart[blockIdx.x * K + k] = v[k];
+        for (int k = 0; k < K; ++k) r.blockPart[blk * K + k] = v[k];
     }
-    reduce_partials<K>((int)gridDim.x, r, fin);
+    reduce_partials<K>(nCta, nCta, r, fin);
+}
+
+template <int K, class F>
+__device__ __forceinline__ void reduce_launch(double (&v)[K], const RSpec& r, F&& fin)
+{
+    reduce_ctas<K>(v, r, (int)blockIdx.x, (int)gridDim.x, fin);
 }
 
 // solverPerformance::checkConvergence, unapMatrixTest.cpp:3-31

@@ -228,16 +228,13 @@ void MgSolver::eigen_estimate(int slot, int k, double* xk, const double* bk)
 {
     // eigenDiagPCG ctor: 10 diagonal-PCG iterations on (x, b), x updated
     Lv& K = lv[(size_t)k];
-    const int n = K.n;
     EigState h{};
     h.wArA = 1.0e37;  // GREAT, eigenDiagPCG.cpp:75
     EigState* es = eig.p + slot;
     UNAP_CK(cudaMemcpyAsync(es, &h, sizeof(EigState), cudaMemcpyHostToDevice, ex.s));
-    Rows<double> R = rows64(*K.L);
-    (void)n;
-    eig_diag_pcg(ex, R, K.rD.p, xk, bk, K.acf.p, K.w.p, K.p.p, es,
-                 pool.site(M_EIGWR, nullptr, FIN_RES_ONLY), pool.site(M_EIGA, nullptr, FIN_RES_ONLY),
-                 10);
+    EigLevel E{rows64(*K.L), K.rD.p, xk, K.acf.p, K.w.p, K.p.p, es,
+               pool.site(M_EIGWR, nullptr, FIN_RES_ONLY), pool.site(M_EIGA, nullptr, FIN_RES_ONLY)};
+    eig_diag_pcg(ex, &E, 1, &bk, 10);
     k_eig_sturm(ex, es, 10);
 }
 

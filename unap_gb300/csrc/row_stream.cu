@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kBlock)
     if constexpr (DOT) {
         __threadfence();
         __syncthreads();
-        reduce_partials<1>(nBlocks, a.red,
+        reduce_partials<1>(nBlocks, (int)gridDim.x, a.red,
                            [&](const double (&t)[1]) { apply_fin(a.red.st, a.red.fin, t, 1); });
     }
 }
