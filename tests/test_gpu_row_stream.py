@@ -55,3 +55,33 @@ def test_products_in_the_callers_order(cuda, orc, n, shift):
     A.spmv(buf[:n], buf[at:at + n])
     assert np.array_equal(buf[at:at + n].cpu().numpy(), orc.spmv(s, x))
     A.close()
+
+
+@pytest.mark.parametrize("exponent", [0, -126, -128])
+def test_fp32_cycles_near_the_smallest_numbers(cuda, exponent):
+    """FP32 results widened to FP64: normal and subnormal numbers, zeros,
+    infinities.  Scaling the right-hand side by a power of two scales the
+    result but for roundings to multiples of 2^-149: some 10^4 of them, of
+    1.4e-45 each, against results of 1e-39 and more."""
+    torch = cuda
+    s = random_system(4000, 9000, 5, symm=True, near=300)
+    A = capi.DeviceMatrix(s)
+    G = capi.DeviceAmg(A, precision=1, n_coarsest=100)
+    z = torch.empty(s.n, dtype=torch.float64, device="cuda")
+
+    def cycle(b):
+        G.vcycle(torch.tensor(b, device="cuda"), z)
+        return z.cpu().numpy().copy()
+
+    want = cycle(s.b) * 2.0 ** exponent
+    got = cycle(s.b * 2.0 ** exponent)
+    assert np.array_equal(got, got.astype(np.float32).astype(np.float64))
+    if exponent == 0:
+        assert np.array_equal(got, want)
+    assert np.abs(got - want).max() <= 1e4 * 2.0 ** -149 or exponent == 0
+    assert np.array_equal(cycle(0.0 * s.b), np.zeros(s.n))
+    b = s.b.copy()
+    b[7] = np.inf
+    assert not np.isfinite(cycle(b)).all()
+    G.close()
+    A.close()

@@ -735,15 +735,23 @@ void AmgHierarchy::appendVcycle(std::vector<Step>& out, std::vector<LevelRows>& 
     }
 }
 
+const float* AmgHierarchy::vcycleSingle(const Exec& ex, const double* r, Gate g)
+{
+    g_ext.r = r;
+    g_ext.z = nullptr;
+    curTail = tailFirst(sizeof(float));
+    // a Chebyshev finest level converts r inside its first step
+    if (!isCheby(0)) k_d2f(ex, lv[0].n, r, lv[0].bf.p);
+    return vcycle_level<float>(ex, 0, g);
+}
+
 void AmgHierarchy::vcycle(const Exec& ex, const double* r, double* z, Gate g)
 {
     g_ext.r = r;
     g_ext.z = z;
     curTail = tailFirst(params.precision == 1 ? sizeof(float) : sizeof(double));
     if (params.precision == 1) {
-        // a Chebyshev finest level converts r inside its first step
-        if (!isCheby(0)) k_d2f(ex, lv[0].n, r, lv[0].bf.p);
-        k_f2d(ex, lv[0].n, vcycle_level<float>(ex, 0, g), z);
+        k_f2d(ex, lv[0].n, vcycleSingle(ex, r, g), z);
     } else {
         vcycle_level<double>(ex, 0, g);
     }

@@ -74,6 +74,8 @@ public:
     std::vector<int> levelWavefronts() const;
     // z = M^-1 r, internal order of the finest level
     void vcycle(const Exec& ex, const double* r, double* z, Gate g);
+    // FP32 cycles (precision 1): the result in FP32, overwritten by the next
+    const float* vcycleSingle(const Exec& ex, const double* r, Gate g);
     // mean V-cycle time over `reps` runs on internal vectors (ms[0]), then
     // per level from one run with events around every level (ms[1 + k]:
     // level k's own steps; a level running in the cluster tail holds the
@@ -186,6 +188,10 @@ public:
                Gate g) override
     {
         H.vcycle(ex, r, w, g);
+    }
+    const float* applySingle(const Exec& ex, const double* r, Gate g) override
+    {
+        return H.params.precision == 1 ? H.vcycleSingle(ex, r, g) : nullptr;
     }
     void check() const override { H.check(); }
     bool appendSteps(std::vector<Step>& out, std::vector<LevelRows>& lv, const double* r,

@@ -411,14 +411,23 @@ void Krylov::enqueuePcgIteration()
 {
     Gate g{d_st, 1};
     Rows<double> Ar = rows64(*A.L);
+    bool direction = false;
     if (P->fusesDot() && !flexible) {
         P->apply(ex, r.p, z.p, &pool, S_WR, d_st, FIN_PCG_WR, g);
+    } else if (const float* zs = P->applySingle(ex, r.p, g)) {
+        // An FP32 result is converted where it is read: writing it out in
+        // FP64 and reading that twice took 176 us an iteration at 256^3, these
+        // two kernels take 134.
+        k_dot2<float>(ex, n, zs, r.p, flexible ? zs : nullptr, flexible ? q.p : nullptr,
+               pool.site(S_WR, d_st, FIN_PCG_WR), g, fusedOuter);
+        k_pcg_direction(ex, n, zs, p.p, d_st, g, fusedOuter);
+        direction = true;
     } else {
         P->apply(ex, r.p, z.p, nullptr, 0, d_st, FIN_NONE, g);
-        k_dot2(ex, n, z.p, r.p, flexible ? z.p : nullptr, flexible ? q.p : nullptr,
+        k_dot2<double>(ex, n, z.p, r.p, flexible ? z.p : nullptr, flexible ? q.p : nullptr,
                pool.site(S_WR, d_st, FIN_PCG_WR), g, fusedOuter);
     }
-    k_pcg_direction(ex, n, z.p, p.p, d_st, g, fusedOuter);
+    if (!direction) k_pcg_direction(ex, n, z.p, p.p, d_st, g, fusedOuter);
     k_spmv<double>(ex, Ar, p.p, q.p, p.p, pool.site(S_ALPHA, d_st, FIN_PCG_ALPHA), g, fusedOuter);
     k_pcg_update(ex, n, x.p, r.p, p.p, q.p, pool.site(S_RES, d_st, FIN_PCG_RES), g, fusedOuter);
 }
@@ -436,7 +445,7 @@ void Krylov::enqueueBicgIteration()
     P->apply(ex, s.p, z.p, nullptr, 0, d_st, FIN_NONE, g3);
     // t = A z; tAtA = t.t and omega numerator t.s
     k_spmv<double>(ex, Ar, z.p, t.p, nullptr, RSpec{}, g3);
-    k_dot2(ex, n, t.p, t.p, t.p, s.p, pool.site(S_BOMEGA, d_st, FIN_BICG_OMEGA), g3);
+    k_dot2<double>(ex, n, t.p, t.p, t.p, s.p, pool.site(S_BOMEGA, d_st, FIN_BICG_OMEGA), g3);
     k_bicg_update(ex, n, x.p, r.p, y.p, z.p, s.p, t.p, r0.p, pool.site(S_RES, d_st, FIN_BICG_RES),
                   g1);
 }

@@ -48,6 +48,14 @@ public:
     virtual bool fusesDot() const { return false; }
     virtual void apply(const Exec& ex, const double* r, double* w, const RedPool* pool, int site,
                        KState* st, int fin, Gate g) = 0;
+    // apply() with the result left in FP32, in a vector of the preconditioner's
+    // own that the next apply overwrites; null (and nothing done) where w is
+    // not formed in FP32
+    virtual const float* applySingle(const Exec& ex, const double* r, Gate g)
+    {
+        (void)ex, (void)r, (void)g;
+        return nullptr;
+    }
     // Step-program form of apply (mega.hpp): appends the steps computing
     // w = M^-1 r; level 0 of `lv` is the system matrix.  When the steps
     // also leave w.r in partial slot `slot`, *dotFused is set.  Returns false

@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(kBlock) residual_kernel(Rows<T> A, const T* __
         T a = row_apply<T, XL_NC, true, CK>(A, i, x);
         T ri = lds<true>(b + i) - a;
         r[i] = ri;
-        v[0] += (double)ri * (double)ri;
+        // FP64 instructions: not without need (FP32 rows have no others)
+        if (red.blockPart) v[0] += (double)ri * (double)ri;
     }
     if (red.blockPart) reduce_and_finalize<1>(v, red);
 }
@@ -277,27 +278,63 @@ __device__ __forceinline__ double mad(double a, double b, double c)
         return c + a * b;
 }
 
-template <bool FM>
-__global__ void __launch_bounds__(kBlock) pcg_direction_kernel(int n, const double* __restrict__ w,
+// (double)v.  A conversion is an FP64 instruction (on a pipe of 0.525 T/s, as
+// dear as a fused multiply-add), so integer instructions do it: the exponent is
+// rebased by 896, subnormal numbers shifted to their leading bit first.
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v)
+{
+    const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
+    const int s = m < 0x00800000u ? __clz((int)m) - 8 : 0;
+    const unsigned t = m << s;
+    unsigned hi = (t >> 3) + 0x38000000u - ((unsigned)s << 20);
+    if (m >= 0x7f800000u) hi += 0x38000000u;  // infinities and NaNs
+    if (m > 0x7f800000u) hi |= 0x00080000u;
+    if (m == 0u) hi = 0u;
+    return __hiloint2double((int)((u & 0x80000000u) | hi), (int)(t << 29));
+}
+
+// Rows a thread has in flight in the two kernels below: with one row at a time
+// a direction of FP32 rows took 75 us at 256^3, this 51 (its bytes: 50); the
+// two dot products are bound by the FP64 pipe (83 us, 64 at the measured rate).
+constexpr int kRowsAhead = 4;
+
+template <bool FM, class Z>
+__global__ void __launch_bounds__(kBlock) pcg_direction_kernel(int n, const Z* __restrict__ w,
                                                                double* __restrict__ p,
                                                                const KState* st, Gate g)
 {
     if (gate_closed(g)) return;
     const bool useBeta = st->useBeta;
     const double beta = st->beta;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        p[i] = useBeta ? mad<FM>(beta, p[i], w[i]) : w[i];
+    const int step = gridDim.x * blockDim.x;
+    for (long long i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kRowsAhead * step) {
+        Z wi[kRowsAhead];
+        double pi[kRowsAhead];
+#pragma unroll
+        for (int k = 0; k < kRowsAhead; ++k) {
+            const long long i = i0 + k * step;
+            wi[k] = i < n ? w[i] : Z(0);
+            pi[k] = useBeta && i < n ? p[i] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kRowsAhead; ++k) {
+            const long long i = i0 + k * step;
+            if (i < n) p[i] = useBeta ? mad<FM>(beta, pi[k], widen(wi[k])) : widen(wi[k]);
+        }
+    }
 }
 
-void k_pcg_direction(const Exec& ex, int n, const double* w, double* p, const KState* st, Gate g,
+template <class Z>
+void k_pcg_direction(const Exec& ex, int n, const Z* w, double* p, const KState* st, Gate g,
                      bool fused)
 {
     if (n <= 0) return;
     tick();
     if (fused)
-        pcg_direction_kernel<true><<<ex.grid(n), kBlock, 0, ex.s>>>(n, w, p, st, g);
+        pcg_direction_kernel<true, Z><<<ex.grid(n), kBlock, 0, ex.s>>>(n, w, p, st, g);
     else
-        pcg_direction_kernel<false><<<ex.grid(n), kBlock, 0, ex.s>>>(n, w, p, st, g);
+        pcg_direction_kernel<false, Z><<<ex.grid(n), kBlock, 0, ex.s>>>(n, w, p, st, g);
 }
 
 template <bool FM>
@@ -330,30 +367,48 @@ void k_pcg_update(const Exec& ex, int n, double* x, double* r, const double* p, 
         pcg_update_kernel<false><<<ex.grid(n), kBlock, 0, ex.s>>>(n, x, r, p, q, red, g);
 }
 
-template <bool FM>
-__global__ void __launch_bounds__(kBlock) dot2_kernel(int n, const double* __restrict__ a,
+template <bool FM, class Z>
+__global__ void __launch_bounds__(kBlock) dot2_kernel(int n, const Z* __restrict__ a,
                                                       const double* __restrict__ b,
-                                                      const double* __restrict__ c,
+                                                      const Z* __restrict__ c,
                                                       const double* __restrict__ d, RSpec red,
                                                       Gate g)
 {
     if (gate_closed(g)) return;
     double v[2] = {0.0, 0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        v[0] = mad<FM>(a[i], b[i], v[0]);
-        if (c) v[1] = mad<FM>(c[i], d[i], v[1]);
+    const int step = gridDim.x * blockDim.x;
+    for (long long i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kRowsAhead * step) {
+        Z ai[kRowsAhead], ci[kRowsAhead];
+        double bi[kRowsAhead], di[kRowsAhead];
+#pragma unroll
+        for (int k = 0; k < kRowsAhead; ++k) {
+            const long long i = i0 + k * step;
+            const bool on = i < n;
+            ai[k] = on ? a[i] : Z(0);
+            bi[k] = on ? b[i] : 0.0;
+            ci[k] = c == a ? ai[k] : on && c ? c[i] : Z(0);
+            di[k] = on && c ? d[i] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kRowsAhead; ++k) {
+            if (i0 + k * step >= n) break;
+            const double x = widen(ai[k]);
+            v[0] = mad<FM>(x, bi[k], v[0]);
+            if (c) v[1] = mad<FM>(c == a ? x : widen(ci[k]), di[k], v[1]);
+        }
     }
     reduce_and_finalize<2>(v, red);
 }
 
-void k_dot2(const Exec& ex, int n, const double* a, const double* b, const double* c,
-            const double* d, RSpec red, Gate g, bool fused)
+template <class Z>
+void k_dot2(const Exec& ex, int n, const Z* a, const double* b, const Z* c, const double* d,
+            RSpec red, Gate g, bool fused)
 {
     tick();
     if (fused)
-        dot2_kernel<true><<<ex.grid(n > 0 ? n : 1), kBlock, 0, ex.s>>>(n, a, b, c, d, red, g);
+        dot2_kernel<true, Z><<<ex.grid(n > 0 ? n : 1), kBlock, 0, ex.s>>>(n, a, b, c, d, red, g);
     else
-        dot2_kernel<false><<<ex.grid(n > 0 ? n : 1), kBlock, 0, ex.s>>>(n, a, b, c, d, red, g);
+        dot2_kernel<false, Z><<<ex.grid(n > 0 ? n : 1), kBlock, 0, ex.s>>>(n, a, b, c, d, red, g);
 }
 
 // --------------------------------------------------------------------------
@@ -654,7 +709,7 @@ __global__ void d2f_kernel(int n, const double* __restrict__ in, float* __restri
 __global__ void f2d_kernel(int n, const float* __restrict__ in, double* __restrict__ out)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = (double)in[i];
+        out[i] = widen(in[i]);
 }
 
 void k_d2f(const Exec& ex, int n, const double* in, float* out)
@@ -799,6 +854,10 @@ int device_max_blocks()
     template void k_spmv<T>(const Exec&, const Rows<T>&, const T*, T*, const T*, RSpec, Gate,      \
                             bool);                                                               \
     template void k_spmv_reference<T>(const Exec&, const Rows<T>&, const int*, const T*, T*, T*); \
+    template void k_pcg_direction<T>(const Exec&, int, const T*, double*, const KState*, Gate,     \
+                                     bool);                                                      \
+    template void k_dot2<T>(const Exec&, int, const T*, const double*, const T*, const double*,    \
+                            RSpec, Gate, bool);                                                  \
     template void k_residual<T>(const Exec&, const Rows<T>&, const T*, const T*, T*, RSpec, Gate); \
     template void k_gs_rows<T>(const Exec&, const Rows<T>&, T*, const T*, int, int, bool, Gate);   \
     template void gs_sweep<T>(const Exec&, const Level&, const Rows<T>&, T*, const T*, bool, bool, \

@@ -57,14 +57,17 @@ void diag_apply(const Exec& ex, int n, const double* rD, const double* r, double
 
 // PCG pieces (fused: fused multiply-adds, as for k_spmv).
 // p = useBeta ? w + beta p : w
-void k_pcg_direction(const Exec& ex, int n, const double* w, double* p, const KState* st, Gate g,
+// w in T: FP32 entries are converted as they are read
+template <class T>
+void k_pcg_direction(const Exec& ex, int n, const T* w, double* p, const KState* st, Gate g,
                      bool fused = false);
 // x += alpha p, r -= alpha q; sums r.r
 void k_pcg_update(const Exec& ex, int n, double* x, double* r, const double* p, const double* q,
                   RSpec red, Gate g, bool fused = false);
 // sums a.b (and c.d when c != nullptr)
-void k_dot2(const Exec& ex, int n, const double* a, const double* b, const double* c,
-            const double* d, RSpec red, Gate g, bool fused = false);
+template <class T>
+void k_dot2(const Exec& ex, int n, const T* a, const double* b, const T* c, const double* d,
+            RSpec red, Gate g, bool fused = false);
 
 // PBiCGStab pieces (PBiCGStab.cpp:155-456)
 void k_bicg_init(const Exec& ex, int n, const double* b, const double* Ax, double* r, double* r0,
