@@ -598,9 +598,9 @@ int unap_cuda_gauss_seidel(long int handle, double* x, const double* b, int nSwe
         // up to four sweeps a launch, each following the one before
         const int per = std::min(nSweeps, 4);
         if (h->sweeps.sweeps < per) h->sweeps.init((size_t)A.n(), sizeof(double), per);
-        const double* y = flow_gs<double>(ex, *A.L, R, h->sweeps, h->s1.p, h->s2.p, nSweeps,
-                                          backward != 0, false, nullptr, nullptr, Gate{});
-        k_to_reference<double>(ex, A.n(), A.L->d_perm.p, y, x);
+        // x and b are copied, so the last sweep may write x
+        flow_gs<double>(ex, *A.L, R, h->sweeps, h->s1.p, h->s2.p, nSweeps, backward != 0, false,
+                        nullptr, x, Gate{}, A.L->d_perm.p);
         UNAP_CK(cudaGetLastError());
         UNAP_CK(cudaStreamSynchronize(A.stream));
         h->sweeps.check();

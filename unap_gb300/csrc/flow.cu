@@ -59,7 +59,8 @@ struct GsArgs {
     T* out;         // sweep s writes out + s * stride ...
     long long stride;
     T* last;        // ... and the last one here
-    T* copy;        // and here, or null
+    T* copy;        // and here, or null,
+    const int* copyAt;  // row r at copyAt[r] if given
     const T* b;
     unsigned* counter;
     int* err;
@@ -182,7 +183,8 @@ __global__ void __launch_bounds__(kFlowThreads)
         if (on && g == 0) {
             acc = acc / d;
             st_flow(out + r, acc);
-            if (a.copy && s == a.nSweeps - 1) a.copy[r] = acc;  // as above
+            if (a.copy && s == a.nSweeps - 1)
+                a.copy[a.copyAt ? ldg(a.copyAt + r) : r] = acc;
         }
     }
 }
@@ -512,7 +514,8 @@ static void launch_gs(const Exec& ex, int wide, int lanes, const GsArgs<T>& a, G
 
 template <class T>
 T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& ring, const T* in,
-           const T* b, int nSweeps, bool backward, bool xIsZero, T* last, T* copy, Gate g)
+           const T* b, int nSweeps, bool backward, bool xIsZero, T* last, T* copy, Gate g,
+           const int* copyAt)
 {
     const int lanes = L.n ? sweep_lanes(L.n, 2.0 * L.nf / L.n, sizeof(T) == 8) : 1;
     const SweepTasks& S = L.tasks[lanes == 8 ? 2 : lanes == 4 ? 1 : 0];
@@ -534,6 +537,7 @@ T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& rin
         a.stride = (long long)(ring.stride / sizeof(T));
         a.last = end && last ? last : reinterpret_cast<T*>(ring.vec(h, m - 1));
         a.copy = end ? copy : nullptr;
+        a.copyAt = copyAt;
         a.b = b;
         a.counter = ring.counter(h);
         a.err = ring.err;
@@ -554,10 +558,10 @@ T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& rin
 
 template float* flow_gs<float>(const Exec&, const Level&, const Rows<float>&, const FlowRing&,
                                const float*, const float*, int, bool, bool, float*, float*,
-                               Gate);
+                               Gate, const int*);
 template double* flow_gs<double>(const Exec&, const Level&, const Rows<double>&, const FlowRing&,
                                  const double*, const double*, int, bool, bool, double*, double*,
-                                 Gate);
+                                 Gate, const int*);
 
 void DicFlow::init(const Level& L)
 {
