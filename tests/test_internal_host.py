@@ -1,0 +1,29 @@
+"""Host-side pieces of the library's internals, compiled alone and run without a GPU."""
+import os
+import subprocess
+
+import pytest
+
+from cxx_util import CXX_DIR, ROOT, compiler
+
+pytestmark = pytest.mark.skipif(compiler() is None, reason="no C++ compiler")
+
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+
+def run_program(name, tmp_path):
+    """Compiles tests/cxx/<name>.cpp against the internal headers (no CUDA
+    runtime linked) and returns its output."""
+    out = str(tmp_path / name)
+    cmd = [compiler(), "-std=c++17", "-O1", "-Wall", "-I",
+           os.path.join(ROOT, "unap_gb300", "csrc"), "-I", CUDA_INCLUDE,
+           os.path.join(CXX_DIR, f"{name}.cpp"), "-o", out, "-pthread"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([out], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
+def test_row_counts_of_long_rows(tmp_path):
+    assert "ok" in run_program("row_info", tmp_path)

@@ -104,7 +104,7 @@ __device__ __forceinline__ void row_task(const Args<T>& a, const Stage<T>& S, in
     int len = 0;
     T d = T(1);
     if (on) {
-        len = ldg(S.A.rowInfo + r) & 0xffff;
+        len = row_len(ldg(S.A.rowInfo + r));
         d = ldg(S.A.diag + r);
     }
     int c[K];

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kBlock, (CK == 8 && sizeof(T) == 4) ? 6 : 1)
     int c[CK];
     T v[CK];
     if (r < A.n) {
-        len = lds<true>(A.rowInfo + r) & 0xffff;
+        len = row_len(lds<true>(A.rowInfo + r));
         base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
         d = lds<true>(A.diag + r);
 #pragma unroll

@@ -172,7 +172,7 @@ __device__ __forceinline__ T row_apply(const Rows<T>& A, int r, const T* x,
 {
     auto at = [&](int c) { return MAP ? ldg(map + c) : c; };
     const int info = lds<ST>(A.rowInfo + r);
-    const int len = info & 0xffff;
+    const int len = row_len(info);
     const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
     T acc = T(0);
     if constexpr (FM)

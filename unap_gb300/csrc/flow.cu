@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(kFlowThreads)
             c[k] = has ? ldg(a.A.col + base + 32 * (k * G + g)) : 0;
             v[k] = has ? ldg(a.A.val + base + 32 * (k * G + g)) : T(0);
         }
-        const int nLow = info >> 16;
-        const int jEnd = !BWD && s == 0 && a.firstFromZero ? nLow : info & 0xffff;
+        const int nLow = row_low(info);
+        const int jEnd = !BWD && s == 0 && a.firstFromZero ? nLow : row_len(info);
         if ((BWD ? nr.y : nr.x) >= 0) wait_near(out + (BWD ? nr.y : nr.x), a.err);
         for (int j0 = 0;;) {
             unsigned need = 0;
@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(kFlowThreads)
         double acc = 1.0;
         if (on) {
             const int info = ldg(A.rowInfo + r);
-            len = info & 0xffff;
-            nLow = info >> 16;
+            len = row_len(info);
+            nLow = row_low(info);
             acc = ldg(A.diag + r);
         }
         const int most = __reduce_max_sync(0xffffffffu, nLow);
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_dic_kernel(const __grid_con
         double acc = 0.0, rr = 0.0;
         if (on) {
             const int info = ldg(A.rowInfo + r);
-            const int len = info & 0xffff, nLow = info >> 16;
+            const int len = row_len(info), nLow = row_low(info);
             const int base = D.z + lane;
             cnt = bwd ? len - nLow : nLow;
             first = bwd ? base + 32 * (len - 1) : base;

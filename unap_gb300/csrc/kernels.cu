@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kBlock) gs_kernel(Rows<T> A, T* x, const T* __
         info = lds<true>(A.rowInfo + r);
         base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
         d = lds<true>(A.diag + r);
-        const int len = info & 0xffff;
+        const int len = row_len(info);
 #pragma unroll
         for (int k = 0; k < CK; ++k) {
             const int e = base + 32 * k;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kBlock) gs_kernel(Rows<T> A, T* x, const T* __
     if (gate_closed(g)) return;
     if (r < r1) {
         bb = __ldcg(b + r);
-        const int jEnd = skipUpper ? (info >> 16) : (info & 0xffff);
+        const int jEnd = skipUpper ? row_low(info) : row_len(info);
         T xv[CK];
 #pragma unroll
         for (int k = 0; k < CK; ++k) xv[k] = k < jEnd ? x[c[k]] : T(0);
@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(kBlock) gs_kernel(Rows<T> A, T* x, const T* __
     }
     for (r += gridDim.x * blockDim.x; r < r1; r += gridDim.x * blockDim.x) {
         const int info2 = lds<true>(A.rowInfo + r);
-        const int len = info2 & 0xffff;
-        const int nLow = info2 >> 16;
+        const int len = row_len(info2);
+        const int nLow = row_low(info2);
         const int base2 = ldg(A.sliceOff + (r >> 5)) + (r & 31);
         T acc = lds<true>(b + r);
         acc = row_subtract<T, true, CK>(A, A.val, base2, 0, nLow, x, acc);

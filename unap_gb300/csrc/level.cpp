@@ -236,7 +236,7 @@ std::unique_ptr<Level> build_level(const HostLdu& A, const std::vector<int>* key
             }
             ++j;
         }
-        rowInfo[(size_t)i] = rowLen[(size_t)i] | (rowLow[(size_t)i] << 16);
+        rowInfo[(size_t)i] = row_info(rowLen[(size_t)i], rowLow[(size_t)i]);
     }
     // padding entries point at the row itself with zero value
     for (int sl = 0; sl < L->nSlices; ++sl) {

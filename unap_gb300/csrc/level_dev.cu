@@ -602,7 +602,7 @@ __global__ void k_rows(const int* __restrict__ perm, int n, const int* __restric
         const int len = lo + ownStart[c + 1] - ownStart[c];
         if (len > 0xffff) atomicOr(tooLong, 1);
         rowLen[i] = len;
-        rowInfo[i] = len | (lo << 16);
+        rowInfo[i] = row_info(len, lo);
     }
 }
 

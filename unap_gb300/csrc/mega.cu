@@ -97,8 +97,8 @@ __device__ void exec_gs(const Step& s, const LevelRows& L, int first, int stride
     const T* b = (const T*)s.b;
     for (int r = s.r0 + first; r < s.r1; r += stride) {
         const int info = ldg(A.rowInfo + r);
-        const int len = info & 0xffff;
-        const int nLow = info >> 16;
+        const int len = row_len(info);
+        const int nLow = row_low(info);
         const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
         T acc = b[r];
         acc = row_subtract<T>(A, A.val, base, 0, nLow, x, acc);
@@ -159,7 +159,7 @@ __device__ void exec_dic_fwd(const Step& s, const LevelRows& L, int first, int s
     const double* rD = (const double*)s.e;
     const double* coef = (const double*)s.d;
     for (int r = s.r0 + first; r < s.r1; r += stride) {
-        const int nLow = ldg(A.rowInfo + r) >> 16;
+        const int nLow = row_low(ldg(A.rowInfo + r));
         const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
         const double rd = ldg(rD + r);
         double acc = rd * rr[r];
@@ -181,8 +181,8 @@ __device__ void exec_dic_bwd(const Step& s, const LevelRows& L, const MegaArgs& 
     double v[1] = {0.0};
     for (int r = s.r0 + first; r < s.r1; r += stride) {
         const int info = ldg(A.rowInfo + r);
-        const int len = info & 0xffff;
-        const int nLow = info >> 16;
+        const int len = row_len(info);
+        const int nLow = row_low(info);
         const int base = ldg(A.sliceOff + (r >> 5)) + (r & 31);
         const double rd = ldg(rD + r);
         double acc = w[r];

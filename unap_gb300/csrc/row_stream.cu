@@ -69,7 +69,7 @@ __device__ __forceinline__ void load_slice(const Rows<T>& A, int r, int off, int
     h.len = 0;
     h.d = T(0);
     if (r < A.n) {
-        h.len = lds<true>(A.rowInfo + r) & 0xffff;
+        h.len = row_len(lds<true>(A.rowInfo + r));
         h.d = lds<true>(A.diag + r);
     }
 #pragma unroll

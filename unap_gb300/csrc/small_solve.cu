@@ -146,7 +146,7 @@ __device__ __forceinline__ void sweep_pre(const SmallSystem& S, const double* sr
     if (i < 0) return;
     const Rows<double>& A = S.A;
     const int info = A.rowInfo[i];
-    const int len = info & 0xffff, nLow = info >> 16;
+    const int len = row_len(info), nLow = row_low(info);
     P.base = A.sliceOff[i >> 5] + (i & 31);
     P.a0 = FWD ? S.rD[i] * src[i] : src[i];
     P.lo = FWD ? 0 : nLow;
@@ -242,7 +242,7 @@ __device__ __noinline__ void cluster_sweeps(const SmallSystem& S, const double* 
         double acc = 0.0;
         if (on) {
             const int info = ldg(A.rowInfo + i);
-            const int len = info & 0xffff, nLow = info >> 16;
+            const int len = row_len(info), nLow = row_low(info);
             cnt = bwd ? len - nLow : nLow;
             first = D.z + lane + (bwd ? 32 * (len - 1) : 0);
             if (!bwd) acc = ldg(S.rD + i) * __ldcg(r + i);

@@ -191,7 +191,7 @@ __device__ __forceinline__ void fetch_row(const TailLevel& L, Row<T, KW>& q)
 {
     if (q.r < 0) return;
     constexpr int EPR = Pk<T>::EPR;
-    const int len = q.info & 0xffff;
+    const int len = row_len(q.info);
     q.b = __ldcg((const T*)L.b + q.r);
     q.d = ldg((const T*)L.diag + q.r);
     const int4* rec = L.prec + q.start;
@@ -208,7 +208,7 @@ __device__ __forceinline__ void gs_row(const TailLevel& L, const Ctx& c, unsigne
 {
     constexpr int EPR = Pk<T>::EPR;
     constexpr int AT = DIST ? XA_DIST : XA_LOCAL;
-    const int jEnd = skipUpper ? (q.info >> 16) : (q.info & 0xffff);
+    const int jEnd = skipUpper ? row_low(q.info) : row_len(q.info);
     T acc = q.b;
 #pragma unroll
     for (int k = 0; k < Row<T, KW>::R; ++k) {
@@ -303,7 +303,7 @@ __device__ __noinline__ void tail_residual(const TailLevel& L, Ctx c)
     const unsigned xOffB = (unsigned)(L.xOff * (int)sizeof(T));
     for_units<DIST>(c, L.n, [&](int i) {
         const int2 m = ldg(L.pmeta + i);
-        const int len = m.y & 0xffff;
+        const int len = row_len(m.y);
         const T bi = __ldcg((const T*)L.b + i);
         T acc = T(0);
         acc += ldg((const T*)L.diag + i) * xget<T, AT>(c, dyn, xOffB, i);
@@ -609,7 +609,7 @@ __global__ void pack_rows_kernel(Rows<T> A, const int* __restrict__ start, int2*
     constexpr int EPR = Pk<T>::EPR;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < A.n; r += gridDim.x * blockDim.x) {
         const int info = A.rowInfo[r];
-        const int len = info & 0xffff;
+        const int len = row_len(info);
         const int base = A.sliceOff[r >> 5] + (r & 31);
         const int s = start[r];
         meta[r] = make_int2(s, info);
@@ -647,7 +647,7 @@ void pack_rows(const Rows<T>& A, PackedRows& out, cudaStream_t s)
     long long total = 0;
     for (int r = 0; r < n; ++r) {
         start[(size_t)r] = (int)total;
-        total += ((info[(size_t)r] & 0xffff) + EPR - 1) / EPR;
+        total += (row_len(info[(size_t)r]) + EPR - 1) / EPR;
         if (total > 0x7fffffffLL) throw std::invalid_argument("level too large to pack");
     }
     DevArray<int> dStart;
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(kBlock) gs_packed_kernel(const int2* __restric
         start = m.x;
         info = m.y;
         d = ldg(diag + r);
-        const int len = info & 0xffff;
+        const int len = row_len(info);
 #pragma unroll
         for (int k = 0; k < R; ++k)
             if (k * EPR < len) q[k] = ldg(rec + start + k);
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kBlock) gs_packed_kernel(const int2* __restric
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (gate_closed(g) || r >= r1) return;
     bb = __ldcg(b + r);
-    const int jEnd = skipUpper ? (info >> 16) : (info & 0xffff);
+    const int jEnd = skipUpper ? row_low(info) : row_len(info);
     T xv[KW];
 #pragma unroll
     for (int k = 0; k < R; ++k) {

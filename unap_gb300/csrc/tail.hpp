@@ -59,7 +59,7 @@ struct TailLevel {
 // so a thread loads its whole row with a few vector loads.  FP32: two
 // entries per record {col, value bits, col, value bits}; FP64: one entry per
 // record {col, 0, value low word, value high word}.  meta[r] = {first record
-// of row r, row info (len | nLow << 16)}.
+// of row r, row_info}.
 struct PackedRows {
     DevArray<int2> meta;
     DevArray<int4> rec;

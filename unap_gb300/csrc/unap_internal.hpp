@@ -259,6 +259,15 @@ struct HostLdu {
     void validate();
 };
 
+// A row's entry counts in one word: all entries in the low 16 bits, those of
+// the lower side in the high 16, both unsigned (rows of up to 65,535 faces).
+__host__ __device__ inline int row_info(int len, int low)
+{
+    return (int)((unsigned)low << 16 | (unsigned)len);
+}
+__host__ __device__ inline int row_len(int info) { return info & 0xffff; }
+__host__ __device__ inline int row_low(int info) { return (int)((unsigned)info >> 16); }
+
 // Rows of a sweep in tasks of one warp: task t is task[t].y rows from
 // task[t].x on, of one SELL slice and one wavefront; their entry 0 starts at
 // task[t].z and they hold up to task[t].w entries.  near[t] names a row two
