@@ -6,6 +6,8 @@ is bit-identical to the oracle (same entry order and roundings, so the
 tolerance is zero); Krylov solutions, whose dot products are summed in another
 order, agree to 1e-10.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -95,3 +97,30 @@ def test_vcycle_sweeps(cuda, orc, precision, packed):
     finally:
         capi.set_device_setup(old_setup)
         capi.set_packed_sweeps(old_packed)
+
+
+@pytest.mark.parametrize("leaves", [2047, 2048, 2049, 40_000])
+def test_hierarchy_with_a_large_aggregate(cuda, orc, leaves):
+    """All cells around the hub join its aggregate.  Up to the longest list the
+    setup kernels sort (2,048) and beyond it, the transfers are the host's and
+    the setup takes no longer than for any system of the size."""
+    torch = cuda
+    s = hub_system(leaves, 0, True, 6)
+    r = np.random.default_rng(7).standard_normal(s.n)
+    old = capi.set_device_setup(1000)
+    try:
+        A = capi.DeviceMatrix(s)
+        t0 = time.perf_counter()
+        G = capi.DeviceAmg(A, n_coarsest=10, precision=0)
+        seconds = time.perf_counter() - t0
+    finally:
+        capi.set_device_setup(old)
+    O = OracleAmg(orc, s, n_coarsest=10, precision=0)
+    assert G.info()["cells"] == O.level_sizes()
+    z = torch.zeros(s.n, dtype=torch.float64, device="cuda")
+    G.vcycle(torch.tensor(r, device="cuda"), z)
+    assert np.array_equal(z.cpu().numpy(), O.vcycle(r))
+    assert seconds < 5.0
+    G.close()
+    O.close()
+    A.close()

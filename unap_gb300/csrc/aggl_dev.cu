@@ -389,8 +389,11 @@ __global__ void k_child_fill(const int* __restrict__ agg, const int* __restrict_
     GRID_LOOP(c, n) list[atomicAdd(&cur[iperm[agg[c]]], 1)] = (int)c;
 }
 
-// every list in ascending cell order, then as internal rows of the finer
-// level (an aggregate has two or three cells; any length is sorted)
+// Every list in ascending cell order, then as internal rows of the finer
+// level.  An aggregate has two or three cells as a rule, but cells without a
+// free neighbour join the cluster across their heaviest face, so a hub's can
+// hold all cells around it: lists above kMaxList, which this insertion would
+// sort in quadratic time on one thread, are left to the host.
 __global__ void k_child_sort(const int* __restrict__ start, int nc, const int* __restrict__ fineIperm,
                              int* list)
 {
@@ -415,16 +418,17 @@ __global__ void k_coarse_of_row(const int* __restrict__ agg, const int* __restri
 
 }  // namespace
 
-void transfer_maps(const Level& F, const Level& C, const std::vector<int>& agg,
+void transfer_maps(const Level& F, const Level& C, const CoarseHost& c,
                    DevArray<int>& childStart, DevArray<int>& child, DevArray<int>& cmap,
                    cudaStream_t s)
 {
     const int n = F.n, nc = C.n;
+    const std::vector<int>& agg = c.restrictAddr;
     const long long minCells = device_setup_min_cells();
-    if (minCells < 0 || n < minCells) {
+    if (minCells < 0 || n < minCells || c.largest > kMaxList) {
         std::vector<int> refStart((size_t)nc + 1, 0);
         for (int i = 0; i < n; ++i) refStart[(size_t)agg[(size_t)i] + 1]++;
-        for (int c = 0; c < nc; ++c) refStart[(size_t)c + 1] += refStart[(size_t)c];
+        for (int k = 0; k < nc; ++k) refStart[(size_t)k + 1] += refStart[(size_t)k];
         std::vector<int> refChild((size_t)n);
         {
             std::vector<int> pos(refStart.begin(), refStart.end() - 1);
@@ -432,12 +436,12 @@ void transfer_maps(const Level& F, const Level& C, const std::vector<int>& agg,
         }
         std::vector<int> cs((size_t)nc + 1, 0), ch((size_t)n), cm((size_t)n);
         for (int r = 0; r < nc; ++r) {
-            const int c = C.perm[(size_t)r];
-            const int len = refStart[(size_t)c + 1] - refStart[(size_t)c];
+            const int k = C.perm[(size_t)r];
+            const int len = refStart[(size_t)k + 1] - refStart[(size_t)k];
             cs[(size_t)r + 1] = cs[(size_t)r] + len;
             for (int j = 0; j < len; ++j)
                 ch[(size_t)(cs[(size_t)r] + j)] =
-                    F.iperm[(size_t)refChild[(size_t)(refStart[(size_t)c] + j)]];
+                    F.iperm[(size_t)refChild[(size_t)(refStart[(size_t)k] + j)]];
         }
         for (int i = 0; i < n; ++i)
             cm[(size_t)i] = C.iperm[(size_t)agg[(size_t)F.perm[(size_t)i]]];
@@ -609,6 +613,7 @@ bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, Co
     // by construction: owner below neighbour, faces grouped by owner
     C.oriented = true;
     C.ownerSorted = true;
+    out.largest = kMaxList;  // longer lists of cells were left to the host above
     return true;
 }
 

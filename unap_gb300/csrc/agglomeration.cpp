@@ -172,6 +172,8 @@ void coarse_addressing(const HostLdu& fine, const std::vector<int>& map, int nCo
         }
     });
     out.restrictAddr = map;
+    std::vector<int> cells((size_t)nCoarse, 0);
+    for (int c : map) out.largest = std::max(out.largest, ++cells[(size_t)c]);
 }
 
 void coarse_coefficients(const HostLdu& fine, CoarseHost& c)

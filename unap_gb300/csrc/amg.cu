@@ -79,7 +79,7 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
         lv[(size_t)k].own = build_level(c.A, &key, k == L, s, !isCheby(k));
         lv[(size_t)k].L = lv[(size_t)k].own.get();
         lv[(size_t)k].n = nC;
-        transfer_maps(F, *lv[(size_t)k].L, c.restrictAddr, lv[(size_t)k].childStart,
+        transfer_maps(F, *lv[(size_t)k].L, c, lv[(size_t)k].childStart,
                       lv[(size_t)k].child, lv[(size_t)k].cmap, s);
     }
     UNAP_CK(cudaStreamSynchronize(s));

@@ -16,6 +16,7 @@ struct CoarseHost {
     HostLdu A;
     std::vector<int> restrictAddr;  // finer cells -> this level's cells
     std::vector<int> faceRestrict;  // finer faces -> coarse face, or -(cell+1)
+    int largest = 0;                // cells of the largest aggregate, or a bound on it
 };
 
 std::vector<int> pairwise_pass(const HostLdu& A, const std::vector<double>& w, int& nCoarse);
@@ -32,13 +33,13 @@ std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, std::vector<doub
 bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, CoarseHost& out,
                               std::vector<double>& cw, int& nCoarse, cudaStream_t s);
 std::vector<double> mg_face_weights(const HostLdu& A);
-// Transfers between a level and the one its cells aggregate into (agg: cell
-// -> coarse cell, reference numbering), in internal rows: the children of
-// coarse row r are child[childStart[r] ..], ascending finer cell (the
-// summation order of restrictField), and cmap[i] is the coarse row of finer
-// row i.  Made by kernels on levels of at least device_setup_min_cells()
-// cells; agg has to live until the stream is synchronized.
-void transfer_maps(const Level& F, const Level& C, const std::vector<int>& agg,
+// Transfers between a level and the one its cells aggregate into (c: that
+// level), in internal rows: the children of coarse row r are
+// child[childStart[r] ..], ascending finer cell (the summation order of
+// restrictField), and cmap[i] is the coarse row of finer row i.  Made by
+// kernels on levels of at least device_setup_min_cells() cells without a
+// large aggregate (c.largest); c has to live until the stream is synchronized.
+void transfer_maps(const Level& F, const Level& C, const CoarseHost& c,
                    DevArray<int>& childStart, DevArray<int>& child, DevArray<int>& cmap,
                    cudaStream_t s);
 

@@ -144,7 +144,7 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
         lv[(size_t)k].n = c.A.n;
         const int nc = c.A.n;
         Lv& K = lv[(size_t)k];
-        transfer_maps(F, *K.L, c.restrictAddr, K.childStart, K.child, K.cmap, s);
+        transfer_maps(F, *K.L, c, K.childStart, K.child, K.cmap, s);
         K.corr.alloc((size_t)nc);
         K.src.alloc((size_t)nc);
         UNAP_CK(cudaStreamSynchronize(s));
