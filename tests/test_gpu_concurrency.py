@@ -110,3 +110,27 @@ def test_concurrent_krylov_solves_match_alone(cuda):
             assert st["nIterations"] == alone[i]["nIterations"], (i, st, alone[i])
     for A in mats:
         A.close()
+
+
+def test_workspaces_from_several_threads(cuda, orc):
+    """Calls whose workspaces come from the shared pool, from threads that
+    also create and destroy their matrices (the last one out empties the
+    pool): the bits of the same calls alone."""
+    torch = cuda
+    N = 6
+    systems = [W.laplace(20 + i, 18, 16, seed=400 + i, permute=True) for i in range(N)]
+    rs = [np.random.default_rng(i).standard_normal(s.n) for i, s in enumerate(systems)]
+    want = [[orc.precond(t, s, r)[0] for t in (2, 3)] for s, r in zip(systems, rs)]
+
+    def work(i):
+        s = systems[i]
+        r = torch.tensor(rs[i], device="cuda")
+        w = torch.zeros_like(r)
+        for _ in range(8):
+            A = capi.DeviceMatrix(s)
+            for t in (2, 3):
+                A.precondition(t, r, w)
+                assert np.array_equal(w.cpu().numpy(), want[i][t - 2]), (i, t)
+            A.close()
+
+    _run_threads(work, N)

@@ -27,3 +27,7 @@ def run_program(name, tmp_path):
 
 def test_row_counts_of_long_rows(tmp_path):
     assert "ok" in run_program("row_info", tmp_path)
+
+
+def test_failed_allocation_gives_the_workspace_pool_back(tmp_path):
+    assert "ok" in run_program("alloc_retry", tmp_path)

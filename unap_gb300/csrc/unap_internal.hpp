@@ -74,16 +74,30 @@ struct CaptureGate {
 };
 // what the workspace pool holds goes back to the driver (the current device)
 void trim_workspace_pool();
-inline cudaError_t gated_malloc(void** p, size_t bytes)
+// get(), and once more without the workspace pool's unused blocks if the
+// device is out of memory
+template <class F>
+cudaError_t malloc_or_trim(F&& get)
 {
-    AllocGate g;
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = get();
     if (e == cudaErrorMemoryAllocation) {
         (void)cudaGetLastError();
         trim_workspace_pool();
-        e = cudaMalloc(p, bytes);
+        e = get();
     }
     return e;
+}
+inline cudaError_t gated_malloc(void** p, size_t bytes)
+{
+    AllocGate g;
+    return malloc_or_trim([&] { return cudaMalloc(p, bytes); });
+}
+// stream-ordered; pool null: the device's default pool
+inline cudaError_t pool_malloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t s)
+{
+    return malloc_or_trim([&] {
+        return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+    });
 }
 inline cudaError_t gated_free(void* p)
 {
@@ -189,11 +203,7 @@ struct DevArray {
         if (s) {
             if (thread_in_capture())
                 throw std::logic_error("device allocation inside a stream capture");
-            if (thread_alloc_pool())
-                UNAP_CK(cudaMallocFromPoolAsync((void**)&p, count * sizeof(T),
-                                                thread_alloc_pool(), s));
-            else
-                UNAP_CK(cudaMallocAsync((void**)&p, count * sizeof(T), s));
+            UNAP_CK(pool_malloc((void**)&p, count * sizeof(T), thread_alloc_pool(), s));
             as = s;
             async = true;
         } else {
@@ -237,7 +247,7 @@ struct StreamScratch {
     cudaStream_t s = 0;
     StreamScratch(size_t count, cudaStream_t st) : s(st)
     {
-        if (count) UNAP_CK(cudaMallocAsync((void**)&p, count * sizeof(T), s));
+        if (count) UNAP_CK(pool_malloc((void**)&p, count * sizeof(T), nullptr, s));
     }
     StreamScratch(const StreamScratch&) = delete;
     StreamScratch& operator=(const StreamScratch&) = delete;
