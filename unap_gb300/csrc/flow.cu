@@ -417,48 +417,6 @@ int flow_grid(long long tasks)
 
 }  // namespace
 
-FlowRing::FlowRing(FlowRing&& o) noexcept
-    : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), err(o.err)
-{
-    o.err = nullptr;
-}
-
-FlowRing& FlowRing::operator=(FlowRing&& o) noexcept
-{
-    mem = std::move(o.mem);
-    stride = o.stride;
-    half = o.half;
-    sweeps = o.sweeps;
-    std::swap(err, o.err);
-    return *this;
-}
-
-FlowRing::~FlowRing() { pinned_block_free(err); }
-
-void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves)
-{
-    sweeps = std::max(1, std::min(sweepsPerHalf, kFlowMaxSweeps));
-    stride = (n * elemBytes + 255) / 256 * 256;
-    half = kFlowHeader + stride * (size_t)sweeps;
-    mem.alloc((size_t)halves * half);
-    if (!err) err = static_cast<int*>(pinned_block_alloc(64));
-    *err = 0;
-}
-
-int FlowRing::other(const void* p) const
-{
-    const unsigned char* q = static_cast<const unsigned char*>(p);
-    return q >= mem.p && q < mem.p + half ? 1 : 0;
-}
-
-void FlowRing::check() const
-{
-    if (err && *(volatile int*)err) {
-        *(volatile int*)err = 0;
-        throw CudaError("wavefront sweep: a wait for a neighbouring row ran out");
-    }
-}
-
 void flow_tasks(Level& L, cudaStream_t s)
 {
     if (!L.sweepable) return;

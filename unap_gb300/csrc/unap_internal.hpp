@@ -197,7 +197,6 @@ struct DevArray {
     void alloc(size_t count)
     {
         release();
-        n = count;
         if (!count) return;
         cudaStream_t s = thread_alloc_stream();
         if (s) {
@@ -209,6 +208,7 @@ struct DevArray {
         } else {
             UNAP_CK(gated_malloc((void**)&p, count * sizeof(T)));
         }
+        n = count;  // not before: a size without memory would pass for an array
     }
     void release()
     {
