@@ -134,3 +134,36 @@ def test_workspaces_from_several_threads(cuda, orc):
             A.close()
 
     _run_threads(work, N)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_sweep_form_switched_by_another_thread(cuda, precision):
+    """The setting of the V-cycle's sweep form changes while cycles are
+    enqueued: every cycle has the bits that all forms share."""
+    torch = cuda
+    s = W.laplace(22, 21, 20, seed=5, permute=True)
+    A = capi.DeviceMatrix(s)
+    G = capi.DeviceAmg(A, n_coarsest=60, precision=precision)
+    r = torch.tensor(np.random.default_rng(6).standard_normal(s.n), device="cuda")
+    z = torch.zeros_like(r)
+    G.vcycle(r, z)
+    want = z.cpu().numpy().copy()
+    stop = threading.Event()
+
+    def toggle():
+        while not stop.is_set():
+            capi.set_packed_sweeps(0)
+            capi.set_packed_sweeps(1)
+
+    th = threading.Thread(target=toggle)
+    th.start()
+    try:
+        for _ in range(300):
+            G.vcycle(r, z)
+            assert np.array_equal(z.cpu().numpy(), want)
+    finally:
+        stop.set()
+        th.join()
+        capi.set_packed_sweeps(1)
+    G.close()
+    A.close()

@@ -485,6 +485,9 @@ const T* AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
     const bool cheb = isCheby(k);
     const Lv& V = lv[(size_t)k];
     const int deg = params.chebyDegree;
+    // one form for the level's whole cycle: the setting it follows may change
+    // meanwhile (another thread), and each form keeps the iterate elsewhere
+    const bool flow = flows(k);
     T* cur = x;  // the level's iterate: the sweeps leave it in one of their vectors
     if (cheb) {
         // pre-smoothing from x = 0 (w shares the residual's buffer); the
@@ -498,7 +501,7 @@ const T* AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
         for (int j = 1; j < deg; ++j)
             k_cheb_step<T>(ex, Rk, chebBuf<T>(k, j - 1), chebBuf<T>(k, j), b, r, (T)V.d1[j],
                            (T)V.d2[j], 0, g);
-    } else if (params.nPre > 0 && !flows(k)) {
+    } else if (params.nPre > 0 && !flow) {
         for (int s = 0; s < params.nPre; ++s) sweep<T>(ex, k, Lk, Rk, x, b, false, s == 0, g);
     } else if (params.nPre > 0) {
         cur = flow_gs<T>(ex, Lk, Rk, V.sweeps, nullptr, b, params.nPre, false, true, nullptr,
@@ -531,7 +534,7 @@ const T* AmgHierarchy::vcycle_level(const Exec& ex, int k, Gate g)
                            j == 0 ? T(0) : (T)V.d2[j], j == 0 ? 1 : 0, g);
             prev = out;
         }
-    } else if (!flows(k)) {
+    } else if (!flow) {
         k_prolong_add<T>(ex, Lk.n, C.cmap.p, e, x, g);
         for (int s = 0; s < params.nPost; ++s) sweep<T>(ex, k, Lk, Rk, x, b, true, false, g);
     } else if (params.nPost > 0) {
@@ -772,13 +775,14 @@ static double time_smoother(AmgHierarchy& H, cudaStream_t s, int k, int reps, do
     k_fill<T>(ex, V.n, b.p, T(1));
     k_fill<T>(ex, V.n, w.p, T(0));
     const bool cheb = H.isCheby(k);
+    const bool flow = !cheb && H.flows(k);
     FlowRing ring;
-    if (!cheb && H.flows(k)) ring.init((size_t)V.n, sizeof(T), 1);
+    if (flow) ring.init((size_t)V.n, sizeof(T), 1);
     auto run = [&]() {
         if (cheb)
             k_cheb_step<T>(ex, R, x.p, t.p, b.p, w.p, (T)V.d1[1 % H.params.chebyDegree],
                            (T)V.d2[1 % H.params.chebyDegree], 0, Gate{});
-        else if (H.flows(k))
+        else if (flow)
             flow_gs<T>(ex, Lk, R, ring, x.p, b.p, 1, false, false, nullptr, nullptr, Gate{});
         else
             H.sweep<T>(ex, k, Lk, R, x.p, b.p, false, false, Gate{});
@@ -798,7 +802,7 @@ static double time_smoother(AmgHierarchy& H, cudaStream_t s, int k, int reps, do
     ring.check();
     if (bytes)
         *bytes = cheb ? cheb_bytes(V.n, Lk.nf, fp32, true) : sweep_bytes(V.n, V.n, Lk.nf, fp32);
-    if (launches) *launches = cheb || H.flows(k) ? 1 : Lk.nWave;
+    if (launches) *launches = cheb || flow ? 1 : Lk.nWave;
     return (double)ms / std::max(reps, 1);
 }
 
