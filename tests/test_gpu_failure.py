@@ -77,3 +77,37 @@ def test_size_mismatch_is_an_error(cuda):
                         ctypes.byref(ctypes.c_int(10)), ctypes.byref(ctypes.c_int(0)),
                         ctypes.byref(it), ctypes.byref(res))
     assert it.value == -1 and np.isnan(res.value)
+
+
+@pytest.mark.parametrize("what", [0, 1, 2, 3])
+def test_sweep_wait_bound_reports_timeout(cuda, orc, what):
+    """A sweep, a factorisation, an application and a whole solve whose waits
+    may poll once end and report it; the same matrix then works as before."""
+    torch = cuda
+    s = W.laplace(40, 30, 20, seed=5)
+    A = capi.DeviceMatrix(s)
+    t = ctypes.c_int(-1)
+    capi.check(capi.load().unap_cuda_selftest_wait_timeout(A.handle, what, ctypes.byref(t)))
+    assert t.value == 1
+    r = np.random.default_rng(1).standard_normal(s.n)
+    w = torch.zeros(s.n, dtype=torch.float64, device="cuda")
+    A.precondition(2, torch.tensor(r, device="cuda"), w)
+    assert np.array_equal(w.cpu().numpy(), orc.precond(2, s, r)[0])
+    x = torch.tensor(r, device="cuda")
+    A.gauss_seidel(x, torch.tensor(s.b, device="cuda"), 2)
+    assert np.array_equal(x.cpu().numpy(), orc.gs(s, r, s.b, 2))
+    A.close()
+
+
+@pytest.mark.parametrize("smoother", [0, 1])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_vcycle_wait_bound_is_an_error(cuda, smoother, precision):
+    """A V-cycle whose waits may poll once fails with an error (Gauss-Seidel
+    sweeps, the Chebyshev tail)."""
+    s = W.laplace(40, 30, 20, seed=6)
+    A = capi.DeviceMatrix(s)
+    G = capi.DeviceAmg(A, n_coarsest=60, precision=precision, smoother=smoother)
+    with pytest.raises(capi.UnapCudaError, match="ran out"):
+        capi.check(capi.load().unap_cuda_selftest_vcycle_timeout(G.handle))
+    G.close()
+    A.close()

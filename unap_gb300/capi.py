@@ -129,6 +129,8 @@ SIGNATURES = {
                                          ctypes.POINTER(_c_ll)]),
     "unap_cuda_tail_cluster_size": (_c_int, [_ip]),
     "unap_cuda_selftest_barrier_timeout": (_c_int, [_ip, _ip]),
+    "unap_cuda_selftest_wait_timeout": (_c_int, [_c_long, _c_int, _ip]),
+    "unap_cuda_selftest_vcycle_timeout": (_c_int, [_c_long]),
     "mgsolversolve_": (None, [_dp, _lp, _dp, _ip, _ip, _ip, _dp, _dp, _ip, _ip, _ip, _dp, _dp]),
     "contruct_solver_mg__": (None, [_lp, _lp, _lp, _dp, _ip, _ip, _ip]),
     "sw_solver_mg_set_maxiter__": (None, [_lp, _ip]),

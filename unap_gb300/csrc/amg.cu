@@ -335,6 +335,12 @@ void AmgHierarchy::check() const
     tail64.check();
 }
 
+void AmgHierarchy::setWaitPolls(int polls)
+{
+    for (auto& l : lv) l.sweeps.polls = polls;
+    tail32.polls = tail64.polls = polls;
+}
+
 int AmgHierarchy::tailFirst(size_t elemBytes) const
 {
     const int L = nLevels() - 1;

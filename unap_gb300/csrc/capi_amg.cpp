@@ -5,6 +5,7 @@
 
 #include "amg.hpp"
 #include "capi_handles.hpp"
+#include "small_solve.hpp"
 #include "../../include/unap_cuda.h"
 
 using namespace unapgpu;
@@ -295,6 +296,88 @@ int unap_cuda_set_tail_rows(int precision, long long tailRows, long long singleR
 int unap_cuda_tail_cluster_size(int* clusterSize)
 {
     return guarded([&] { *clusterSize = tail_cluster_size(); });
+}
+
+int unap_cuda_selftest_wait_timeout(long int handle, int what, int* timedOut)
+{
+    return guarded([&] {
+        Matrix& A = mat_from(handle)->get();
+        const Level& L = *A.L;
+        if (!L.sweepable) throw std::invalid_argument("the matrix has no wavefronts");
+        const int n = A.n();
+        Exec ex{A.stream, device_max_blocks()};
+        DevArray<double> x((size_t)n), b((size_t)n);
+        k_fill<double>(ex, n, x.p, 1.0);
+        k_fill<double>(ex, n, b.p, 1.0);
+        FlowRing ring;
+        DicFlow D;
+        DevArray<double> work;
+        DevArray<unsigned char> sys;
+        std::vector<unsigned char> hostSys(sizeof(SmallSystem));
+        if (what != 0) D.init(L);
+        if (what >= 2) flow_dic_factor(ex, L, !L.symm, D);
+        UNAP_CK(cudaStreamSynchronize(ex.s));
+        D.check();
+        D.ring.polls = 1;
+        if (what == 0) {
+            ring.init((size_t)n, sizeof(double), 2);
+            ring.polls = 1;
+            flow_gs<double>(ex, L, rows64(L), ring, x.p, b.p, 2, false, false, nullptr, nullptr,
+                            Gate{});
+        } else if (what == 1) {
+            flow_dic_factor(ex, L, !L.symm, D);
+        } else if (what == 2) {
+            flow_dic_apply(ex, L, D, b.p, x.p, nullptr, 0, nullptr, FIN_NONE, Gate{});
+        } else if (what == 3) {
+            work.alloc((size_t)kTeamWorkPcg * (size_t)n);
+            SmallSystem S{};
+            S.A = rows64(L);
+            S.nWave = L.nWave;
+            small_sweeps(S, L, D);
+            S.precond = L.symm ? 2 : 3;
+            S.maxIter = 3;
+            S.zeroX = 1;
+            S.x = x.p;
+            S.b = b.p;
+            S.work = work.p;
+            std::memcpy(hostSys.data(), &S, sizeof S);
+            sys.upload(hostSys, ex.s);
+            launch_small_krylov(ex.s, reinterpret_cast<const SmallSystem*>(sys.p), 1, nullptr, 256, 8);
+        } else {
+            throw std::invalid_argument("what is 0 to 3");
+        }
+        UNAP_CK(cudaGetLastError());
+        UNAP_CK(cudaStreamSynchronize(ex.s));
+        int out = 0;
+        try {
+            ring.check();
+            D.check();
+        } catch (const CudaError&) {
+            out = 1;
+        }
+        if (timedOut) *timedOut = out;
+    });
+}
+
+int unap_cuda_selftest_vcycle_timeout(long int amg)
+{
+    return guarded([&] {
+        AmgHandle* h = amg_from(amg);
+        Matrix& A = *h->A;
+        Exec ex{A.stream, device_max_blocks()};
+        const int n = A.n();
+        DevArray<double> r((size_t)n), z((size_t)n);
+        k_fill<double>(ex, n, r.p, 1.0);
+        struct Restore {
+            AmgHierarchy& H;
+            ~Restore() { H.setWaitPolls(kWaitPolls); }
+        } restore{*h->H};
+        h->H->setWaitPolls(1);
+        h->H->vcycle(ex, r.p, z.p, Gate{});
+        UNAP_CK(cudaGetLastError());
+        UNAP_CK(cudaStreamSynchronize(A.stream));
+        h->H->check();
+    });
 }
 
 int unap_cuda_selftest_barrier_timeout(int* timedOut, int* recovered)

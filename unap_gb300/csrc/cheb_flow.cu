@@ -68,7 +68,7 @@ struct Args {
     double* part;      // its chunk sums, [chunk][row]
     int nc;
     unsigned* counter;
-    int* err;
+    WaitBound bound;
 };
 
 // the next task of this warp (flow.cu's counters)
@@ -83,10 +83,10 @@ __device__ __forceinline__ int take(unsigned* counters)
 
 // one value that another row of this launch writes; all lanes call it
 template <class T>
-__device__ __forceinline__ T wait_one(const T* p, bool on, int* err)
+__device__ __forceinline__ T wait_one(const T* p, bool on, WaitBound b)
 {
     T v[1] = {T(0)};
-    wait_values<T, 1>(on ? 1u : 0u, [&](int) { return p; }, v, err);
+    wait_values<T, 1>(on ? 1u : 0u, [&](int) { return p; }, v, b);
     return v[0];
 }
 
@@ -116,7 +116,7 @@ __device__ __forceinline__ void row_task(const Args<T>& a, const Stage<T>& S, in
         v[k] = has ? ldg(S.A.val + base + 32 * (k * G + g)) : T(0);
     }
     const T rD = T(1) / d;
-    if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.err);
+    if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.bound);
     // the row's own values: x, b and w, a lane each
     const T* own = g == 0 ? S.a + r : g == 1 ? S.b + r : S.w + r;
     const bool mine = on && (g < 2 || (g == 2 && S.type == CF_STEP && !S.first));
@@ -132,7 +132,7 @@ __device__ __forceinline__ void row_task(const Args<T>& a, const Stage<T>& S, in
         all[K] = T(0);
         if (j0 == 0 && mine) need |= 1u << K;
         wait_values<T, K + 1>(
-            need, [&](int k) { return k == K ? own : S.a + c[k]; }, all, a.err);
+            need, [&](int k) { return k == K ? own : S.a + c[k]; }, all, a.bound);
 #pragma unroll
         for (int k = 0; k < K; ++k) pw[row * P + k * G + g] = v[k] * all[k];
         if (j0 == 0) {
@@ -204,7 +204,7 @@ __device__ __forceinline__ void restrict_task(const Args<T>& a, const Stage<T>& 
         k1 = ldg(S.i0 + r + 1);
         if (S.type == CF_ZERO) d = ldg(S.A.diag + r);
     }
-    if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.err);
+    if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.bound);
     T acc = T(0);
     for (; __any_sync(0xffffffffu, k0 < k1); k0 += 4) {
         int c[4];
@@ -218,7 +218,7 @@ __device__ __forceinline__ void restrict_task(const Args<T>& a, const Stage<T>& 
             if (has) need |= 1u << k;
         }
         if (S.pollA) {
-            wait_values<T, 4>(need, [&](int k) { return S.a + c[k]; }, v, a.err);
+            wait_values<T, 4>(need, [&](int k) { return S.a + c[k]; }, v, a.bound);
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -264,9 +264,9 @@ __global__ void __launch_bounds__(kThreads) cheb_flow_kernel(const __grid_consta
             const int r0 = i * 32, r = r0 + lane;
             const bool on = r < S.n;
             const int c = on ? ldg(S.i0 + r) : 0;
-            if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.err);
+            if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.bound);
             T v[2];
-            wait_values<T, 2>(on ? 3u : 0u, [&](int k) { return k ? S.a + c : S.b + r; }, v, a.err);
+            wait_values<T, 2>(on ? 3u : 0u, [&](int k) { return k ? S.a + c : S.b + r; }, v, a.bound);
             if (on) st_flow(S.x + r, v[0] + v[1]);
         } else if (S.type == CF_CHUNK) {
             // a column chunk of 32 rows of x = Minv b, summed in ascending
@@ -277,10 +277,10 @@ __global__ void __launch_bounds__(kThreads) cheb_flow_kernel(const __grid_consta
             double mv[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) mv[k] = k < m ? ldg(M + (size_t)k * a.nc) : 0.0;
-            if (S.wait) wait_near(S.near + (int)((long long)j0 * S.wait / S.n), a.err);
+            if (S.wait) wait_near(S.near + (int)((long long)j0 * S.wait / S.n), a.bound);
             __syncwarp();
             for (int j = lane; j < kDenseChunk; j += 32) {
-                const T b = wait_one<T>(S.a + j0 + j, j < m, a.err);
+                const T b = wait_one<T>(S.a + j0 + j, j < m, a.bound);
                 sb[warp][j] = (double)b;
             }
             __syncwarp();
@@ -309,13 +309,13 @@ __global__ void __launch_bounds__(kThreads) cheb_flow_kernel(const __grid_consta
             const int r = i * 32 + lane;
             const bool on = r < a.nc;
             const int nq = (a.nc + kDenseChunk - 1) / kDenseChunk;
-            if (S.wait) wait_near(S.near + (int)((long long)i * 32 * S.wait / S.n), a.err);
+            if (S.wait) wait_near(S.near + (int)((long long)i * 32 * S.wait / S.n), a.bound);
             double t_ = 0.0;
             for (int q0 = 0; q0 < nq; q0 += 4) {
                 double v[4];
                 const unsigned need = on ? (1u << min(4, nq - q0)) - 1u : 0u;
                 wait_values<double, 4>(
-                    need, [&](int k) { return a.part + (size_t)(q0 + k) * a.nc + r; }, v, a.err);
+                    need, [&](int k) { return a.part + (size_t)(q0 + k) * a.nc + r; }, v, a.bound);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     if (q0 + k < nq) t_ += v[k];
@@ -492,7 +492,7 @@ void ChebFlow<T>::launch(const Exec& ex, Gate g) const
     a.part = part;
     a.nc = nc;
     a.counter = reinterpret_cast<unsigned*>(arena.p);
-    a.err = err;
+    a.bound = wait_bound(err, polls);
     UNAP_CK(cudaMemsetAsync(arena.p, 0xff, arena.n, ex.s));
     if (!capturing()) count_launches(1);
     cheb_flow_kernel<T><<<grid, kThreads, 0, ex.s>>>(a, g);

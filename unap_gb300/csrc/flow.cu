@@ -18,9 +18,9 @@
 // another still reads, and several sweeps run in one launch, each following
 // the one before by its own waits.
 //
-// Every wait is bounded: after kSpinLimit polls, or once another wait of the
-// same ring gave up, it sets the ring's error word and goes on with what it
-// has; the host turns that into an error (FlowRing::check).
+// Every wait is bounded (WaitBound): one that runs out, or that sees that
+// another wait of the same ring did, goes on with what it has, and the host
+// turns the ring's error word into an error (FlowRing::check).
 #include <algorithm>
 
 #include "flow.hpp"
@@ -63,7 +63,7 @@ struct GsArgs {
     const int* copyAt;  // row r at copyAt[r] if given
     const T* b;
     unsigned* counter;
-    int* err;
+    WaitBound bound;
 };
 
 // G lanes a row, K entries a lane, so that a row is loaded whole before its
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kFlowThreads)
         }
         const int nLow = row_low(info);
         const int jEnd = !BWD && s == 0 && a.firstFromZero ? nLow : row_len(info);
-        if ((BWD ? nr.y : nr.x) >= 0) wait_near(out + (BWD ? nr.y : nr.x), a.err);
+        if ((BWD ? nr.y : nr.x) >= 0) wait_near(out + (BWD ? nr.y : nr.x), a.bound);
         for (int j0 = 0;;) {
             unsigned need = 0;
             auto at = [&](int k) {
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kFlowThreads)
                         xv[k] = *at(k);
                 }
             }
-            wait_values<T, K>(need, at, xv, a.err);
+            wait_values<T, K>(need, at, xv, a.bound);
             if (G == 1) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) xv[k] = v[k] * xv[k];
@@ -199,7 +199,7 @@ template <int CK>
 __global__ void __launch_bounds__(kFlowThreads)
     flow_factor_kernel(Rows<double> A, const int4* task, const int2* near, int nTasks,
                        const double* c1, const double* c2, double* d, double* rD, double* f,
-                       unsigned* counter, int* err)
+                       unsigned* counter, WaitBound bound)
 {
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(kFlowThreads)
                 xv[k] = 1.0;
                 if (has) need |= 1u << k;
             }
-            if (j0 == 0 && wait >= 0) wait_near(d + wait, err);
-            wait_values<double, CK>(need, [&](int k) { return (const double*)d + c[k]; }, xv, err);
+            if (j0 == 0 && wait >= 0) wait_near(d + wait, bound);
+            wait_values<double, CK>(need, [&](int k) { return (const double*)d + c[k]; }, xv, bound);
 #pragma unroll
             for (int k = 0; k < CK; ++k)
                 if (j0 + k < most) xv[k] = v[k] / xv[k];
@@ -271,7 +271,7 @@ struct DicArgs {
     double* w;
     double* part;  // partial of w.r per task, or null
     unsigned* counter;
-    int* err;
+    WaitBound bound;
 };
 
 // w = M^-1 r (lduDICPrecond.cpp:45-77, lduDILUPrecond.cpp:46-86): the forward
@@ -330,10 +330,10 @@ __global__ void __launch_bounds__(kFlowThreads) flow_dic_kernel(const __grid_con
             }
             xv[CK] = 0.0;
             if (bwd && on && j0 == 0) need |= 1u << CK;
-            if (j0 == 0 && wait >= 0) wait_near(out + wait, a.err);
+            if (j0 == 0 && wait >= 0) wait_near(out + wait, a.bound);
             wait_values<double, CK + 1>(
                 need, [&](int k) { return k == CK ? a.wf + r : (const double*)out + c[k]; }, xv,
-                a.err);
+                a.bound);
             if (bwd && j0 == 0) acc = xv[CK];
 #pragma unroll
             for (int k = 0; k < CK; ++k) {
@@ -498,7 +498,7 @@ T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& rin
         a.copyAt = copyAt;
         a.b = b;
         a.counter = ring.counter(h);
-        a.err = ring.err;
+        a.bound = ring.bound();
         const int own = end && last ? m - 1 : m;  // vectors of the ring this launch writes
         UNAP_CK(cudaMemsetAsync(ring.counter(h), 0xff, kFlowHeader + ring.stride * (size_t)own, ex.s));
         if (own < m) UNAP_CK(cudaMemsetAsync(last, 0xff, vecBytes, ex.s));
@@ -543,7 +543,7 @@ void flow_dic_factor(const Exec& ex, const Level& L, bool dilu, DicFlow& D)
     tick();
     flow_factor_kernel<8><<<flow_grid(L.tasks[0].n), kFlowThreads, 0, ex.s>>>(
         A, L.tasks[0].task.p, L.tasks[0].near.p, L.tasks[0].n, c1, c2, d, D.rD.p, D.f.p,
-        D.ring.counter(0), D.ring.err);
+        D.ring.counter(0), D.ring.bound());
     UNAP_CK(cudaGetLastError());
 }
 
@@ -563,7 +563,7 @@ void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const doub
     a.w = w;
     a.part = pool ? D.part.p : nullptr;
     a.counter = D.ring.counter(1);
-    a.err = D.ring.err;
+    a.bound = D.ring.bound();
     UNAP_CK(cudaMemsetAsync(a.counter, 0xff, kFlowHeader + D.ring.stride, ex.s));
     UNAP_CK(cudaMemsetAsync(w, 0xff, (size_t)L.n * sizeof(double), ex.s));
     tick();
@@ -583,7 +583,7 @@ void small_sweeps(SmallSystem& S, const Level& L, const DicFlow& D)
     S.task = L.tasks[0].task.p;
     S.near = L.tasks[0].near.p;
     S.nTasks = L.tasks[0].n;
-    S.err = D.ring.err;
+    S.bound = D.ring.bound();
 }
 
 }  // namespace unapgpu

@@ -24,6 +24,7 @@ struct FlowRing {
     size_t half = 0;     // bytes of one half
     int sweeps = 0;      // vectors of one half
     int* err = nullptr;  // pinned: set by a launch whose wait ran out
+    int polls = kWaitPolls;  // of its waits
     FlowRing() = default;
     FlowRing(const FlowRing&) = delete;
     FlowRing& operator=(const FlowRing&) = delete;
@@ -32,6 +33,7 @@ struct FlowRing {
     ~FlowRing();
     void init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves = 2);
     size_t bytes() const { return mem.bytes(); }
+    WaitBound bound() const { return wait_bound(err, polls); }
     // the half (0 or 1) that does not hold p
     int other(const void* p) const;
     unsigned* counter(int h) const { return reinterpret_cast<unsigned*>(mem.p + h * half); }

@@ -6,7 +6,7 @@
 namespace unapgpu {
 
 FlowRing::FlowRing(FlowRing&& o) noexcept
-    : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), err(o.err)
+    : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), err(o.err), polls(o.polls)
 {
     o.err = nullptr;
 }
@@ -18,6 +18,7 @@ FlowRing& FlowRing::operator=(FlowRing&& o) noexcept
     half = o.half;
     sweeps = o.sweeps;
     std::swap(err, o.err);
+    polls = o.polls;
     return *this;
 }
 

@@ -1,13 +1,11 @@
 // Values as their own flags (see flow.cu): a vector starts as 0xff bytes, a
 // row's value is one relaxed store, a reader loads until it sees something
-// else.  Waits are bounded by kSpinLimit polls.
+// else.  Waits are bounded (WaitBound).
 #pragma once
 
 #include "device_common.cuh"
 
 namespace unapgpu {
-
-constexpr int kSpinLimit = 1 << 23;  // polls; one is 0.3 us or more
 
 // ---- values that say whether they are there -------------------------------
 __device__ __forceinline__ float ld_flow(const float* p)
@@ -36,11 +34,11 @@ __device__ __forceinline__ void st_flow(double* p, double v)
 }
 
 // One more poll of a wait: true when the wait has to be given up.
-__device__ __forceinline__ bool give_up(int& spins, int* err)
+__device__ __forceinline__ bool give_up(int& spins, WaitBound b)
 {
-    if ((++spins & 0xfff) == 0) {
-        if (spins >= kSpinLimit) *(volatile int*)err = 1;
-        if (*(volatile int*)err) return true;
+    if ((++spins & b.mask) == 0) {
+        if (spins >= b.polls) *(volatile int*)b.err = 1;
+        if (*(volatile int*)b.err) return true;
     }
     return false;
 }
@@ -48,7 +46,7 @@ __device__ __forceinline__ bool give_up(int& spins, int* err)
 // Loads at(k) for the entries in `need` (one bit each) until every value is
 // there; all lanes of the warp call it.
 template <class T, int CK, class At>
-__device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], int* err)
+__device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], WaitBound b)
 {
     int spins = 0;
     for (;;) {
@@ -59,7 +57,7 @@ __device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], 
         for (int k = 0; k < CK; ++k)
             if ((need >> k & 1u) && !absent(v[k])) need &= ~(1u << k);
         if (!__any_sync(0xffffffffu, need != 0)) return;
-        if (give_up(spins, err)) return;
+        if (give_up(spins, b)) return;
     }
 }
 
@@ -67,12 +65,12 @@ __device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], 
 // until a row two wavefronts before its own is there, the whole warp polls
 // that one address, with pauses.
 template <class T>
-__device__ __forceinline__ void wait_near(const T* p, int* err)
+__device__ __forceinline__ void wait_near(const T* p, WaitBound b)
 {
     int spins = 0;
     while (absent(ld_flow(p))) {
         __nanosleep(64);
-        if (give_up(spins, err)) return;
+        if (give_up(spins, b)) return;
     }
 }
 

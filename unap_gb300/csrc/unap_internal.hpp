@@ -269,6 +269,21 @@ struct HostLdu {
     void validate();
 };
 
+// Bound of a launch's waits for values that other warps write: after `polls`
+// polls (0.3 us or more each), or once *err is set, a wait goes on with what it
+// has; the one that ran out sets *err (pinned host memory), which the host turns
+// into an error once the launch is done.
+constexpr int kWaitPolls = 1 << 23;
+struct WaitBound {
+    int* err;
+    int polls;  // a power of two
+    int mask;   // both are looked at every mask + 1 polls
+};
+inline WaitBound wait_bound(int* err, int polls)
+{
+    return {err, polls, polls < 4096 ? polls - 1 : 4095};
+}
+
 // A row's entry counts in one word: all entries in the low 16 bits, those of
 // the lower side in the high 16, both unsigned (rows of up to 65,535 faces).
 __host__ __device__ inline int row_info(int len, int low)
