@@ -111,3 +111,23 @@ def test_vcycle_wait_bound_is_an_error(cuda, smoother, precision):
         capi.check(capi.load().unap_cuda_selftest_vcycle_timeout(G.handle))
     G.close()
     A.close()
+
+
+@pytest.mark.parametrize("smoother", [0, 1])
+def test_vcycle_works_after_a_wait_ran_out(cuda, smoother):
+    """Waits run out on every level of one V-cycle: it fails, once, and the
+    next one has the bits of the one before."""
+    torch = cuda
+    s = W.laplace(40, 30, 20, seed=7)
+    A = capi.DeviceMatrix(s)
+    G = capi.DeviceAmg(A, n_coarsest=60, precision=0, smoother=smoother)
+    r = torch.tensor(np.random.default_rng(2).standard_normal(s.n), device="cuda")
+    z = torch.zeros_like(r)
+    G.vcycle(r, z)
+    want = z.cpu().numpy().copy()
+    assert capi.load().unap_cuda_selftest_vcycle_timeout(G.handle) != 0
+    z.zero_()
+    G.vcycle(r, z)
+    assert np.array_equal(z.cpu().numpy(), want)
+    G.close()
+    A.close()

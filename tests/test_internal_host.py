@@ -37,3 +37,7 @@ def test_failed_allocation_gives_the_workspace_pool_back(tmp_path):
 
 def test_failed_allocation_leaves_nothing_behind(tmp_path):
     assert "ok" in run_program("alloc_state", tmp_path, units=["flow_ring.cpp"])
+
+
+def test_growing_ring_keeps_its_error_word(tmp_path):
+    assert "ok" in run_program("ring_error_word", tmp_path, units=["flow_ring.cpp"])

@@ -330,9 +330,11 @@ std::vector<double> AmgHierarchy::eigenvalues() const
 
 void AmgHierarchy::check() const
 {
-    for (auto& l : lv) l.sweeps.check();
-    tail32.check();
-    tail64.check();
+    bool out = false;
+    for (auto& l : lv) out |= l.sweeps.ranOut();
+    out |= tail32.ranOut();
+    out |= tail64.ranOut();
+    if (out) throw_ran_out();
 }
 
 void AmgHierarchy::setWaitPolls(int polls)

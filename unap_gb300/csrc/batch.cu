@@ -386,10 +386,12 @@ void BatchSolver::solveSmall(const std::vector<BatchItem>& items, const std::vec
                             cudaMemcpyDeviceToHost, stream));
     UNAP_CK(cudaStreamSynchronize(stream));
     UNAP_CK(cudaGetLastError());
+    bool ranOut = false;
     for (int i : idx) {
         const BatchItem& it = items[(size_t)i];
-        if (it.precond >= 2 && it.precond <= 3) factor(*it.A, it.precond).check();
+        if (it.precond >= 2 && it.precond <= 3) ranOut |= factor(*it.A, it.precond).ring.ranOut();
     }
+    if (ranOut) throw_ran_out();
     for (int j = 0; j < m; ++j) {
         SolveStats& s = out[(size_t)idx[(size_t)j]];
         s.nIter = res[(size_t)j].nIter;

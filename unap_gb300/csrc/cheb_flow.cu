@@ -500,15 +500,6 @@ void ChebFlow<T>::launch(const Exec& ex, Gate g) const
 }
 
 template <class T>
-void ChebFlow<T>::check() const
-{
-    if (err && *(volatile int*)err) {
-        *(volatile int*)err = 0;
-        throw CudaError("Chebyshev tail: a wait for a value ran out");
-    }
-}
-
-template <class T>
 ChebFlow<T>::~ChebFlow()
 {
     pinned_block_free(err);

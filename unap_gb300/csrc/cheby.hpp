@@ -125,7 +125,7 @@ struct ChebFlow {
                const int* cChildStart, const int* cChild, const int* cCmap, const double* Minv,
                T* result, cudaStream_t s);
     void launch(const Exec& ex, Gate g) const;
-    void check() const;  // throws when a wait ran out (after synchronizing)
+    bool ranOut() const { return wait_ran_out(err); }  // a wait (after synchronizing)
     size_t bytes() const { return arena.bytes() + stages.bytes(); }
 };
 

@@ -38,10 +38,13 @@ struct FlowRing {
     int other(const void* p) const;
     unsigned* counter(int h) const { return reinterpret_cast<unsigned*>(mem.p + h * half); }
     unsigned char* vec(int h, int i) const { return mem.p + h * half + kFlowHeader + i * stride; }
-    // throws when a wait of one of this ring's launches ran out (call after
-    // synchronizing with them)
+    // whether a wait of one of this ring's launches ran out since the last call
+    // (after synchronizing with them); check() throws if so
+    bool ranOut() const { return wait_ran_out(err); }
     void check() const;
 };
+
+[[noreturn]] void throw_ran_out();
 
 // nSweeps Gauss-Seidel sweeps (forward, or backward in reverse cell order)
 // from `in`; xIsZero: in is zero (forward, the first sweep then reads only

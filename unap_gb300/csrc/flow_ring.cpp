@@ -31,8 +31,11 @@ void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves)
     const int per = std::max(1, std::min(sweepsPerHalf, kFlowMaxSweeps));
     stride = (n * elemBytes + 255) / 256 * 256;
     half = kFlowHeader + stride * (size_t)per;
-    if (!err) err = static_cast<int*>(pinned_block_alloc(64));
-    *err = 0;
+    if (!err) {
+        // not cleared when the ring grows: a launch on it may have set it
+        err = static_cast<int*>(pinned_block_alloc(64));
+        *err = 0;
+    }
     mem.alloc((size_t)halves * half);
     sweeps = per;
 }
@@ -43,12 +46,14 @@ int FlowRing::other(const void* p) const
     return q >= mem.p && q < mem.p + half ? 1 : 0;
 }
 
+void throw_ran_out()
+{
+    throw CudaError("a wait for another row of a sweep ran out");
+}
+
 void FlowRing::check() const
 {
-    if (err && *(volatile int*)err) {
-        *(volatile int*)err = 0;
-        throw CudaError("wavefront sweep: a wait for a neighbouring row ran out");
-    }
+    if (ranOut()) throw_ran_out();
 }
 
 }  // namespace unapgpu

@@ -389,8 +389,10 @@ SolveStats MgSolver::solveDevice(double* x_ref, const double* b_ref)
             UNAP_CK(cudaGetLastError());
             UNAP_CK(cudaMemcpyAsync(h_st, d_st, sizeof(KState), cudaMemcpyDeviceToHost, ex.s));
             UNAP_CK(cudaStreamSynchronize(ex.s));
-            for (auto& K : lv) K.sweeps.check();
-            lv.back().dic.check();
+            bool ranOut = false;
+            for (auto& K : lv) ranOut |= K.sweeps.ranOut();
+            ranOut |= lv.back().dic.ring.ranOut();
+            if (ranOut) throw_ran_out();
             if (h_st->done) break;
         }
     } else {

@@ -279,6 +279,16 @@ struct WaitBound {
     int polls;  // a power of two
     int mask;   // both are looked at every mask + 1 polls
 };
+// Whether a launch that used the word set it; the word is cleared.  A call over
+// several words reads them all before it throws, or those after the first one
+// set would stay set and fail a later call.
+inline bool wait_ran_out(int* err)
+{
+    volatile int* e = err;
+    if (!e || !*e) return false;
+    *e = 0;
+    return true;
+}
 inline WaitBound wait_bound(int* err, int polls)
 {
     return {err, polls, polls < 4096 ? polls - 1 : 4095};
