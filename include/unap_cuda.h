@@ -447,6 +447,9 @@ typedef struct {
     double queueSeconds, setupSeconds, solveSeconds, latencySeconds;
 } unap_cuda_request_info;
 
+/* Device memory that the admission counts for a request of this size and
+ * method: the most it holds at once, its setup included. */
+int unap_cuda_server_request_bytes(int nCells, int nFaces, int symm, int method, long long* bytes);
 int unap_cuda_server_create(long int* server, long long memoryBudget, int maxSlots,
                             int smallCells);
 int unap_cuda_server_submit(long int server, int nCells, int nFaces, const int* lowerAddr,

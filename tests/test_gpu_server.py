@@ -3,6 +3,7 @@ are on the GPU are admitted as slots and memory free up, small ones are
 batched into one launch, and every result is the same as the same solve run
 alone (within the solver tolerance: +-1 iteration, 2.2 relTol ||r0|| in
 residual space), including under a memory budget that forces queueing."""
+import ctypes
 import threading
 import time
 
@@ -73,3 +74,37 @@ def test_results_same_alone_and_in_the_mix(cuda, orc, budget):
         assert info["latencySeconds"] >= info["solveSeconds"] >= 0
     assert batched >= 1
     srv.close()
+
+
+@pytest.mark.parametrize("method", sorted(capi.SERVE_METHODS))
+@pytest.mark.parametrize("dims,small_cells", [((20, 20, 20), 0), ((31, 32, 30), 0),
+                                              ((110, 66, 70), 0), ((300, 300, 3), 0),
+                                              ((31, 32, 30), 65536)])
+def test_admission_covers_what_a_request_holds(cuda, method, dims, small_cells):
+    """The most device memory a request holds at once (its slot allocates from
+    the device's default pool) is within what the admission counts for it."""
+    lib = capi.load()
+    pool = ctypes.c_void_p()
+    assert lib.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+    def used(attribute):  # cudaMemPoolAttrUsedMemCurrent 7, ...UsedMemHigh 8
+        v = ctypes.c_ulonglong()
+        assert lib.cudaMemPoolGetAttribute(pool, attribute, ctypes.byref(v)) == 0
+        return v.value
+
+    make = W.convdiff if method == "bicgstab_dilu" else W.lognormal
+    s = make(*dims, seed=1, permute=True)
+    estimate = ctypes.c_longlong()
+    capi.check(lib.unap_cuda_server_request_bytes(s.n, s.nf, int(s.symm),
+                                                  capi.SERVE_METHODS[method],
+                                                  ctypes.byref(estimate)))
+    srv = capi.Server(max_slots=1, small_cells=small_cells)
+    srv.wait(srv.submit(s, method, rel_tol=1e-2), s.n)
+    before = used(7)
+    zero = ctypes.c_ulonglong(0)
+    assert lib.cudaMemPoolSetAttribute(pool, 8, ctypes.byref(zero)) == 0
+    _, info = srv.wait(srv.submit(s, method, rel_tol=1e-2), s.n)
+    held = used(8) - before
+    srv.close()
+    assert info["status"] == 0
+    assert 0 < held <= estimate.value, (held, estimate.value)

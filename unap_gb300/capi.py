@@ -159,6 +159,8 @@ SIGNATURES = {
     "unap_cuda_set_cheby_tail_rows": (_c_int, [_c_int]),
     "unap_cuda_set_server_team_cells": (_c_int, [_c_int]),
     "unap_cuda_set_server_amg": (_c_int, [_c_int, _c_dbl]),
+    "unap_cuda_server_request_bytes": (_c_int, [_c_int, _c_int, _c_int, _c_int,
+                                                ctypes.POINTER(_c_ll)]),
     "unap_cuda_server_create": (_c_int, [_lp, _c_ll, _c_int, _c_int]),
     "unap_cuda_server_submit": (_c_int, [_c_long, _c_int, _c_int, _vp, _vp, _vp, _vp, _vp, _vp,
                                          _c_int, _c_dbl, _c_int, ctypes.POINTER(_c_ll)]),

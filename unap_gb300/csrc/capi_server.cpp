@@ -49,6 +49,16 @@ int guarded(F&& f)
 
 extern "C" {
 
+int unap_cuda_server_request_bytes(int nCells, int nFaces, int symm, int method, long long* bytes)
+{
+    return guarded([&] {
+        if (nCells < 0 || nFaces < 0 || method < 0 || method > SERVE_BICG_DILU)
+            throw std::invalid_argument("request size or method out of range");
+        if (bytes)
+            *bytes = (long long)serve_request_bytes((size_t)nCells, (size_t)nFaces, symm != 0, method);
+    });
+}
+
 int unap_cuda_server_create(long int* server, long long memoryBudget, int maxSlots,
                             int smallCells)
 {

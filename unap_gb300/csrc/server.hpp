@@ -50,6 +50,9 @@ int set_server_team_cells(int cells);
 // interval ratio (default 30), for requests started afterwards
 void set_server_amg(int nCoarsest, double eigRatio);
 
+// Device memory that the admission of a request counts for it.
+size_t serve_request_bytes(size_t nCells, size_t nFaces, bool symm, int method);
+
 struct ServerParams {
     long long memoryBudget = 0;  // bytes; 0: 80% of free device memory at start
     int maxSlots = 4;            // concurrent large solves (one stream each)
