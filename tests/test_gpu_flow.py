@@ -118,3 +118,19 @@ def test_chebyshev_tail_long_rows(cuda, precision, degree):
         G.close()
     assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
     A.close()
+
+
+def test_matrix_keeps_one_vector_a_sweep(cuda):
+    """Four sweeps leave four vectors (and the call's two) with the matrix."""
+    torch = cuda
+    s = W.laplace(160, 160, 80, seed=1)
+    A = capi.DeviceMatrix(s)
+    b = torch.tensor(s.b, device="cuda")
+    x = torch.zeros_like(b)
+    A.spmv(b, x)  # the call's two vectors
+    torch.cuda.synchronize()
+    free0, _ = torch.cuda.mem_get_info()
+    A.gauss_seidel(x, b, 4)
+    free1, _ = torch.cuda.mem_get_info()
+    assert free0 - free1 <= 4 * 8 * s.n + (4 << 20)
+    A.close()

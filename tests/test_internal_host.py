@@ -41,3 +41,7 @@ def test_failed_allocation_leaves_nothing_behind(tmp_path):
 
 def test_growing_ring_keeps_its_error_word(tmp_path):
     assert "ok" in run_program("ring_error_word", tmp_path, units=["flow_ring.cpp"])
+
+
+def test_sweeps_keep_what_their_launches_write(tmp_path):
+    assert "ok" in run_program("ring_storage", tmp_path, units=["flow_ring.cpp"])

@@ -220,6 +220,7 @@ const DicFlow& BatchSolver::factor(Matrix& A, int precond)
         flow_dic_factor(Exec{stream, device_max_blocks()}, *A.L, precond == 3, f.D);
         UNAP_CK(cudaStreamSynchronize(stream));
         f.D.check();
+        f.D.keepFactor();
     }
     UNAP_CK(cudaStreamSynchronize(stream));
     auto& slot = factors[k];

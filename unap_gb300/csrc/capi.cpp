@@ -596,8 +596,7 @@ int unap_cuda_gauss_seidel(long int handle, double* x, const double* b, int nSwe
         k_to_internal<double>(ex, A.n(), A.L->d_perm.p, b, h->s2.p);
         Rows<double> R = rows64(*A.L);
         // up to four sweeps a launch, each following the one before
-        const int per = std::min(nSweeps, 4);
-        if (h->sweeps.sweeps < per) h->sweeps.init((size_t)A.n(), sizeof(double), per);
+        h->sweeps.ensure((size_t)A.n(), sizeof(double), nSweeps, 4);
         // x and b are copied, so the last sweep may write x
         flow_gs<double>(ex, *A.L, R, h->sweeps, h->s1.p, h->s2.p, nSweeps, backward != 0, false,
                         nullptr, x, Gate{}, A.L->d_perm.p);

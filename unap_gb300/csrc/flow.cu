@@ -521,14 +521,6 @@ template double* flow_gs<double>(const Exec&, const Level&, const Rows<double>&,
                                  const double*, const double*, int, bool, bool, double*, double*,
                                  Gate, const int*);
 
-void DicFlow::init(const Level& L)
-{
-    rD.alloc((size_t)L.n);
-    f.alloc((size_t)L.nEntries);
-    part.alloc((size_t)std::max(L.tasks[0].n, 1));
-    ring.init((size_t)L.n, sizeof(double), 1);
-}
-
 void flow_dic_factor(const Exec& ex, const Level& L, bool dilu, DicFlow& D)
 {
     if (L.n <= 0) return;
@@ -559,10 +551,10 @@ void flow_dic_apply(const Exec& ex, const Level& L, const DicFlow& D, const doub
     a.f = D.f.p;
     a.rD = D.rD.p;
     a.r = r;
-    a.wf = reinterpret_cast<double*>(D.ring.vec(1, 0));
+    a.wf = reinterpret_cast<double*>(D.ring.vec(0, 0));
     a.w = w;
     a.part = pool ? D.part.p : nullptr;
-    a.counter = D.ring.counter(1);
+    a.counter = D.ring.counter(0);
     a.bound = D.ring.bound();
     UNAP_CK(cudaMemsetAsync(a.counter, 0xff, kFlowHeader + D.ring.stride, ex.s));
     UNAP_CK(cudaMemsetAsync(w, 0xff, (size_t)L.n * sizeof(double), ex.s));

@@ -23,6 +23,7 @@ struct FlowRing {
     size_t stride = 0;   // bytes of one vector
     size_t half = 0;     // bytes of one half
     int sweeps = 0;      // vectors of one half
+    int halves = 0;
     int* err = nullptr;  // pinned: set by a launch whose wait ran out
     int polls = kWaitPolls;  // of its waits
     FlowRing() = default;
@@ -31,10 +32,15 @@ struct FlowRing {
     FlowRing(FlowRing&& o) noexcept;
     FlowRing& operator=(FlowRing&& o) noexcept;
     ~FlowRing();
-    void init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves = 2);
+    void init(size_t n, size_t elemBytes, int sweepsPerHalf, int nHalves = 2);
+    // grows to what nSweeps sweeps from an input outside the ring need, with up
+    // to `most` of them in a launch: one half, or two if a launch follows that
+    // reads the one before
+    void ensure(size_t n, size_t elemBytes, int nSweeps, int most);
     size_t bytes() const { return mem.bytes(); }
     WaitBound bound() const { return wait_bound(err, polls); }
-    // the half (0 or 1) that does not hold p
+    // the half (0 or 1) that does not hold p; throws if the ring has one and
+    // p is in it
     int other(const void* p) const;
     unsigned* counter(int h) const { return reinterpret_cast<unsigned*>(mem.p + h * half); }
     unsigned char* vec(int h, int i) const { return mem.p + h * half + kFlowHeader + i * stride; }
@@ -60,12 +66,15 @@ T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& rin
 
 // DIC / DILU.  rD: the factored diagonal's reciprocal; f: every entry times
 // its row's reciprocal (rD coef on the lower side, rD upper on the upper
-// side); part: partial sums of w.r, one per task; ring: the factored diagonal
-// and the forward sweep's vector.
+// side); part: partial sums of w.r, one per task; ring: the factored diagonal,
+// then the forward sweep's vector.
 struct DicFlow {
     DevArray<double> rD, f, part;
     FlowRing ring;
     void init(const Level& L);
+    // after the factorisation, where only whole-solve launches use it (their
+    // sweeps' vectors are in the solve's workspace): drops what they do not read
+    void keepFactor();
     void check() const { ring.check(); }
 };
 // factors the level's matrix (DIC, or DILU); check() once it is done

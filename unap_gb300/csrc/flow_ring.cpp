@@ -1,4 +1,4 @@
-// FlowRing: the vectors of wavefront sweeps (see flow.hpp).
+// The storage of wavefront sweeps (see flow.hpp).
 #include <algorithm>
 
 #include "flow.hpp"
@@ -6,7 +6,8 @@
 namespace unapgpu {
 
 FlowRing::FlowRing(FlowRing&& o) noexcept
-    : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), err(o.err), polls(o.polls)
+    : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), halves(o.halves),
+      err(o.err), polls(o.polls)
 {
     o.err = nullptr;
 }
@@ -17,6 +18,7 @@ FlowRing& FlowRing::operator=(FlowRing&& o) noexcept
     stride = o.stride;
     half = o.half;
     sweeps = o.sweeps;
+    halves = o.halves;
     std::swap(err, o.err);
     polls = o.polls;
     return *this;
@@ -24,10 +26,10 @@ FlowRing& FlowRing::operator=(FlowRing&& o) noexcept
 
 FlowRing::~FlowRing() { pinned_block_free(err); }
 
-void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves)
+void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int nHalves)
 {
     // set last: an allocation that throws leaves the ring without vectors
-    sweeps = 0;
+    sweeps = halves = 0;
     const int per = std::max(1, std::min(sweepsPerHalf, kFlowMaxSweeps));
     stride = (n * elemBytes + 255) / 256 * 256;
     half = kFlowHeader + stride * (size_t)per;
@@ -36,14 +38,40 @@ void FlowRing::init(size_t n, size_t elemBytes, int sweepsPerHalf, int halves)
         err = static_cast<int*>(pinned_block_alloc(64));
         *err = 0;
     }
-    mem.alloc((size_t)halves * half);
+    mem.alloc((size_t)nHalves * half);
     sweeps = per;
+    halves = nHalves;
+}
+
+void FlowRing::ensure(size_t n, size_t elemBytes, int nSweeps, int most)
+{
+    if (nSweeps <= 0) return;
+    const int per = std::min(nSweeps, most), h = nSweeps > per ? 2 : 1;
+    if (sweeps < per || halves < h)
+        init(n, elemBytes, std::max(per, sweeps), std::max(h, halves));
 }
 
 int FlowRing::other(const void* p) const
 {
     const unsigned char* q = static_cast<const unsigned char*>(p);
-    return q >= mem.p && q < mem.p + half ? 1 : 0;
+    if (!(q >= mem.p && q < mem.p + half)) return 0;
+    if (halves < 2) throw std::logic_error("sweeps in place on a ring of one half");
+    return 1;
+}
+
+void DicFlow::init(const Level& L)
+{
+    rD.alloc((size_t)L.n);
+    f.alloc((size_t)L.nEntries);
+    part.alloc((size_t)std::max(L.tasks[0].n, 1));
+    ring.init((size_t)L.n, sizeof(double), 1, 1);
+}
+
+void DicFlow::keepFactor()
+{
+    ring.mem.release();
+    ring.sweeps = ring.halves = 0;
+    part.release();
 }
 
 void throw_ran_out()

@@ -204,7 +204,10 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
     UNAP_CK(cudaEventCreate(&ev0));
     UNAP_CK(cudaEventCreate(&ev1));
     UNAP_CK(cudaStreamSynchronize(s));
-    lv.back().dic.check();
+    if (nC > 0) {
+        lv.back().dic.check();
+        lv.back().dic.keepFactor();
+    }
 }
 
 MgSolver::~MgSolver()
@@ -270,8 +273,7 @@ void MgSolver::smooth(int slot, int k, double* xk, const double* bk, int nSweeps
     // of them), each following the one before at a wavefront's distance
     Lv& K = lv[(size_t)k];
     const Level& L = *K.L;
-    const int per = std::min(nSweeps, kFlowMaxSweeps);
-    if (K.sweeps.sweeps < per) K.sweeps.init((size_t)K.n, sizeof(double), per);
+    K.sweeps.ensure((size_t)K.n, sizeof(double), nSweeps, kFlowMaxSweeps);
     flow_gs<double>(ex, L, rows64(L), K.sweeps, xk, bk, nSweeps, false, false, nullptr, xk,
                     Gate{});
 }
