@@ -198,9 +198,11 @@ int unap_cuda_matrix_info(long int handle, int* nWavefronts, long long* nEntries
 int unap_cuda_matrix_layout(long int handle, int* nWavefronts, int* perm, int* waveStart);
 /* Matrices (and AMG levels) of at least minCells cells build their device
  * structure (internal order, SELL-32 layout, values) with kernels instead
- * of host loops; minCells < 0 builds every one on the host.  Both give the
- * same structure bit for bit.  Default 8192; the previous value is
- * returned through the (nullable) pointer.  No reference counterpart. */
+ * of host loops; minCells < 0 builds every one on the host.  Coarse levels of
+ * a hierarchy and COO/CSR input of at least 2 minCells entries do so from a
+ * quarter of minCells on, levels only where the level above shows that it
+ * pays.  Both give the same structure bit for bit.  Default 32768; the previous
+ * value is returned through the (nullable) pointer.  No reference counterpart. */
 int unap_cuda_set_device_setup(long long minCells, long long* oldMinCells);
 
 /* Kernels on device vectors in the caller's cell order (FP64). */

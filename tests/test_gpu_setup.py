@@ -8,6 +8,8 @@ build declines go to the host with the same result (a cell with more lower
 neighbours than it takes, a chain with more wavefronts, more connected
 components than it follows).
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -303,3 +305,33 @@ def test_device_agglomeration_asymmetric_mg_same_bits(cuda):
     assert out[0][0] == out[1][0]
     assert out[0][1] == out[1][1]
     assert np.array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("n", [8192, 24000])
+def test_setup_of_long_chains_stays_on_the_host(cuda, n):
+    """A chain has a BFS level, a wavefront and a dependent turn per cell; below
+    the limit its matrix and hierarchy are made by host loops.  By kernels
+    they took 72 and 89 ms at 24,000 cells, host loops 1 and 6 ms."""
+    s = chain(n)
+
+    def milliseconds(make):
+        best = 1e9
+        for _ in range(5):
+            t0 = time.perf_counter()
+            make()
+            best = min(best, time.perf_counter() - t0)
+        return 1e3 * best
+
+    A = capi.DeviceMatrix(s)
+    made = {}
+    for mc in (None, -1):
+        old = capi.set_device_setup(-1) if mc is not None else None
+        try:
+            made[mc] = (milliseconds(lambda: capi.DeviceMatrix(s).close()),
+                        milliseconds(lambda: capi.DeviceAmg(A, n_coarsest=200).close()))
+        finally:
+            if mc is not None:
+                capi.set_device_setup(old)
+    A.close()
+    for here, host in zip(made[None], made[-1]):
+        assert here <= 2.0 * host + 3.0, made

@@ -45,3 +45,7 @@ def test_growing_ring_keeps_its_error_word(tmp_path):
 
 def test_sweeps_keep_what_their_launches_write(tmp_path):
     assert "ok" in run_program("ring_storage", tmp_path, units=["flow_ring.cpp"])
+
+
+def test_where_setup_runs_by_kernels(tmp_path):
+    assert "ok" in run_program("setup_limits", tmp_path)

@@ -425,7 +425,7 @@ void transfer_maps(const Level& F, const Level& C, const CoarseHost& c,
     const int n = F.n, nc = C.n;
     const std::vector<int>& agg = c.restrictAddr;
     const long long minCells = device_setup_min_cells();
-    if (minCells < 0 || n < minCells || c.largest > kMaxList) {
+    if (minCells < 0 || n < minCells / 4 || c.largest > kMaxList) {
         std::vector<int> refStart((size_t)nc + 1, 0);
         for (int i = 0; i < n; ++i) refStart[(size_t)agg[(size_t)i] + 1]++;
         for (int k = 0; k < nc; ++k) refStart[(size_t)k + 1] += refStart[(size_t)k];
@@ -472,9 +472,11 @@ void transfer_maps(const Level& F, const Level& C, const CoarseHost& c,
 // One level: returns false (nothing produced) when the device form leaves
 // the level to the host (a list longer than kMaxList, or more than
 // kMaxRounds rounds).  On success `out` and `cw` are what pairwise_pass,
-// coarse_addressing, coarse_coefficients and the weight restriction give.
+// coarse_addressing, coarse_coefficients and the weight restriction give;
+// rounds: the matching rounds it took.
 bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, CoarseHost& out,
-                              std::vector<double>& cw, int& nCoarse, cudaStream_t s)
+                              std::vector<double>& cw, int& nCoarse, int& rounds,
+                              cudaStream_t s)
 {
     const int n = A.n, nf = A.nf;
     if (n <= 0) return false;
@@ -524,6 +526,7 @@ bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, Co
             k_turn<<<grid, kThreads, 0, s>>>(start.p, nbr.p, wt.p, n, mp.p, lead.p, done.p,
                                              former.p, round < kMaxRounds, pending.p + k);
         }
+        rounds = round + m;
         if (read_int(pending.p + m - 1, s) == 0) break;
         if (round >= kMaxRounds) return false;
     }

@@ -224,15 +224,15 @@ std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, std::vector<doub
     if (maxLevels <= 0) maxLevels = 50;
     if (nCoarsest <= 0) nCoarsest = 50;
     std::vector<CoarseHost> levels;
+    int rounds = -1;  // of the level above, if it was matched by kernels
     while ((int)levels.size() < maxLevels - 1) {
         const HostLdu& fm = levels.empty() ? fine : levels.back().A;
         if (stopRule == 1 && fm.n <= nCoarsest) break;
-        const long long minCells = device_setup_min_cells();
-        if (minCells >= 0 && fm.n >= minCells) {
+        if (setup_level_on_device(device_setup_min_cells(), fm.n, rounds, kCellsPerRound)) {
             CoarseHost c;
             std::vector<double> cw;
             int nc = -1;
-            if (agglomerate_level_device(fm, w, c, cw, nc, s)) {
+            if (agglomerate_level_device(fm, w, c, cw, nc, rounds, s)) {
                 bool keep = stopRule == 1 ? (nc < fm.n) : (nc >= nCoarsest);
                 if (!keep) break;
                 w.swap(cw);
@@ -240,6 +240,7 @@ std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, std::vector<doub
                 continue;
             }
         }
+        rounds = -1;
         int nc = -1;
         std::vector<int> map = pairwise_pass(fm, w, nc);
         bool keep = stopRule == 1 ? (nc < fm.n) : (nc >= nCoarsest);

@@ -76,7 +76,7 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
             key[(size_t)C] = std::min(key[(size_t)C], F.locRank[(size_t)i]);
         }
         // Chebyshev levels are never swept: locality order, no wavefronts
-        lv[(size_t)k].own = build_level(c.A, &key, k == L, s, !isCheby(k));
+        lv[(size_t)k].own = build_level(c.A, &key, k == L, s, !isCheby(k), &F);
         lv[(size_t)k].L = lv[(size_t)k].own.get();
         lv[(size_t)k].n = nC;
         transfer_maps(F, *lv[(size_t)k].L, c, lv[(size_t)k].childStart,

@@ -25,20 +25,21 @@ void coarse_addressing(const HostLdu& fine, const std::vector<int>& map, int nCo
 void coarse_coefficients(const HostLdu& fine, CoarseHost& c);
 // stopRule 0: the reference's rule (keep a level while it has >= nCoarsest
 // cells); stopRule 1: agglomerate until the coarsest has <= nCoarsest cells.
-// Levels of at least device_setup_min_cells() cells are agglomerated by
-// kernels on stream s (aggl_dev.cu), with the same result.
+// Levels for which setup_level_on_device says so are agglomerated by kernels on
+// stream s (aggl_dev.cu), with the same result.
 std::vector<CoarseHost> agglomerate_levels(const HostLdu& fine, std::vector<double> weights,
                                            int nCoarsest, int maxLevels, int stopRule,
                                            cudaStream_t s = 0);
 bool agglomerate_level_device(const HostLdu& A, const std::vector<double>& w, CoarseHost& out,
-                              std::vector<double>& cw, int& nCoarse, cudaStream_t s);
+                              std::vector<double>& cw, int& nCoarse, int& rounds,
+                              cudaStream_t s);
 std::vector<double> mg_face_weights(const HostLdu& A);
 // Transfers between a level and the one its cells aggregate into (c: that
 // level), in internal rows: the children of coarse row r are
 // child[childStart[r] ..], ascending finer cell (the summation order of
 // restrictField), and cmap[i] is the coarse row of finer row i.  Made by
-// kernels on levels of at least device_setup_min_cells() cells without a
-// large aggregate (c.largest); c has to live until the stream is synchronized.
+// kernels on levels of at least a quarter of device_setup_min_cells() cells
+// without a large aggregate (c.largest); c has to live until the stream is synchronized.
 void transfer_maps(const Level& F, const Level& C, const CoarseHost& c,
                    DevArray<int>& childStart, DevArray<int>& child, DevArray<int>& cmap,
                    cudaStream_t s);

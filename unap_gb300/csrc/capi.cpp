@@ -233,8 +233,7 @@ void coo2ldumatrixcreat_(long int* APtrPtr, const double* dataPtr, const int* ro
 {
     int rc = guarded([&] {
         auto m = std::make_unique<MatHandle>();
-        const long long minCells = device_setup_min_cells();
-        if (!(minCells >= 0 && *nCells >= minCells &&
+        if (!(setup_input_on_device(device_setup_min_cells(), *nCells, *size) &&
               coo_to_ldu_device(dataPtr, rowsPtr, columnPtr, *nCells, *size, *symm != 0, false,
                                 0, m->pending))) {
             std::vector<int> r((size_t)*size), c((size_t)*size);
@@ -260,8 +259,7 @@ void csr2ldumatrixcreat_(long int* APtrPtr, const double* dataPtr, const int* co
         // csr2ldu (coo2ldu.cpp:116-148) expands the row pointer and calls
         // coo2ldu without re-sorting; indices are used as given (0-based)
         auto m = std::make_unique<MatHandle>();
-        const long long minCells = device_setup_min_cells();
-        if (!(minCells >= 0 && *nCells >= minCells &&
+        if (!(setup_input_on_device(device_setup_min_cells(), *nCells, *size) &&
               coo_to_ldu_device(dataPtr, compRowsPtr, columnPtr, *nCells, *size, *symm != 0, true,
                                 0, m->pending))) {
             if (compRowsPtr[0] != 0 || compRowsPtr[*nCells] != *size)

@@ -83,11 +83,12 @@ std::vector<int> bfs_rank(int n, const std::vector<int>& loStart, const std::vec
 }  // namespace
 
 std::unique_ptr<Level> build_level(const HostLdu& A, const std::vector<int>* key,
-                                   bool identityOrder, cudaStream_t s, bool wavefronts)
+                                   bool identityOrder, cudaStream_t s, bool wavefronts,
+                                   const Level* finer)
 {
-    const long long minCells = device_setup_min_cells();
-    if (!identityOrder && A.oriented && A.ownerSorted && minCells >= 0 && A.n > 0 &&
-        A.n >= minCells) {
+    const int links = !finer ? -1 : wavefronts ? finer->nWave : 0;
+    if (!identityOrder && A.oriented && A.ownerSorted && A.n > 0 &&
+        setup_level_on_device(device_setup_min_cells(), A.n, links, kCellsPerWavefront)) {
         if (auto D = build_level_device(A, key, s, wavefronts)) {
             D->version = next_version();
             flow_tasks(*D, s);

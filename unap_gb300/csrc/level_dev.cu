@@ -707,9 +707,7 @@ struct Readback {
     }
 };
 
-// The hierarchy of a 508,200-cell log-normal system took 50.7 / 44.0 / 43.2 /
-// 44.4 / 48.7 ms to set up with this at 32768 / 16384 / 8192 / 4096 / 1024.
-std::atomic<long long> g_deviceMinCells{8192};
+std::atomic<long long> g_deviceMinCells{kDeviceSetupCells};
 
 }  // namespace
 

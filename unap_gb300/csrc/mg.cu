@@ -139,7 +139,7 @@ MgSolver::MgSolver(Matrix& A_, const std::vector<double>& weights, const MgParam
             int C = c.restrictAddr[(size_t)i];
             key[(size_t)C] = std::min(key[(size_t)C], F.iperm[(size_t)i]);
         }
-        lv[(size_t)k].own = build_level(c.A, &key, false, s);
+        lv[(size_t)k].own = build_level(c.A, &key, false, s, true, &F);
         lv[(size_t)k].L = lv[(size_t)k].own.get();
         lv[(size_t)k].n = c.A.n;
         const int nc = c.A.n;

@@ -356,17 +356,47 @@ void update_level_values(Level& L, const HostLdu& A, cudaStream_t s);
 // keeps the reference numbering (used for the dense coarsest level).
 // wavefronts == false puts every row in one range in locality order (for
 // levels that are never swept: SpMV-shaped smoothing only); such a level is
-// marked not sweepable.
+// marked not sweepable.  finer: the level above, for a level of a hierarchy.
 std::unique_ptr<Level> build_level(const HostLdu& A, const std::vector<int>* key,
-                                   bool identityOrder, cudaStream_t s, bool wavefronts = true);
+                                   bool identityOrder, cudaStream_t s, bool wavefronts = true,
+                                   const Level* finer = nullptr);
 void make_fp32(Level& L, cudaStream_t s);
 // The same Level built by kernels on stream s (level_dev.cu); nullptr when
 // the matrix has a shape the device build leaves to the host.
 std::unique_ptr<Level> build_level_device(const HostLdu& A, const std::vector<int>* key,
                                           cudaStream_t s, bool wavefronts = true);
-// Levels of at least this many cells are built on the device (< 0: none).
+// Setup by kernels instead of host loops: matrices of at least this many cells
+// (< 0: none), and what the rules below say.
 long long set_device_setup_min_cells(long long minCells);
 long long device_setup_min_cells();
+// Default.  A single matrix's device build has a fixed price of about 1 ms, a
+// read-back per wavefront and a BFS level after another.  DeviceMatrix, ms, host
+// loops against kernels: Laplacians in natural order 0.8 / 2.6 at 8,192 cells,
+// 1.2 / 3.3 at 16,000, 2.5 / 4.1 at 32,000, 4.1 / 5.0 at 48,000, 6.4 / 5.9 at
+// 80,000; permuted 1.0 / 1.6, 1.8 / 1.8, 4.0 / 2.2, 6.7 / 2.5; a chain of 8,192
+// cells 0.6 / 72.
+constexpr long long kDeviceSetupCells = 32768;
+// Smaller work that pays from a quarter of the limit on:
+// a hierarchy's levels below the finest, whose order is given.  What a step of a
+// level takes on the device is a chain of `links` (matching rounds of 15 us,
+// read-backs of 27 us for the wavefronts of a level that has them), about as
+// many as the level above took (-1: unknown, or left to the host), against 0.1 us
+// a cell in the host loops.  cellsPerLink: cells that pay for a link.
+inline bool setup_level_on_device(long long minCells, long long n, long long links,
+                                  int cellsPerLink)
+{
+    if (minCells < 0) return false;
+    if (n >= minCells) return true;
+    return n >= minCells / 4 && links >= 0 && links * cellsPerLink <= n;
+}
+constexpr int kCellsPerRound = 256, kCellsPerWavefront = 512;
+// ... and COO/CSR input of many entries (8,192 / 11,000 / 32,000 cells with 7
+// entries: 0.39 / 0.50 / 1.46 ms on the host, 0.43 / 0.44 / 0.50 by kernels)
+inline bool setup_input_on_device(long long minCells, long long n, long long entries)
+{
+    if (minCells < 0) return false;
+    return n >= minCells || (n >= minCells / 4 && entries >= 2 * minCells);
+}
 // out[i] = in[0] + ... + in[i-1] for i <= n (n + 1 outputs), on stream s
 void device_exclusive_scan(const int* in, int* out, long long n, cudaStream_t s);
 // COO (1-based rows and columns) or CSR (0-based row pointer and columns)
