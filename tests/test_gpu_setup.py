@@ -335,3 +335,42 @@ def test_setup_of_long_chains_stays_on_the_host(cuda, n):
     A.close()
     for here, host in zip(made[None], made[-1]):
         assert here <= 2.0 * host + 3.0, made
+
+
+def layered(widths, seed):
+    """Layers of cells, every cell joined to one to three cells of the layer
+    before (several claim it), numbered at random: a BFS from any cell of the
+    first layer has the layers as its frontiers."""
+    rng = np.random.default_rng(seed)
+    first = np.concatenate([[0], np.cumsum(widths)])
+    pairs = []
+    for k in range(1, len(widths)):
+        cells = np.arange(first[k], first[k + 1])
+        for j in range(3):
+            some = cells if j == 0 else cells[rng.random(cells.size) < 0.4]
+            pairs.append(np.stack([rng.integers(first[k - 1], first[k], some.size), some]))
+    n = int(first[-1])
+    # the first layer's cell is cell 0, where the order starts
+    name = np.concatenate([[0], 1 + rng.permutation(n - 1)])
+    a, b = np.sort(name[np.concatenate(pairs, axis=1)], axis=0)
+    key = np.unique(a.astype(np.int64) * n + b)
+    l, u = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    upper = -rng.random(l.size) - 0.1
+    diag = W._fast_row_abs_sum(n, l, u, upper, upper) + 1.0
+    return W.LduSystem(n, l, u, None, diag, upper, rng.standard_normal(n), name="layered")
+
+
+@pytest.mark.parametrize("widths", [
+    [1, 30, 900, 32768, 60000, 50000, 9000, 4],          # out of one cluster's reach and back
+    [1, 30, 900, 16384, 32769, 16384, 16385, 32768, 1],  # each side of both limits
+])
+def test_bfs_order_of_wide_frontiers(cuda, widths):
+    """Frontiers above 32,768 cells leave the one-cluster kernel for the whole
+    GPU, those of up to 16,384 return to it: the host's order either way."""
+    s = layered(widths, 11)
+    D, H = built(s, 1), built(s, -1)
+    pd, wd = D.layout()
+    ph, wh = H.layout()
+    assert np.array_equal(pd, ph) and np.array_equal(wd, wh)
+    D.close()
+    H.close()
