@@ -186,6 +186,13 @@ def barrier(dist, device=None):
             dist.barrier()
 
 
+def spmv64_kernel(n: int, nf: int) -> str:
+    """The kernel of an FP64 product (row_stream.hpp: from 2^19 rows of up to
+    8.5 entries on average)."""
+    return ("row_stream_kernel" if n >= 1 << 19 and 2 * nf <= 8.5 * n else "spmv_kernel") + \
+        "<double>"
+
+
 def spmv64_bytes(n: int, nf: int, symm: bool = True) -> int:
     """Algorithmic bytes of an FP64 LDU SpMV: diag, x, y (8 B each) per cell;
     per face one value (two if asymmetric) and two int32 addresses."""
@@ -370,11 +377,10 @@ def config_block(name: str, steps: int, warmup: int, cpu: bool):
         out["whole_solve_gbs"] = st[-1]["algorithmicBytes"] / out["gpu_s"] / 1e9
     prof = A.profile(reps=10)
     symm = s.symm
-    k = {"spmv": ("spmv_kernel<double>", spmv64_bytes(s.n, s.nf, symm))}
+    k = {"spmv": (spmv64_kernel(s.n, s.nf), spmv64_bytes(s.n, s.nf, symm))}
     if cfg["kind"] == "krylov":
         key = "dic_apply" if cfg["precond"] == 2 else "dilu_apply"
-        k[key] = (("dic" if cfg["precond"] == 2 else "dilu") + "_fwd/bwd_kernel",
-                  40 * s.n + (32 if symm else 40) * s.nf)
+        k[key] = ("flow_dic_kernel", 40 * s.n + (32 if symm else 40) * s.nf)
     out["kernels"] = {key: {"kernel": nm, "ms": prof[key], "algorithmic_bytes": by,
                             "achieved_gbs": by / (prof[key] * 1e-3) / 1e9,
                             "frac": by / (prof[key] * 1e-3) / 1e9 / peak}
@@ -773,8 +779,10 @@ def smoother_roofline(G, info, mixed: bool, peak: float, deg: int, sweeps: int):
     (unap_cuda_amg_profile_smoother), and the kernel family with the largest
     device time per V-cycle: Chebyshev steps (2 deg - 1 launches per level
     and V-cycle: the first pre-smoothing step runs inside the restriction)
-    or Gauss-Seidel sweeps (`sweeps` = nPre + nPost per level)."""
+    or Gauss-Seidel sweeps (`sweeps` = nPre + nPost per level; one launch a
+    sweep, or one per wavefront on large FP32 levels)."""
     fam = {"cheb": {"ms": 0.0, "bytes": 0.0, "levels": []},
+           "gs_flow": {"ms": 0.0, "bytes": 0.0, "levels": []},
            "gs_fine": {"ms": 0.0, "bytes": 0.0, "levels": []},
            "gs_coarse": {"ms": 0.0, "bytes": 0.0, "levels": []}}
     lam = G.eigenvalues()
@@ -783,7 +791,7 @@ def smoother_roofline(G, info, mixed: bool, peak: float, deg: int, sweeps: int):
         ms, by, launches = G.profile_smoother(k, reps=10)
         cheb = lam[k] > 0
         reps = (2 * deg - 1) if cheb else sweeps
-        f = "cheb" if cheb else ("gs_fine" if k == 0 else "gs_coarse")
+        f = "cheb" if cheb else "gs_flow" if launches == 1 else "gs_fine" if k == 0 else "gs_coarse"
         fam[f]["ms"] += reps * ms
         fam[f]["bytes"] += reps * by
         fam[f]["levels"].append(k)
@@ -791,6 +799,7 @@ def smoother_roofline(G, info, mixed: bool, peak: float, deg: int, sweeps: int):
                           "ms": ms, "launches": launches, "algorithmic_bytes": by,
                           "achieved_gbs": by / (ms * 1e-3) / 1e9})
     names = {"cheb": "cheb_step_kernel<%s>" % ("float" if mixed else "double"),
+             "gs_flow": "flow_gs_kernel<%s>" % ("float" if mixed else "double"),
              "gs_fine": "gs_kernel<%s>" % ("float" if mixed else "double"),
              "gs_coarse": "gs_packed_kernel<%s>" % ("float" if mixed else "double")}
     groups = {}
@@ -941,7 +950,7 @@ def main():
                                                kw.get("n_pre", 2) + kw.get("n_post", 2))
     vprof = G.profile_vcycle(reps=10)
     mprof = A.profile(reps=10)
-    spmv = {"kernel": "spmv_kernel<double>", "ms": mprof["spmv"],
+    spmv = {"kernel": spmv64_kernel(s.n, s.nf), "ms": mprof["spmv"],
             "achieved": spmv64_bytes(s.n, s.nf) / (mprof["spmv"] * 1e-3) / 1e9}
     spmv["frac"] = spmv["achieved"] / peak
     solve_bytes = stats[-1].get("algorithmicBytes", 0.0)
