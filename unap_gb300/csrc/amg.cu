@@ -337,10 +337,10 @@ void AmgHierarchy::check() const
     if (out) throw_ran_out();
 }
 
-void AmgHierarchy::setWaitPolls(int polls)
+void AmgHierarchy::setWaitSpent(int polls)
 {
-    for (auto& l : lv) l.sweeps.polls = polls;
-    tail32.polls = tail64.polls = polls;
+    for (auto& l : lv) l.sweeps.spent = polls;
+    tail32.spent = tail64.spent = polls;
 }
 
 int AmgHierarchy::tailFirst(size_t elemBytes) const

@@ -133,8 +133,8 @@ public:
     std::vector<double> eigenvalues() const;
     // throws when a wait of a sweep ran out (after synchronizing)
     void check() const;
-    // polls that the waits of later V-cycles take (WaitBound)
-    void setWaitPolls(int polls);
+    // polls that the waits of later V-cycles count as spent (WaitBound)
+    void setWaitSpent(int polls);
 
     // Level k's sweeps are one launch each (flow_gs) in FP64 and on FP32
     // levels of up to kFlowRows32 rows; above that an FP32 wavefront alone

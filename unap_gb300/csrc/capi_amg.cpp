@@ -318,10 +318,10 @@ int unap_cuda_selftest_wait_timeout(long int handle, int what, int* timedOut)
         if (what >= 2) flow_dic_factor(ex, L, !L.symm, D);
         UNAP_CK(cudaStreamSynchronize(ex.s));
         D.check();
-        D.ring.polls = 1;
+        D.ring.spent = kWaitPolls - 1;
         if (what == 0) {
             ring.init((size_t)n, sizeof(double), 2);
-            ring.polls = 1;
+            ring.spent = kWaitPolls - 1;
             flow_gs<double>(ex, L, rows64(L), ring, x.p, b.p, 2, false, false, nullptr, nullptr,
                             Gate{});
         } else if (what == 1) {
@@ -370,9 +370,9 @@ int unap_cuda_selftest_vcycle_timeout(long int amg)
         k_fill<double>(ex, n, r.p, 1.0);
         struct Restore {
             AmgHierarchy& H;
-            ~Restore() { H.setWaitPolls(kWaitPolls); }
+            ~Restore() { H.setWaitSpent(0); }
         } restore{*h->H};
-        h->H->setWaitPolls(1);
+        h->H->setWaitSpent(kWaitPolls - 1);
         h->H->vcycle(ex, r.p, z.p, Gate{});
         UNAP_CK(cudaGetLastError());
         UNAP_CK(cudaStreamSynchronize(A.stream));

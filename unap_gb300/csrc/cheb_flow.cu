@@ -83,10 +83,10 @@ __device__ __forceinline__ int take(unsigned* counters)
 
 // one value that another row of this launch writes; all lanes call it
 template <class T>
-__device__ __forceinline__ T wait_one(const T* p, bool on, WaitBound b)
+__device__ __forceinline__ T wait_one(const T* p, bool on, int* err)
 {
     T v[1] = {T(0)};
-    wait_values<T, 1>(on ? 1u : 0u, [&](int) { return p; }, v, b);
+    wait_values<T, 1>(on ? 1u : 0u, [&](int) { return p; }, v, err);
     return v[0];
 }
 
@@ -132,7 +132,7 @@ __device__ __forceinline__ void row_task(const Args<T>& a, const Stage<T>& S, in
         all[K] = T(0);
         if (j0 == 0 && mine) need |= 1u << K;
         wait_values<T, K + 1>(
-            need, [&](int k) { return k == K ? own : S.a + c[k]; }, all, a.bound);
+            need, [&](int k) { return k == K ? own : S.a + c[k]; }, all, a.bound.err);
 #pragma unroll
         for (int k = 0; k < K; ++k) pw[row * P + k * G + g] = v[k] * all[k];
         if (j0 == 0) {
@@ -218,7 +218,7 @@ __device__ __forceinline__ void restrict_task(const Args<T>& a, const Stage<T>& 
             if (has) need |= 1u << k;
         }
         if (S.pollA) {
-            wait_values<T, 4>(need, [&](int k) { return S.a + c[k]; }, v, a.bound);
+            wait_values<T, 4>(need, [&](int k) { return S.a + c[k]; }, v, a.bound.err);
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kThreads) cheb_flow_kernel(const __grid_consta
             const int c = on ? ldg(S.i0 + r) : 0;
             if (S.wait) wait_near(S.near + (int)((long long)r0 * S.wait / S.n), a.bound);
             T v[2];
-            wait_values<T, 2>(on ? 3u : 0u, [&](int k) { return k ? S.a + c : S.b + r; }, v, a.bound);
+            wait_values<T, 2>(on ? 3u : 0u, [&](int k) { return k ? S.a + c : S.b + r; }, v, a.bound.err);
             if (on) st_flow(S.x + r, v[0] + v[1]);
         } else if (S.type == CF_CHUNK) {
             // a column chunk of 32 rows of x = Minv b, summed in ascending
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kThreads) cheb_flow_kernel(const __grid_consta
             if (S.wait) wait_near(S.near + (int)((long long)j0 * S.wait / S.n), a.bound);
             __syncwarp();
             for (int j = lane; j < kDenseChunk; j += 32) {
-                const T b = wait_one<T>(S.a + j0 + j, j < m, a.bound);
+                const T b = wait_one<T>(S.a + j0 + j, j < m, a.bound.err);
                 sb[warp][j] = (double)b;
             }
             __syncwarp();
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kThreads) cheb_flow_kernel(const __grid_consta
                 double v[4];
                 const unsigned need = on ? (1u << min(4, nq - q0)) - 1u : 0u;
                 wait_values<double, 4>(
-                    need, [&](int k) { return a.part + (size_t)(q0 + k) * a.nc + r; }, v, a.bound);
+                    need, [&](int k) { return a.part + (size_t)(q0 + k) * a.nc + r; }, v, a.bound.err);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     if (q0 + k < nq) t_ += v[k];
@@ -492,7 +492,7 @@ void ChebFlow<T>::launch(const Exec& ex, Gate g) const
     a.part = part;
     a.nc = nc;
     a.counter = reinterpret_cast<unsigned*>(arena.p);
-    a.bound = wait_bound(err, polls);
+    a.bound = {err, spent};
     UNAP_CK(cudaMemsetAsync(arena.p, 0xff, arena.n, ex.s));
     if (!capturing()) count_launches(1);
     cheb_flow_kernel<T><<<grid, kThreads, 0, ex.s>>>(a, g);

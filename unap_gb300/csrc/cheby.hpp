@@ -114,7 +114,7 @@ struct ChebFlow {
     const double* M = nullptr;
     double* part = nullptr;
     int* err = nullptr;              // pinned: set when a wait ran out
-    int polls = kWaitPolls;  // of its waits
+    int spent = 0;                   // of its waits' polls (WaitBound)
     ChebFlow() = default;
     ChebFlow(const ChebFlow&) = delete;
     ChebFlow& operator=(const ChebFlow&) = delete;

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kFlowThreads)
                         xv[k] = *at(k);
                 }
             }
-            wait_values<T, K>(need, at, xv, a.bound);
+            wait_values<T, K>(need, at, xv, a.bound.err);
             if (G == 1) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) xv[k] = v[k] * xv[k];
@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(kFlowThreads)
                 if (has) need |= 1u << k;
             }
             if (j0 == 0 && wait >= 0) wait_near(d + wait, bound);
-            wait_values<double, CK>(need, [&](int k) { return (const double*)d + c[k]; }, xv, bound);
+            wait_values<double, CK>(need, [&](int k) { return (const double*)d + c[k]; }, xv,
+                                    bound.err);
 #pragma unroll
             for (int k = 0; k < CK; ++k)
                 if (j0 + k < most) xv[k] = v[k] / xv[k];
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_dic_kernel(const __grid_con
             if (j0 == 0 && wait >= 0) wait_near(out + wait, a.bound);
             wait_values<double, CK + 1>(
                 need, [&](int k) { return k == CK ? a.wf + r : (const double*)out + c[k]; }, xv,
-                a.bound);
+                a.bound.err);
             if (bwd && j0 == 0) acc = xv[CK];
 #pragma unroll
             for (int k = 0; k < CK; ++k) {
@@ -575,7 +576,8 @@ void small_sweeps(SmallSystem& S, const Level& L, const DicFlow& D)
     S.task = L.tasks[0].task.p;
     S.near = L.tasks[0].near.p;
     S.nTasks = L.tasks[0].n;
-    S.bound = D.ring.bound();
+    S.err = D.ring.err;
+    S.spent = D.ring.spent;
 }
 
 }  // namespace unapgpu

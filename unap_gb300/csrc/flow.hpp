@@ -25,7 +25,7 @@ struct FlowRing {
     int sweeps = 0;      // vectors of one half
     int halves = 0;
     int* err = nullptr;  // pinned: set by a launch whose wait ran out
-    int polls = kWaitPolls;  // of its waits
+    int spent = 0;       // of its waits' polls (WaitBound)
     FlowRing() = default;
     FlowRing(const FlowRing&) = delete;
     FlowRing& operator=(const FlowRing&) = delete;
@@ -38,7 +38,7 @@ struct FlowRing {
     // reads the one before
     void ensure(size_t n, size_t elemBytes, int nSweeps, int most);
     size_t bytes() const { return mem.bytes(); }
-    WaitBound bound() const { return wait_bound(err, polls); }
+    WaitBound bound() const { return {err, spent}; }
     // the half (0 or 1) that does not hold p; throws if the ring has one and
     // p is in it
     int other(const void* p) const;
@@ -56,8 +56,10 @@ struct FlowRing {
 // from `in`; xIsZero: in is zero (forward, the first sweep then reads only
 // its lower side, in may be null).  Returns the result's address: `last`
 // where it is given (n elements, not `in`), else one of the ring's vectors.
-// copy (optional, may be `in`): the result is written there too, row r at
-// copyAt[r] if that is given (a launch that put the result into the caller's
+// copy (optional, may be `in`: an entry is overwritten only by a row whose value
+// depends, over its neighbours' values, on every row that read the old entry; a
+// plain store cannot pass the loads that its value is made of): the result is
+// written there too, row r at copyAt[r] if that is given (a launch that put the result into the caller's
 // order took 16 of 278 us for two sweeps at 128^3).
 template <class T>
 T* flow_gs(const Exec& ex, const Level& L, const Rows<T>& A, const FlowRing& ring, const T* in,

@@ -7,7 +7,7 @@ namespace unapgpu {
 
 FlowRing::FlowRing(FlowRing&& o) noexcept
     : mem(std::move(o.mem)), stride(o.stride), half(o.half), sweeps(o.sweeps), halves(o.halves),
-      err(o.err), polls(o.polls)
+      err(o.err), spent(o.spent)
 {
     o.err = nullptr;
 }
@@ -20,7 +20,7 @@ FlowRing& FlowRing::operator=(FlowRing&& o) noexcept
     sweeps = o.sweeps;
     halves = o.halves;
     std::swap(err, o.err);
-    polls = o.polls;
+    spent = o.spent;
     return *this;
 }
 

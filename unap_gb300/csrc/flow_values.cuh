@@ -34,11 +34,11 @@ __device__ __forceinline__ void st_flow(double* p, double v)
 }
 
 // One more poll of a wait: true when the wait has to be given up.
-__device__ __forceinline__ bool give_up(int& spins, WaitBound b)
+__device__ __forceinline__ bool give_up(int& spins, int* err)
 {
-    if ((++spins & b.mask) == 0) {
-        if (spins >= b.polls) *(volatile int*)b.err = 1;
-        if (*(volatile int*)b.err) return true;
+    if ((++spins & 0xfff) == 0) {
+        if (spins >= kWaitPolls) *(volatile int*)err = 1;
+        if (*(volatile int*)err) return true;
     }
     return false;
 }
@@ -46,7 +46,7 @@ __device__ __forceinline__ bool give_up(int& spins, WaitBound b)
 // Loads at(k) for the entries in `need` (one bit each) until every value is
 // there; all lanes of the warp call it.
 template <class T, int CK, class At>
-__device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], WaitBound b)
+__device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], int* err)
 {
     int spins = 0;
     for (;;) {
@@ -57,7 +57,7 @@ __device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], 
         for (int k = 0; k < CK; ++k)
             if ((need >> k & 1u) && !absent(v[k])) need &= ~(1u << k);
         if (!__any_sync(0xffffffffu, need != 0)) return;
-        if (give_up(spins, b)) return;
+        if (give_up(spins, err)) return;
     }
 }
 
@@ -67,10 +67,10 @@ __device__ __forceinline__ void wait_values(unsigned need, At&& at, T (&v)[CK], 
 template <class T>
 __device__ __forceinline__ void wait_near(const T* p, WaitBound b)
 {
-    int spins = 0;
+    int spins = b.spent;
     while (absent(ld_flow(p))) {
         __nanosleep(64);
-        if (give_up(spins, b)) return;
+        if (give_up(spins, b.err)) return;
     }
 }
 

@@ -266,10 +266,10 @@ __device__ __noinline__ void cluster_sweeps(const SmallSystem& S, const double* 
             }
             xv[CK] = 0.0;
             if (bwd && on && j0 == 0) need |= 1u << CK;
-            if (j0 == 0 && wait >= 0) wait_near(out + wait, S.bound);
+            if (j0 == 0 && wait >= 0) wait_near(out + wait, WaitBound{S.err, S.spent});
             wait_values<double, CK + 1>(
                 need, [&](int k) { return k == CK ? wf + i : (const double*)out + c[k]; }, xv,
-                S.bound);
+                S.err);
             if (bwd && j0 == 0) acc = xv[CK];
 #pragma unroll
             for (int k = 0; k < CK; ++k) {

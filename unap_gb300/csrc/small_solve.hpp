@@ -30,7 +30,8 @@ struct SmallSystem {
     const int4* task;           // the level's sweep tasks (SweepTasks, a lane a row)
     const int2* near;
     int nTasks;
-    WaitBound bound;            // of the sweeps' waits
+    int spent;                  // WaitBound of the sweeps' waits
+    int* err;
     int method;                 // 0 PCG, 1 PBiCGStab
     int precond;                // 0 none, 1 Diag, 2 DIC, 3 DILU
     double tol, relTol;

@@ -269,15 +269,16 @@ struct HostLdu {
     void validate();
 };
 
-// Bound of a launch's waits for values that other warps write: after `polls`
+// Bound of a launch's waits for values that other warps write: after kWaitPolls
 // polls (0.3 us or more each), or once *err is set, a wait goes on with what it
 // has; the one that ran out sets *err (pinned host memory), which the host turns
-// into an error once the launch is done.
+// into an error once the launch is done.  A launch may count some polls as spent
+// when a row's first wait starts, to see it run out (in every wait, or with the
+// bound itself as an argument, that cost 0.7 % of an MG solve of 97,812 cells).
 constexpr int kWaitPolls = 1 << 23;
 struct WaitBound {
     int* err;
-    int polls;  // a power of two
-    int mask;   // both are looked at every mask + 1 polls
+    int spent;
 };
 // Whether a launch that used the word set it; the word is cleared.  A call over
 // several words reads them all before it throws, or those after the first one
@@ -288,10 +289,6 @@ inline bool wait_ran_out(int* err)
     if (!e || !*e) return false;
     *e = 0;
     return true;
-}
-inline WaitBound wait_bound(int* err, int polls)
-{
-    return {err, polls, polls < 4096 ? polls - 1 : 4095};
 }
 
 // A row's entry counts in one word: all entries in the low 16 bits, those of
