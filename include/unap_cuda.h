@@ -554,7 +554,8 @@ int unap_cuda_set_matrix_wavefronts(int on);
 int unap_cuda_set_cheby_chunk(int entries);
 /* Chebyshev V-cycles run their coarse levels of at most `rows` rows (and
  * every level below them) in one launch instead of a launch per step
- * (default 60000; 0: never).  Results are identical.  Returns the previous
+ * (default 60000, levels whose rows average more than 32 entries apart;
+ * other values go by rows alone; 0: never).  Results are identical.  Returns the previous
  * value; applies to AMG handles created afterwards.  No counterpart in the
  * reference. */
 int unap_cuda_set_cheby_tail_rows(int rows);

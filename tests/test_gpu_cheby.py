@@ -286,3 +286,27 @@ def test_matrix_without_wavefronts(cuda, orc, precision):
             A.close()
     finally:
         capi.set_matrix_wavefronts(old)
+
+
+def test_tail_leaves_long_rows_to_launches(cuda):
+    """By default a level whose rows average more than 32 entries, and every
+    level above it, takes a launch per step (an FP32 V-cycle of this system
+    took 725 us with all levels in the tail, 519 without); a hierarchy of short
+    rows has all its levels in the tail.  A level in the tail below its first
+    one has no time of its own in the profile."""
+    from test_gpu_flow import random_system
+    for s, in_tail in ((random_system(30000, 300000, 1, symm=True), False),
+                       (W.laplace(30, seed=2, permute=True), True)):
+        s.upper = -np.abs(s.upper)
+        s.diag = W._fast_row_abs_sum(s.n, s.lower_addr, s.upper_addr, s.upper, s.upper) + 0.1
+        A = capi.DeviceMatrix(s)
+        G = capi.DeviceAmg(A, n_coarsest=100, precision=1, smoother=1, cheby_from=0)
+        sizes = G.level_sizes()
+        ms = G.profile_vcycle(reps=1)["level_ms"]
+        long_rows = [k for k, (n, nf, _) in enumerate(sizes[1:-1], 1) if 2 * nf > 32 * n]
+        first = max(long_rows, default=0) + 1  # the tail's first level
+        assert (first == 1) == in_tail
+        assert all(t > 0 for t in ms[:first + 1])
+        assert all(t == 0 for t in ms[first + 1:] if first < len(sizes) - 1)
+        G.close()
+        A.close()

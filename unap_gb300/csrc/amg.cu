@@ -169,12 +169,15 @@ AmgHierarchy::AmgHierarchy(Matrix& A_, const AmgParams& p) : params(p), A(A_)
     // the Chebyshev levels of at most cheby_tail_rows() rows, and all below,
     // in one launch
     if (params.smoother == 1 && cheby_tail_rows() > 0) {
-        for (int k = std::max(1, params.chebyFrom); k < L; ++k)
-            if (lv[(size_t)k].n <= cheby_tail_rows() &&
-                cheb_flow_stages(L - k, params.chebyDegree) <= kChebTailMaxStages) {
-                chebTail = k;
-                break;
-            }
+        const int rows = cheby_tail_rows();
+        auto fits = [&](int k) {
+            const Level& Lk = *lv[(size_t)k].L;
+            if (Lk.n > rows || cheb_flow_stages(L - k, params.chebyDegree) > kChebTailMaxStages)
+                return false;
+            return rows != kChebTailRows || 2.0 * Lk.nf <= (double)kChebTailEntries * Lk.n ||
+                   (params.precision == 0 && Lk.n <= kChebTailLongRows64);
+        };
+        for (int k = L - 1; k >= std::max(1, params.chebyFrom) && fits(k); --k) chebTail = k;
         if (chebTail > 0) {
             if (params.precision == 1)
                 buildChebTail<float>(s);

@@ -86,6 +86,16 @@ void k_prolong_add_to(const Exec& ex, int n, const int* cmap, const T* coarse, c
 
 // ---- the coarse end of a Chebyshev V-cycle in one launch (cheb_flow.cu) --
 constexpr int kChebTailRows = 60000;   // default of set_cheby_tail_rows
+// By default a tail level's rows also hold up to this many entries on average,
+// what a task loads before any wait: longer rows take another dependent load per
+// 32 entries, past L1, where the per-step kernels' gathers hit it.  What one more
+// level in the tail changes of a V-cycle, us: FP32, 4 to 25 entries, -6 to -18 at
+// 100 to 30,000 rows; 50 to 100 entries, +5 to +40; 150 to 900, +15 to +165 (a
+// hierarchy of a random graph of 30,000 cells and 20 entries: 512 without a tail,
+// 736 with all levels in it).  FP64, where the sums are longer than the loads:
+// 32 to 900 entries, -35 to +57 up to 2,048 rows, -30 to +424 at 2,500 to 8,000.
+constexpr int kChebTailEntries = 32;
+constexpr int kChebTailLongRows64 = 2048;  // FP64 levels of any row length
 constexpr int kChebTailMaxStages = 600;
 constexpr int kChebTailCtas = 8;       // CTAs of 128 threads an SM at most
 
@@ -130,7 +140,8 @@ struct ChebFlow {
 };
 
 // Chebyshev V-cycles run their levels of at most `rows` rows (and every
-// level below them) in the tail launch; 0 turns it off.  Returns the
+// level below them) in the tail launch; 0 turns it off.  The default also
+// looks at the rows' length (above), other values do not.  Returns the
 // previous value; applies to hierarchies built afterwards.
 int set_cheby_tail_rows(int rows);
 int cheby_tail_rows();
