@@ -85,3 +85,28 @@ def test_fp32_cycles_near_the_smallest_numbers(cuda, exponent):
     assert not np.isfinite(cycle(b)).all()
     G.close()
     A.close()
+
+
+@pytest.mark.parametrize("leaves", [255, 256, 257, 3000])
+@pytest.mark.parametrize("entries", [8, 20])
+def test_products_with_a_long_row(cuda, orc, leaves, entries):
+    """A row on each side of the longest one whose columns are looked up, in
+    systems of short and of longer rows; more than 2^20 entries are left to
+    the copying form too."""
+    torch = cuda
+    n = 60_000
+    g = random_system(n, n * entries // 2, 7, near=2000)
+    key = np.concatenate([g.lower_addr.astype(np.int64) * (n + 1) + g.upper_addr,
+                          np.arange(leaves).astype(np.int64) * (n + 1) + n])
+    order = np.argsort(key)
+    rng = np.random.default_rng(leaves)
+    s = type(g)(n + 1, (key[order] // (n + 1)).astype(np.int32),
+                (key[order] % (n + 1)).astype(np.int32), rng.standard_normal(key.size),
+                rng.standard_normal(n + 1), rng.standard_normal(key.size),
+                rng.standard_normal(n + 1))
+    A = capi.DeviceMatrix(s)
+    x = rng.standard_normal(s.n)
+    y = torch.empty(s.n, dtype=torch.float64, device="cuda")
+    A.spmv(torch.tensor(x, device="cuda"), y)
+    assert np.array_equal(y.cpu().numpy(), orc.spmv(s, x))
+    A.close()

@@ -553,7 +553,7 @@ int unap_cuda_spmv(long int handle, const double* x, double* y)
         order_after_default_stream(A.stream);
         Exec ex{A.stream, device_max_blocks()};
         h->ensureScratch();
-        k_spmv_reference<double>(ex, rows64(*A.L), A.L->d_perm.p, x, y, h->s1.p);
+        k_spmv_reference<double>(ex, *A.L, rows64(*A.L), x, y, h->s1.p);
         UNAP_CK(cudaGetLastError());
         UNAP_CK(cudaStreamSynchronize(A.stream));
     });

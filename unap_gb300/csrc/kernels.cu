@@ -570,16 +570,23 @@ __global__ void __launch_bounds__(kBlock)
 // internal order first.  A whole call, us, copy first against lookups: 16.7
 // and 13.6 at 20^3, 21.8 and 19.0 at 50^3, 36.9 and 33.4 at 80^3, 50.2 and
 // 52.5 at 100^3, 299 and 481 at 200^3.  (With the result scattered by a launch
-// of its own as well: 22.7 at 20^3, 384 at 200^3.)
-static constexpr int kLookupRows = 1 << 19;
+// of its own as well: 22.7 at 20^3, 384 at 200^3.)  Two more limits: the entries
+// of rows of more than 8 (100,000 rows of 12, 20, 45: 38.7 and 41.3, 40.6 and 43.2,
+// 55.0 and 62.4; 30,000 rows 27.4 and 24.7, 30.4 and 27.8, 34.8 and 32.5), and the
+// longest row, where a lookup is one more dependent load per chunk (20^3 with a
+// hub of 128, 256, 512, 4,096 entries: 37.6 and 35.1, 53.3 and 53.4, 85.4 and 90.4,
+// 524 and 587).
+static constexpr int kLookupRows = 1 << 19, kLookupEntries = 1 << 20, kLookupRowLen = 256;
 
 template <class T>
-void k_spmv_reference(const Exec& ex, const Rows<T>& A, const int* perm, const T* x, T* y, T* xi)
+void k_spmv_reference(const Exec& ex, const Level& L, const Rows<T>& A, const T* x, T* y, T* xi)
 {
+    const int* perm = L.d_perm.p;
     if (A.n <= 0) return;
     // an x that y overlaps is copied first
     const bool apart = x + A.n <= y || y + A.n <= x;
-    const bool look = A.n < kLookupRows && apart;
+    const bool look = A.n < kLookupRows && apart && L.maxRowLen <= kLookupRowLen &&
+                      (!A.wide || 2LL * L.nf <= kLookupEntries);
     if (!look) k_to_internal<T>(ex, A.n, perm, x, xi);
     if (!look && row_streams(A, RSpec{})) {
         stream_spmv_reference<T>(ex, A, perm, xi, y);
@@ -853,7 +860,7 @@ int device_max_blocks()
 #define INST(T)                                                                                   \
     template void k_spmv<T>(const Exec&, const Rows<T>&, const T*, T*, const T*, RSpec, Gate,      \
                             bool);                                                               \
-    template void k_spmv_reference<T>(const Exec&, const Rows<T>&, const int*, const T*, T*, T*); \
+    template void k_spmv_reference<T>(const Exec&, const Level&, const Rows<T>&, const T*, T*, T*); \
     template void k_pcg_direction<T>(const Exec&, int, const T*, double*, const KState*, Gate,     \
                                      bool);                                                      \
     template void k_dot2<T>(const Exec&, int, const T*, const double*, const T*, const double*,    \

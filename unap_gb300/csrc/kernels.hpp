@@ -31,9 +31,9 @@ constexpr int kDenseChunk = 64;
 template <class T>
 void k_spmv(const Exec& ex, const Rows<T>& A, const T* x, T* y, const T* dotWith, RSpec red,
             Gate g, bool fused = false);
-// y = A x, both in the caller's row order; xi: scratch of A.n entries
+// y = A x (A: L's rows), both in the caller's row order; xi: scratch of A.n entries
 template <class T>
-void k_spmv_reference(const Exec& ex, const Rows<T>& A, const int* perm, const T* x, T* y, T* xi);
+void k_spmv_reference(const Exec& ex, const Level& L, const Rows<T>& A, const T* x, T* y, T* xi);
 
 // r = b - A x; with a reduction spec, sums r.r (sum0)
 template <class T>
