@@ -424,8 +424,8 @@ void transfer_maps(const Level& F, const Level& C, const CoarseHost& c,
 {
     const int n = F.n, nc = C.n;
     const std::vector<int>& agg = c.restrictAddr;
-    const long long minCells = device_setup_min_cells();
-    if (minCells < 0 || n < minCells / 4 || c.largest > kMaxList) {
+    if (!setup_level_on_device(device_setup_min_cells(), n, F.byKernels ? 0 : -1, 1) ||
+        c.largest > kMaxList) {
         std::vector<int> refStart((size_t)nc + 1, 0);
         for (int i = 0; i < n; ++i) refStart[(size_t)agg[(size_t)i] + 1]++;
         for (int k = 0; k < nc; ++k) refStart[(size_t)k + 1] += refStart[(size_t)k];

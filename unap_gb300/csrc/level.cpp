@@ -30,8 +30,7 @@ size_t Level::deviceBytes() const
 {
     return d_perm.bytes() + d_iperm.bytes() + d_sliceOff.bytes() + d_rowInfo.bytes() +
            d_col.bytes() + d_val.bytes() + d_valT.bytes() + d_diag.bytes() + d_val32.bytes() +
-           d_diag32.bytes() + tasks[0].bytes() + tasks[1].bytes() +
-           tasks[2].bytes();
+           d_diag32.bytes() + taskMem.bytes();
 }
 
 namespace {
@@ -91,6 +90,7 @@ std::unique_ptr<Level> build_level(const HostLdu& A, const std::vector<int>* key
         setup_level_on_device(device_setup_min_cells(), A.n, links, kCellsPerWavefront)) {
         if (auto D = build_level_device(A, key, s, wavefronts)) {
             D->version = next_version();
+            D->byKernels = true;
             flow_tasks(*D, s);
             return D;
         }

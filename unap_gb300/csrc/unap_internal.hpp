@@ -307,16 +307,16 @@ __host__ __device__ inline int row_low(int info) { return (int)((unsigned)info >
 struct SweepTasks {
     int lanes;  // lanes a row: tasks of up to 32 / lanes rows
     int n = 0;
-    DevArray<int4> task;
-    DevArray<int2> near;
+    int4* task = nullptr;  // in the level's taskMem
+    int2* near = nullptr;
     SweepTasks(int l) : lanes(l) {}
-    size_t bytes() const { return task.bytes() + near.bytes(); }
 };
 
 // Per-matrix topology on the device (shared by FP64 and FP32 values).
 struct Level {
     int n = 0, nf = 0;
     bool symm = true;
+    bool byKernels = false;  // its structure was made by kernels
     bool sweepable = true;   // oriented && ownerSorted: DIC/DILU/GS allowed
     int nWave = 0;           // number of forward wavefronts
     std::vector<int> waveStart;  // nWave+1, internal row ranges
@@ -333,6 +333,7 @@ struct Level {
     DevArray<int> d_sliceOff, d_rowInfo, d_col;
     // sweeps (flow.hpp), sweepable levels only
     SweepTasks tasks[3] = {1, 4, 8};
+    DevArray<int4> taskMem;  // their tables, one after another
     // FP64 values
     DevArray<double> d_val, d_valT, d_diag;
     // FP32 values (mixed precision); filled on demand
@@ -386,7 +387,7 @@ inline bool setup_level_on_device(long long minCells, long long n, long long lin
     if (n >= minCells) return true;
     return n >= minCells / 4 && links >= 0 && links * cellsPerLink <= n;
 }
-constexpr int kCellsPerRound = 256, kCellsPerWavefront = 512;
+constexpr int kCellsPerRound = 256, kCellsPerWavefront = 768;
 // ... and COO/CSR input of many entries (8,192 / 11,000 / 32,000 cells with 7
 // entries: 0.39 / 0.50 / 1.46 ms on the host, 0.43 / 0.44 / 0.50 by kernels)
 inline bool setup_input_on_device(long long minCells, long long n, long long entries)
