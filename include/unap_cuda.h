@@ -586,15 +586,15 @@ int unap_cuda_tail_cluster_size(int* clusterSize);
  * (*recovered = 1).  Nothing faults and nothing waits without a bound. */
 int unap_cuda_selftest_barrier_timeout(int* timedOut, int* recovered);
 
-/* The same for the sweeps' waits for neighbouring rows, which by default give
- * up after 2^23 polls (2.5 s or more): with a bound of one poll a launch on
- * the matrix ends with waits run out and *timedOut = 1.  what: 0 Gauss-Seidel
+/* The same for the sweeps' waits for neighbouring rows, which give up after
+ * 2^23 polls (2.5 s or more): a launch on the matrix whose rows have one poll
+ * left in their first wait ends with waits run out and *timedOut = 1.  what: 0 Gauss-Seidel
  * sweeps, 1 DIC/DILU factorisation, 2 its application, 3 a whole solve by a
  * thread-block cluster (symmetric matrices).  The launch works on vectors of
  * its own. */
 int unap_cuda_selftest_wait_timeout(long int handle, int what, int* timedOut);
-/* One V-cycle of an AMG handle whose waits have a bound of one poll: fails
- * with UNAP_CUDA_ECUDA, as any call does whose waits ran out. */
+/* One V-cycle of an AMG handle with one poll left in such waits: fails with
+ * UNAP_CUDA_ECUDA, as any call does whose waits ran out. */
 int unap_cuda_selftest_vcycle_timeout(long int amg);
 
 /* ---- Text dumps in the reference's on-disk formats (host only; no GPU

@@ -356,8 +356,8 @@ def set_team_solve_cells(cells: int) -> int:
 
 def set_cheby_tail_rows(rows: int) -> int:
     """Chebyshev V-cycles run their levels of at most `rows` rows (and all
-    below) in one launch (default 60000; 0: never), for AMG handles created
-    afterwards; returns the previous value."""
+    below) in one launch (default 60000, levels of long rows apart; 0: never), for
+    AMG handles created afterwards; returns the previous value."""
     return int(load().unap_cuda_set_cheby_tail_rows(int(rows)))
 
 

@@ -40,8 +40,8 @@ double now_seconds()
 // The most that a request of this kind holds at once, setup scratch included,
 // on grids (rows of similar length; SELL padding of others comes on top).
 // Measured at 8,000 / 29,760 / 118,800 / 508,200 cells, against this, bytes a
-// cell: PCG+DIC 269 / 240 / 232 / 230 against 283 / 261 / 256 / 255, PBiCGStab+
-// DILU 356 / 328 / 320 / 318 against 374 / 354 / 350 / 350, mixed AMG 617 /
+// cell: PCG+DIC 259 / 231 / 224 / 222 against 283 / 261 / 256 / 255, PBiCGStab+
+// DILU 346 / 319 / 312 / 310 against 374 / 354 / 350 / 350, mixed AMG 617 /
 // 504 / 497 / 460 against 1465 / 739 / 541 / 492 (FP64 AMG a little less).  The
 // fixed terms: task counters and allocation granules; the dense coarsest
 // inverse of up to 1,000 cells.
